@@ -504,8 +504,9 @@ std::vector<std::pair<std::string, uint64_t>> Builder::device_allocations() cons
         {"staged records", stage_rec_.bytes},
         {"staged LUT", stage_lut_.bytes},
         {"sub-step words", leaf_frac_.bytes + stage_frac_.bytes},
+        {"octant tables", units_.bytes + unit_sync_.bytes + oct_off_.bytes},
         {"subsampling scratch", key_cache_.bytes + unit_cache_.bytes + acc_best_.bytes + acc_sel_.bytes +
-                                    cell_slot_.bytes + acc_intra_.bytes + emit_maps_.bytes + emit_state_.bytes + csr_count_.bytes +
+                                    acc_intra_.bytes + emit_maps_.bytes + emit_state_.bytes +
                                     csr_start_.bytes + csr_pts_.bytes},
         {"brick tables", g_key_.bytes + g_mask_.bytes + g_base_.bytes},
         {"level tables", sub_nodes_.bytes + out_points_.bytes + stage_off_.bytes + post_ii_.bytes + node_dst_.bytes +
@@ -822,10 +823,20 @@ void Builder::generate() {
                                   data_idx_.as<uint64_t>(), fill_.as<uint32_t>(), cfg_.n, err_.as<uint32_t>(), stream_);
     launches_ += launch_push_tags(pyr_.as<uint32_t>(), loff_.as<uint64_t>(), depth_, cfg_.chunk_grid, occ,
                                   err_.as<uint32_t>(), stream_);
-    launches_ += launch_distribute(cloud_.as<uint8_t>(), cfg_.n, cfg_.stride, f32, g, op, pyr_.as<uint32_t>(),
-                                   data_idx_.as<uint64_t>(), fill_.as<uint32_t>(), lut_.as<uint32_t>(),
-                                   rec_.as<uint8_t>(), leaf_frac_.as<uint32_t>(), err_.as<uint32_t>(), num_sms_,
-                                   stream_);
+    leaf_cells_ = octant_subsampling();
+    if (leaf_cells_) {
+        FineAxis fine[3];
+        for (int a = 0; a < 3; ++a) fine[a] = make_fine_axis(cfg_.bb_min[a], cfg_.bb_max[0] - cfg_.bb_min[0], depth_);
+        launches_ += launch_distribute_cells(cloud_.as<uint8_t>(), cfg_.n, cfg_.stride, f32, g, op, fine,
+                                             pyr_.as<uint32_t>(), data_idx_.as<uint64_t>(), fill_.as<uint32_t>(),
+                                             lut_.as<uint32_t>(), rec_.as<uint8_t>(), leaf_frac_.as<uint32_t>(),
+                                             err_.as<uint32_t>(), num_sms_, stream_);
+    } else {
+        launches_ += launch_distribute(cloud_.as<uint8_t>(), cfg_.n, cfg_.stride, f32, g, op, pyr_.as<uint32_t>(),
+                                       data_idx_.as<uint64_t>(), fill_.as<uint32_t>(), lut_.as<uint32_t>(),
+                                       rec_.as<uint8_t>(), leaf_frac_.as<uint32_t>(), err_.as<uint32_t>(), num_sms_,
+                                       stream_);
+    }
     stage_mark("distribute");
     check_cuda(cudaGetLastError(), "launch");
     build_tree_host();
@@ -931,6 +942,14 @@ void Builder::build_tree_host() {
         }
     }
     if (off != cfg_.n) throw Error("leaf points do not add up to the point amount");
+}
+
+// Octant subsampling (k_units.cu) takes power-of-two grids from 8 to 128: cells
+// of coarser levels are then unions of the finest level's.  Waves and other
+// grids use the kernels of k_subsample.cu.
+bool Builder::octant_subsampling() const {
+    const uint32_t S = cfg_.sub_grid;
+    return !wave_ && S >= 8 && S <= 128 && (S & (S - 1)) == 0;
 }
 
 void Builder::subsample() {
@@ -1047,6 +1066,52 @@ void Builder::subsample() {
             ++nc;
         }
         sn.nchild = nc;
+        sn.child_kind |= (uint32_t)v.mask << 8;
+    }
+    // ---- units of octant subsampling: the children of every node in octant
+    // order.  On levels of fewer units than the blocks the chip holds at once
+    // (the top of the tree) inner children are split in parts, down to 4096
+    // candidates.
+    bool octants = leaf_cells_ && octant_subsampling();
+    std::vector<UnitEntry> units;
+    std::vector<uint32_t> unit_first(depth_ + 2, 0);
+    std::vector<uint8_t> any_split(depth_ + 2, 0);
+    uint32_t s_log2 = 0;
+    while ((1u << s_log2) < S) ++s_log2;
+    if (octants) {
+        for (uint32_t l = 1; l <= depth_; ++l) {
+            unit_first[l] = (uint32_t)units.size();
+            uint64_t whole = 0;
+            for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) whole += table[k].nchild;
+            const bool few = S >= 64 && whole < (uint64_t)num_sms_ * 3;
+            for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
+                const NodeHost& v = nodes_[order[k]];
+                uint32_t c = v.child_first, number = 0, q0 = 0;
+                for (uint32_t s = 0; s < 8; ++s) {
+                    if (!(v.mask & (1u << s))) continue;
+                    const uint32_t ci = c++;
+                    const NodeHost& ch = nodes_[ci];
+                    const bool split = few && ch.internal && out_bound[ci] > 4096;
+                    if (split) {
+                        any_split[l] = 1;
+                        table[k].child_kind |= 1u << (16 + s);
+                    }
+                    for (uint32_t part = split ? 8 : 0; part < (split ? 16u : 1u); ++part) {
+                        UnitEntry e;
+                        e.node = k - level_first[l];
+                        e.flags = s | (part << 3) | ((uint32_t)ch.internal << 7) | ((uint32_t)(number == 0) << 8) |
+                                  (number << 10) | (q0 << 16);
+                        e.src = ch.internal ? ii_of[ci] : (uint32_t)ch.data_idx;
+                        e.count = ch.internal ? 0 : ch.points;
+                        units.push_back(e);
+                        ++number;
+                    }
+                    q0 = s + 1;
+                }
+                units.back().flags |= 1u << 9;
+            }
+        }
+        unit_first[depth_ + 1] = (uint32_t)units.size();
     }
 
     // ---- capacities: the staging arrays hold every level's candidates
@@ -1056,7 +1121,7 @@ void Builder::subsample() {
     const uint64_t out_cap = (uint64_t)((float)cfg_.n * cfg_.output_factor);   // octree_processor_impl.cu:24-31
     uint64_t stage_cap = std::max<uint64_t>(sub_stage_cap_, std::max<uint64_t>(out_cap, cfg_.n));
     uint64_t scratch_cap = std::max<uint64_t>(sub_scratch_cap_, std::min(max_level_bound, stage_cap));
-    {
+    auto size_brick_tables = [&]() {
         // global brick tables: enough slots for the largest node at 68% load
         // (bricks <= candidates and <= bricks of the grid)
         const uint64_t bs = (S + 3) / 4;
@@ -1074,17 +1139,20 @@ void Builder::subsample() {
         g_base_.ensure(blocks * cap * 4);
         g_cap_ = (uint32_t)cap;
         g_shift_ = shift;
-    }
+    };
     // final record arrays: N leaf records (written) + P_out internal records
     uint64_t rec_cap = std::max<uint64_t>(sub_rec_cap_, std::max<uint64_t>(out_cap, cfg_.n));
     // node table and post order staged in pinned memory (copied on the build
     // stream; the previous build's copies completed before it returned)
     const size_t table_bytes = (size_t)n_internal * sizeof(SubNode);
     const size_t o_post = (table_bytes + 15) & ~(size_t)15;
-    table_host_.ensure(o_post + (size_t)n_internal * 4 + 16);
+    const size_t o_units = (o_post + (size_t)n_internal * 4 + 15) & ~(size_t)15;
+    const size_t units_bytes = units.size() * sizeof(UnitEntry);
+    table_host_.ensure(o_units + units_bytes + 16);
     if (n_internal) {
         std::memcpy(table_host_.p, table.data(), table_bytes);
         std::memcpy(table_host_.as<uint8_t>(o_post), post.data(), (size_t)n_internal * 4);
+        if (units_bytes) std::memcpy(table_host_.as<uint8_t>(o_units), units.data(), units_bytes);
     }
     post_ii_.ensure(std::max<size_t>((size_t)n_internal * 4, 4));
     sub_nodes_.ensure(std::max<size_t>(table_bytes, sizeof(SubNode)));
@@ -1096,7 +1164,8 @@ void Builder::subsample() {
     // internal node its points, staged offset and final position
     const size_t o_pts = 32, o_soff = (o_pts + (size_t)n_internal * 4 + 7) & ~(size_t)7;
     const size_t o_dst = o_soff + (size_t)n_internal * 8;
-    back_host_.ensure(o_dst + (size_t)n_internal * 8);
+    const size_t o_used = o_dst + (size_t)n_internal * 8;   // octants: scratch slots taken per level
+    back_host_.ensure(o_used + 16 * 8);
     place_src_.ensure((size_t)n_internal * 8 + 8);
     place_dst_.ensure((size_t)n_internal * 8 + 8);
     place_cnt_.ensure((size_t)n_internal * 4 + 4);
@@ -1108,21 +1177,36 @@ void Builder::subsample() {
     work_.ensure(4);
 
     for (int attempt = 0;; ++attempt) {
-        key_cache_.ensure(scratch_cap * 4);
-        acc_best_.ensure(scratch_cap * 8);
-        cell_slot_.ensure(scratch_cap * 4);
-        if (cfg_.random) acc_sel_.ensure(scratch_cap * 4);
-        if (averaged && !weighted) acc_intra_.ensure(scratch_cap * 8);
+        // Octant subsampling works in the buffers of the other kernels (a
+        // server's lane serves both): staged colours and face sums in the
+        // record staging (8 + 8 of its 18 bytes), face lists in key cache and
+        // cell list, weighted sums of face cells in the cell-unit cache.
+        if (octants) {
+            if (cfg_.random) acc_best_.ensure(scratch_cap * 8);
+            if (averaged) stage_rec_.ensure(stage_cap * 18 + 64);
+            if (inter) key_cache_.ensure(scratch_cap * 8);
+            units_.ensure(std::max<size_t>(units_bytes, sizeof(UnitEntry)));
+            unit_sync_.ensure(kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 8);
+            oct_off_.ensure((size_t)n_internal * 32 + 32);
+        } else {
+            size_brick_tables();
+            key_cache_.ensure(scratch_cap * 8);   // key cache and cell list
+            acc_best_.ensure(scratch_cap * 8);
+            if (cfg_.random) acc_sel_.ensure(scratch_cap * 4);
+            stage_rec_.ensure(stage_cap * 18 + 64);
+        }
+        if (inter && !weighted) acc_intra_.ensure(scratch_cap * 8);
+        else if (averaged && !weighted && !octants) acc_intra_.ensure(scratch_cap * 8);
         if (weighted) {
-            unit_cache_.ensure(scratch_cap * 12);
-            csr_count_.ensure(scratch_cap * 4);
+            unit_cache_.ensure(scratch_cap * 16);   // cell units and counts
             csr_start_.ensure(scratch_cap * 4);
             csr_pts_.ensure(scratch_cap * 20);
-            emit_maps_.ensure((size_t)kSplitEmitNodes * kBrickMapBytes);
-            emit_state_.ensure((size_t)kSplitEmitNodes * 16);
+            if (!octants) {
+                emit_maps_.ensure((size_t)kSplitEmitNodes * kBrickMapBytes);
+                emit_state_.ensure((size_t)kSplitEmitNodes * 16);
+            }
         }
         stage_lut_.ensure(stage_cap * 4);
-        stage_rec_.ensure(stage_cap * 18 + 64);
         stage_frac_.ensure(stage_cap * 4);
         if (copy_stream_) check_cuda(cudaStreamSynchronize(copy_stream_), "output copies");
         lut_.ensure_keep(rec_cap * 4, (size_t)cfg_.n * 4, stream_);
@@ -1154,7 +1238,7 @@ void Builder::subsample() {
         a.leaf_rec = rec_.as<uint8_t>();
         a.stage_lut = stage_lut_.as<uint32_t>();
         a.stage_rec = stage_rec_.as<uint8_t>();
-        a.leaf_frac = leaf_frac_.as<uint32_t>();
+        a.leaf_frac = leaf_cells_ ? nullptr : leaf_frac_.as<uint32_t>();
         a.stage_frac = stage_frac_.as<uint32_t>();
         a.out_frac = stage_frac_.as<uint32_t>();
         a.out_lut = stage_lut_.as<uint32_t>();
@@ -1163,9 +1247,9 @@ void Builder::subsample() {
         a.unit_cache = unit_cache_.as<float>();
         a.acc_best = acc_best_.as<uint64_t>();
         a.acc_sel = acc_sel_.as<uint32_t>();
-        a.cell_slot = cell_slot_.as<uint32_t>();
+        a.cell_slot = key_cache_.as<uint32_t>() + scratch_cap;
         a.acc_intra = acc_intra_.as<uint64_t>();
-        a.csr_count = csr_count_.as<uint32_t>();
+        a.csr_count = unit_cache_.as<uint32_t>() + scratch_cap * 3;
         a.csr_start = csr_start_.as<uint32_t>();
         a.csr_pts = csr_pts_.as<uint8_t>();
         a.out = op;
@@ -1180,7 +1264,65 @@ void Builder::subsample() {
         // wave, which issues it with the other builds' (one subsampling
         // launch per level over all of them); repeats run alone
         const bool in_wave = wave_ && attempt == 0;
-        if (in_wave) {
+        if (octants) {
+            if (units_bytes)
+                check_cuda(cudaMemcpyAsync(units_.p, table_host_.as<uint8_t>(o_units), units_bytes,
+                                           cudaMemcpyHostToDevice, stream_),
+                           "H2D units");
+            check_cuda(cudaMemsetAsync(unit_sync_.p, 0,
+                                       kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 8,
+                                       stream_),
+                       "memset");
+            uint8_t* sync = unit_sync_.as<uint8_t>();
+            UnitNodeState* node_state = reinterpret_cast<UnitNodeState*>(sync + kUnitSyncHead);
+            uint64_t* unit_state = reinterpret_cast<uint64_t*>(node_state + n_internal);
+            for (uint32_t l = 1; l <= depth_; ++l) {
+                const uint32_t first = level_first[l], cnt = level_first[l + 1] - first;
+                if (!cnt) continue;
+                UnitLevelArgs u{};
+                u.nodes = sub_nodes_.as<SubNode>() + first;
+                u.units = units_.as<UnitEntry>() + unit_first[l];
+                u.n_nodes = cnt;
+                u.n_units = unit_first[l + 1] - unit_first[l];
+                u.s = s_log2;
+                u.level = l;
+                u.first_internal = first;
+                u.seed = cfg_.seed;
+                u.cloud = cloud_.as<uint8_t>();
+                u.stride = cfg_.stride;
+                u.float_input = cfg_.cloud_type == 0;
+                u.leaf_lut = lut_.as<uint32_t>();
+                u.leaf_word = leaf_frac_.as<uint32_t>();
+                u.leaf_rec = rec_.as<uint8_t>();
+                u.stage_lut = stage_lut_.as<uint32_t>();
+                u.stage_word = stage_frac_.as<uint32_t>();
+                u.stage_col = stage_rec_.as<uint64_t>();
+                u.out_points = out_points_.as<uint32_t>();
+                u.stage_off = stage_off_.as<uint64_t>();
+                u.oct_off = oct_off_.as<uint32_t>();
+                u.node_state = node_state + first;
+                u.unit_state = unit_state + unit_first[l];
+                u.level_used = reinterpret_cast<uint64_t*>(sync);
+                u.stage_cap = stage_cap;
+                u.scratch_cap = scratch_cap;
+                u.best = acc_best_.as<uint64_t>();
+                u.sum = acc_intra_.as<uint64_t>();
+                u.faces = key_cache_.as<uint2>();
+                u.face_sum = stage_rec_.as<uint64_t>() + stage_cap;
+                u.partial = unit_cache_.as<uint64_t>();
+                u.partial_cap = scratch_cap * 12 / 32;
+                u.partials = reinterpret_cast<uint64_t*>(sync + 192) + l;
+                u.csr_count = unit_cache_.as<uint32_t>() + scratch_cap * 3;
+                u.csr_start = csr_start_.as<uint32_t>();
+                u.csr_pts = csr_pts_.as<float4>();
+                u.ticket = reinterpret_cast<uint32_t*>(sync + 128) + l;
+                u.err = err_.as<uint32_t>();
+                launches_ += launch_units_level(u, mode, any_split[l], num_sms_, stream_);
+                char mark[32];
+                std::snprintf(mark, sizeof mark, "sub_l%u", l);
+                stage_mark(mark);
+            }
+        } else if (in_wave) {
             if (!level_ready_) check_cuda(cudaEventCreateWithFlags(&level_ready_, cudaEventDisableTiming), "event");
             std::vector<WaveLevel> plan(depth_);
             for (uint32_t l = 1; l <= depth_; ++l) {
@@ -1239,8 +1381,15 @@ void Builder::subsample() {
                                           place_dst_.as<uint64_t>(), place_cnt_.as<uint32_t>(),
                                           node_dst_.as<uint64_t>(), out_total_.as<uint64_t>(), err_.as<uint32_t>(),
                                           stream_);
-        launches_ += launch_place(place_src_.as<uint64_t>(), place_dst_.as<uint64_t>(), place_cnt_.as<uint32_t>(),
-                                  n_internal, stage_rec_.as<uint8_t>(), rec_.as<uint8_t>(), stream_);
+        if (octants)
+            launches_ += launch_place_units(place_src_.as<uint64_t>(), place_dst_.as<uint64_t>(),
+                                            place_cnt_.as<uint32_t>(), n_internal, cfg_.n, out_total_.as<uint64_t>(),
+                                            op, cloud_.as<uint8_t>(), cfg_.stride, cfg_.cloud_type == 0, averaged,
+                                            stage_lut_.as<uint32_t>(), stage_rec_.as<uint64_t>(), rec_.as<uint8_t>(),
+                                            err_.as<uint32_t>(), num_sms_, stream_);
+        else
+            launches_ += launch_place(place_src_.as<uint64_t>(), place_dst_.as<uint64_t>(), place_cnt_.as<uint32_t>(),
+                                      n_internal, stage_rec_.as<uint8_t>(), rec_.as<uint8_t>(), stream_);
         stage_mark("place");
         check_cuda(cudaGetLastError(), "subsample launch");
         check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(0), err_.p, 4, cudaMemcpyDeviceToHost, stream_), "D2H err");
@@ -1257,11 +1406,27 @@ void Builder::subsample() {
                                        cudaMemcpyDeviceToHost, stream_),
                        "D2H");
         }
+        if (octants)
+            check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(o_used), unit_sync_.p, 16 * 8, cudaMemcpyDeviceToHost,
+                                       stream_),
+                       "D2H");
         check_cuda(cudaStreamSynchronize(stream_), "subsample");
         const uint32_t e = *back_host_.as<uint32_t>(0);
         p_out_ = *back_host_.as<uint64_t>(16);
+        if ((e & kErrForeign) && attempt < 6 && !(e & ~(kErrForeign | kErrCapacity))) {
+            // a point that two levels' formulas put on different sides of an
+            // octant boundary: the pass is repeated by the kernels of whole nodes
+            octants = false;
+            const uint32_t none = 0;
+            check_cuda(cudaMemcpyAsync(err_.p, &none, 4, cudaMemcpyHostToDevice, stream_), "H2D err");
+            continue;
+        }
         if (!(e & kErrCapacity)) {
             stage_used_ = *back_host_.as<uint64_t>(8);
+            if (octants) {
+                stage_used_ = 0;
+                for (uint32_t l = 1; l <= depth_; ++l) stage_used_ += back_host_.as<uint64_t>(o_used)[l];
+            }
             sub_err_ = e;
             sub_err_valid_ = true;
             stats_.subsample_passes = (uint32_t)attempt + 1;

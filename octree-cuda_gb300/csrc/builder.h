@@ -248,6 +248,7 @@ private:
     void params_writable();
     void record_params();
     void size_for_config();
+    bool octant_subsampling() const;
     void subsample();
     void compute_stats();
 
@@ -273,11 +274,13 @@ private:
     DevBuf lut_, rec_;                  // final outputs (N + P_out records)
     DevBuf stage_lut_, stage_rec_;      // staged internal outputs
     DevBuf sub_nodes_, out_points_, work_;
-    DevBuf key_cache_, unit_cache_, acc_best_, acc_sel_, cell_slot_, acc_intra_, emit_maps_, emit_state_, csr_count_, csr_start_, csr_pts_;
+    DevBuf key_cache_, unit_cache_, acc_best_, acc_sel_, acc_intra_, emit_maps_, emit_state_, csr_start_, csr_pts_;
     DevBuf place_src_, place_dst_, place_cnt_;
     DevBuf g_key_, g_mask_, g_base_;   // per-block global brick tables
     DevBuf cell_keys_, spread_;         // chunking-grid boundary keys and Morton spread table
-    DevBuf leaf_frac_, stage_frac_;     // sub-step words of leaf and staged records
+    DevBuf leaf_frac_, stage_frac_;     // sub-step or cell words of leaf and staged records
+    bool leaf_cells_ = false;           // the leaf words are cell words (octant subsampling)
+    DevBuf units_, unit_sync_, oct_off_;   // octant subsampling: unit table, counters and waits, octant offsets
     DevBuf bbox_keys_;                  // ordered keys of the coordinate minima / maxima
     DevBuf stage_off_, level_base_;     // staged position of each internal node's outputs; staging fill
     uint8_t* host_rec_ = nullptr;      // caller's output arrays (set_output_host)

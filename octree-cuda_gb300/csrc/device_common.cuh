@@ -67,6 +67,30 @@ __host__ __device__ inline OutAxis make_out_axis(double mn, double sf) {
 
 constexpr int32_t kCoordError = (int32_t)0x80000000;
 
+// Finest subsampling cells along one axis of the cloud's cube: those of a
+// 128^3 grid in a node of level 1 (see out_coord_cell).
+struct FineAxis {
+    float b_hi, b_lo;   // cells per coordinate unit
+    float e;            // 2^-22 + what binary64 rounding at any level is worth, in cells
+};
+
+// mn: box minimum, side: cube side, depth: tree depth.  A node's box minimum
+// comes from at most `depth` additions of binary64, its cell size from two more
+// roundings of numbers up to M = max(|mn|, |mn + side|, side), and the formula
+// adds the rounding of p - min and of the quotient: together under
+// (depth + 8) * 2^-52 * M in coordinate units; twice that is allowed for.
+inline FineAxis make_fine_axis(double mn, double side, uint32_t depth) {
+    FineAxis f;
+    const double cells = (double)(64ull << depth);
+    const double B = cells / side;
+    f.b_hi = (float)B;
+    f.b_lo = (float)(B - (double)f.b_hi);
+    const double a = mn < 0 ? -mn : mn, z = mn + side < 0 ? -(mn + side) : mn + side;
+    const double M = a > z ? (a > side ? a : side) : (z > side ? z : side);
+    f.e = (float)((2.384185791015625e-07 + (depth + 8.0) * 4.440892098500626e-16 * M * B) * 1.000001);   // 2^-22, 2^-51
+    return f;
+}
+
 // ---------------------------------------------------------------------------
 // Morton order with x as the most significant bit of every triple: the child
 // slot of a cell inside its parent is the low three bits (x<<2 | y<<1 | z),
@@ -126,6 +150,7 @@ enum : uint32_t {
     kErrTag = 1u << 4,           // a point found no leaf
     kErrTimeout = 1u << 5,       // a bounded wait on a bulk copy gave up
     kErrNodeCap = 1u << 6,       // the tree has more nodes than the node table holds
+    kErrForeign = 1u << 7,       // a candidate's cell lies outside its child's octant (the pass is repeated)
 };
 
 // ---------------------------------------------------------------------------
@@ -320,6 +345,61 @@ __device__ __forceinline__ uint32_t pack_frac(uint32_t fx, uint32_t fy, uint32_t
 }
 
 // ---------------------------------------------------------------------------
+// Cell words of octant subsampling: bit 31 says that the cell is proven at
+// every level, bits 0-20 its coordinates x | y << 7 | z << 14 (a leaf's points:
+// in their parent's grid of 128^3 cells; an inner node's: in its own grid).
+
+constexpr uint32_t kSafeWord = 0x80000000u;
+
+// Quantised output coordinate (as out_coord) and cell of the finest grid of
+// one axis, which share the exact difference to the box minimum.  `safe` is
+// set when the cell-unit position U = (p - min) * B lies at least E from every
+// integer and inside [0, cells): E covers the rounding of this evaluation
+// (the first two terms, as in out_coord_frac) and, in f.e, what the binary64
+// formula of any level can differ from U, so that every level's formula and
+// the counting grid's give the cell (int)U or an ancestor of it.
+template <bool kFloatInput>
+__device__ __forceinline__ int32_t out_coord_cell(const Coord& c, const OutAxis& o, const FineAxis& f, uint32_t cells,
+                                                  uint32_t& cell, bool& safe) {
+    safe = false;
+    cell = 0;
+    if (kFloatInput || c.ok) {
+        // s + e1 = hi - m_hi exactly (Knuth TwoSum)
+        const float nm = -o.m_hi;
+        const float s = __fadd_rn(c.hi, nm);
+        const float bb = __fsub_rn(s, c.hi);
+        const float e1 = __fadd_rn(__fsub_rn(c.hi, __fsub_rn(s, bb)), __fsub_rn(nm, bb));
+        const float lo2 = __fsub_rn(__fadd_rn(e1, c.lo), o.m_lo);
+        const float reach = __fadd_rn(fabsf(c.hi), fabsf(o.m_hi));
+        {
+            const float ph = __fmul_rn(s, f.b_hi);
+            const float pl = __fmaf_rn(s, f.b_lo, __fmaf_rn(lo2, f.b_hi, __fmaf_rn(s, f.b_hi, -ph)));
+            const float fl = floorf(ph);
+            const float frac = __fadd_rn(__fsub_rn(ph, fl), pl);
+            const float g = floorf(frac);
+            const float rem = __fsub_rn(frac, g);
+            const float E = __fmaf_rn(__fmaf_rn(reach, f.b_hi, fabsf(ph)), 2.2737367544323206e-13f, f.e);   // 2^-42
+            if (fabsf(ph) < 1.0e9f && rem >= E && rem <= __fsub_rn(1.0f, E)) {
+                cell = (uint32_t)((int32_t)fl + (int32_t)g);
+                safe = cell < cells;
+            }
+        }
+        const float ph = __fmul_rn(s, o.sf_hi);
+        const float pl = __fmaf_rn(s, o.sf_lo, __fmaf_rn(lo2, o.sf_hi, __fmaf_rn(s, o.sf_hi, -ph)));
+        if (fabsf(ph) < 1.0e9f) {
+            const float fl = floorf(ph);
+            const float frac = __fadd_rn(__fsub_rn(ph, fl), pl);
+            const float g = floorf(frac);
+            const float rem = __fsub_rn(frac, g);
+            const float E = __fmaf_rn(__fmaf_rn(reach, fabsf(o.sf_hi), fabsf(ph)), 2.2737367544323206e-13f,
+                                      2.384185791015625e-07f);   // 2^-42, 2^-22
+            if (rem >= E && rem <= __fsub_rn(1.0f, E)) return (int32_t)fl + (int32_t)g;
+        }
+    }
+    return exact_out_coord(exact_value<kFloatInput>(c), o.mn, o.sf);
+}
+
+// ---------------------------------------------------------------------------
 // Packed colour sums (encodeColors kernel_helpers.cuh:49-53, decode
 // fp_subsampling.cuh:95-101).  A zero count field (a multiple of 1024 points)
 // divides by zero in the reference; here it yields 0xFFFF.
@@ -383,15 +463,20 @@ __device__ __forceinline__ float exp_neg(float x) {
     return __fmul_rn(p, __uint_as_float((unsigned)(k + 127) << 23));
 }
 
-__device__ __forceinline__ uint32_t weight_q(float ux, float uy, float uz, int nx, int ny, int nz) {
-    float dx = __fsub_rn(__fadd_rn((float)nx, 0.5f), ux);
-    float dy = __fsub_rn(__fadd_rn((float)ny, 0.5f), uy);
-    float dz = __fsub_rn(__fadd_rn((float)nz, 0.5f), uz);
+// cx, cy, cz: the neighbour cell's centre (n + 0.5).
+__device__ __forceinline__ uint32_t weight_at(float ux, float uy, float uz, float cx, float cy, float cz) {
+    float dx = __fsub_rn(cx, ux);
+    float dy = __fsub_rn(cy, uy);
+    float dz = __fsub_rn(cz, uz);
     float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
     float q = __fmul_rn(d2, (float)(4.0 / 27.0));
     q = fminf(q, 1.5f);
     float w = exp_neg(__fmul_rn(-10.0f, q));
     return (uint32_t)__fadd_rn(__fmul_rn(w, 268435456.0f), 0.5f);
+}
+
+__device__ __forceinline__ uint32_t weight_q(float ux, float uy, float uz, int nx, int ny, int nz) {
+    return weight_at(ux, uy, uz, __fadd_rn((float)nx, 0.5f), __fadd_rn((float)ny, 0.5f), __fadd_rn((float)nz, 0.5f));
 }
 
 // ---------------------------------------------------------------------------
@@ -437,6 +522,40 @@ __device__ __forceinline__ void load_point(const uint8_t* rec, Coord c[3], uint3
         col[0] = (uint32_t)r3 & 0xFF;
         col[1] = (uint32_t)(r3 >> 8) & 0xFF;
         col[2] = (uint32_t)(r3 >> 16) & 0xFF;
+    }
+}
+
+// As load_point, from the two or three 16-byte words that cover the record:
+// where the lanes of a warp read records far apart, the load units work per
+// word and lane (a 27-byte record by load_point takes five).
+template <bool kFloatInput, bool kColour>
+__device__ __forceinline__ void gather_point(const uint8_t* rec, Coord c[3], uint32_t col[3]) {
+    constexpr uint32_t kBytes = (kFloatInput ? 12u : 24u) + (kColour ? 3u : 0u);
+    constexpr int kWords = kFloatInput ? 4 : 7;
+    const uintptr_t addr = reinterpret_cast<uintptr_t>(rec);
+    const uint4* q = reinterpret_cast<const uint4*>(addr & ~(uintptr_t)15);
+    const uint32_t o = (uint32_t)addr & 15u;
+    const uint4 v0 = q[0];
+    const uint4 v1 = o + kBytes > 16 ? q[1] : make_uint4(0, 0, 0, 0);
+    const uint4 v2 = o + kBytes > 32 ? q[2] : make_uint4(0, 0, 0, 0);
+    const uint32_t w[12] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w};
+    uint32_t a[kWords + 2], r[kWords];   // shifted by two words, then one, then bytes
+#pragma unroll
+    for (int j = 0; j < kWords + 2; ++j) a[j] = (o & 8) ? w[j + 2 < 12 ? j + 2 : 11] : w[j];
+#pragma unroll
+    for (int j = 0; j < kWords; ++j) {
+        const uint32_t lo = (o & 4) ? a[j + 1] : a[j], hi = (o & 4) ? a[j + 2] : a[j + 1];
+        r[j] = __funnelshift_r(lo, hi, (o & 3u) * 8u);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        c[k] = kFloatInput ? coord_f32(__uint_as_float(r[k]))
+                           : coord_f64(__hiloint2double((int)r[kFloatInput ? 0 : 2 * k + 1], (int)r[kFloatInput ? 0 : 2 * k]));
+    if (kColour) {
+        const uint32_t v = r[kWords - 1];
+        col[0] = v & 0xFF;
+        col[1] = (v >> 8) & 0xFF;
+        col[2] = (v >> 16) & 0xFF;
     }
 }
 

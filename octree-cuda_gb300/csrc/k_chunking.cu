@@ -58,10 +58,11 @@ struct ChunkSmem {
     uint32_t keys_off, spread_off, buf_off, buf_bytes, total;
 };
 
-__host__ __device__ inline ChunkSmem chunk_smem(uint32_t stride, uint32_t grid, bool f32, uint32_t tile) {
+__host__ __device__ inline ChunkSmem chunk_smem(uint32_t stride, uint32_t grid, bool f32, uint32_t tile,
+                                                bool keys = true) {
     ChunkSmem m;
     m.keys_off = 128;
-    m.spread_off = align_up(m.keys_off + 3 * (grid + 2) * (f32 ? 4u : 8u), 16);
+    m.spread_off = align_up(m.keys_off + (keys ? 3 * (grid + 2) * (f32 ? 4u : 8u) : 0u), 16);
     m.buf_off = align_up(m.spread_off + grid * 4, 128);
     m.buf_bytes = align_up(tile * stride + 48, 128);
     m.total = m.buf_off + 2 * m.buf_bytes;
@@ -70,11 +71,12 @@ __host__ __device__ inline ChunkSmem chunk_smem(uint32_t stride, uint32_t grid, 
 
 // Copies the boundary keys and the spread table into shared memory.
 template <bool kF32>
-__device__ __forceinline__ void load_tables(const CloudGrid& g, uint8_t* smem, const ChunkSmem& L) {
+__device__ __forceinline__ void load_tables(const CloudGrid& g, uint8_t* smem, const ChunkSmem& L, bool keys = true) {
     using K = typename std::conditional<kF32, int32_t, long long>::type;
     const K* src = static_cast<const K*>(g.keys);
     K* dst = reinterpret_cast<K*>(smem + L.keys_off);
-    for (uint32_t i = threadIdx.x; i < 3 * (g.grid + 2); i += blockDim.x) dst[i] = src[i];
+    if (keys)
+        for (uint32_t i = threadIdx.x; i < 3 * (g.grid + 2); i += blockDim.x) dst[i] = src[i];
     uint32_t* sp = reinterpret_cast<uint32_t*>(smem + L.spread_off);
     for (uint32_t i = threadIdx.x; i < g.grid; i += blockDim.x) sp[i] = g.spread[i];
 }
@@ -460,7 +462,7 @@ __global__ void __launch_bounds__(1024) k_leaf_prep(const uint32_t* __restrict__
         const uint64_t pre = block_exclusive_scan64(c, warp_sums, tot);
         if (i < n) {
             fill[i] = 0;
-            data_idx[i] = leaf ? running + pre : 0;
+            data_idx[i] = leaf ? (running + pre) | ((uint64_t)level[i] << kLeafLevelShift) : 0;
             if (leaf) pyr[loff[level[i]] + key[i]] = kLeafTag | i;
         }
         running += tot;
@@ -509,16 +511,24 @@ __global__ void k_push_tags(uint32_t* __restrict__ pyr, const uint64_t* __restri
 // equal leaves reserves the run's slots with one atomic.  At most 40
 // registers, so that three 448-thread blocks share an SM (47 registers leave
 // room for two: 119.7M-point build 2.73 -> 2.56 ms).
-template <bool kF32>
+// kCells: the cell words of octant subsampling instead of sub-step words.  The
+// proven finest cell gives the counting cell as well (its upper bits), so the
+// boundary-key lookup is left out; an unproven axis is evaluated in binary64.
+struct FineAxes {
+    FineAxis ax[3];
+    uint32_t cells;   // finest cells per axis
+};
+
+template <bool kF32, bool kCells>
 __global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* __restrict__ cloud, uint64_t n,
-                                                              uint32_t stride, CloudGrid g, OutParams op,
+                                                              uint32_t stride, CloudGrid g, OutParams op, FineAxes fa,
                                                               const uint32_t* __restrict__ pyr0,
                                                               const uint64_t* __restrict__ data_idx, uint32_t* fill,
                                                               uint32_t* __restrict__ lut, uint8_t* __restrict__ rec,
                                                               uint32_t* __restrict__ frac, uint32_t* err) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const ChunkSmem L = chunk_smem(stride, g.grid, kF32, kDistTile);
-    load_tables<kF32>(g, smem, L);
+    const ChunkSmem L = chunk_smem(stride, g.grid, kF32, kDistTile, !kCells);
+    load_tables<kF32>(g, smem, L, !kCells);
     const uint32_t lane = threadIdx.x & 31;
     tile_loop<kDistTile>(cloud, n, stride, smem, L, err, [&](const uint8_t* recs, uint64_t p0, uint32_t cnt) {
 #pragma unroll 1
@@ -527,11 +537,31 @@ __global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* _
             constexpr int kWords = kF32 ? 4 : 7;
             uint32_t w[kWords];
             uint32_t m = kNoKey;
+            int32_t q[3];      // kCells: output coordinates, finest cells, colour
+            uint32_t fine[3];
+            bool proven = true;
             if (k < cnt) {
                 record_words<kWords>(recs + (uint64_t)k * stride, w);
                 int cell[3];
-                if (point_cells<kF32>(w, g, smem, L, cell)) m = cell_morton(cell, smem, L);
-                else set_error(err, kErrBelowBox);
+                if (kCells) {
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        const Coord c = kF32 ? coord_f32(__uint_as_float(w[a]))
+                                             : coord_f64(__hiloint2double((int)w[2 * a + 1], (int)w[2 * a]));
+                        bool safe;
+                        q[a] = out_coord_cell<kF32>(c, op.ax[a], fa.ax[a], fa.cells, fine[a], safe);
+                        cell[a] = (int)(fine[a] >> 6);
+                        if (!safe) {
+                            proven = false;
+                            cell[a] = exact_axis_cell(exact_value<kF32>(c), g.ax[a].mn, g.ax[a].t, g.grid);
+                        }
+                    }
+                    if ((cell[0] | cell[1] | cell[2]) >= 0) m = cell_morton(cell, smem, L);
+                    else set_error(err, kErrBelowBox);
+                } else {
+                    if (point_cells<kF32>(w, g, smem, L, cell)) m = cell_morton(cell, smem, L);
+                    else set_error(err, kErrBelowBox);
+                }
             }
             uint32_t starts = run_starts(m);
             uint32_t leader = run_leader(starts);
@@ -544,10 +574,12 @@ __global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* _
             }
             starts = run_starts(node);
             leader = run_leader(starts);
-            uint64_t first = 0;
+            uint64_t first = 0;   // the leaf's level above kLeafLevelShift
             if (node != kNoKey && lane == leader) first = data_idx[node] + atomicAdd(&fill[node], run_end(starts) - lane);
             first = ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(first >> 32), leader) << 32) |
                     __shfl_sync(0xffffffffu, (uint32_t)first, leader);
+            const uint32_t lv = (uint32_t)(first >> kLeafLevelShift);
+            first &= (1ull << kLeafLevelShift) - 1;
             uint32_t nw[5] = {0, 0, 0, 0, 0};
             bool ok = false;
             if (node != kNoKey) {
@@ -557,22 +589,29 @@ __global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* _
                 } else {
                     ok = true;
                     lut[pos] = (uint32_t)(p0 + k);
-                    Coord c[3];
-                    uint32_t col;
-                    if (kF32) {
-                        for (int a = 0; a < 3; ++a) c[a] = coord_f32(__uint_as_float(w[a]));
-                        col = w[3];
+                    const uint32_t col = w[kF32 ? 3 : 6];
+                    int32_t x, y, z;
+                    uint32_t fw;
+                    if (kCells) {
+                        x = q[0];
+                        y = q[1];
+                        z = q[2];
+                        fw = proven ? kSafeWord | ((fine[0] >> lv) & 127u) | (((fine[1] >> lv) & 127u) << 7) |
+                                          (((fine[2] >> lv) & 127u) << 14)
+                                    : 0u;
                     } else {
+                        Coord c[3];
                         for (int a = 0; a < 3; ++a)
-                            c[a] = coord_f64(__hiloint2double((int)w[2 * a + 1], (int)w[2 * a]));
-                        col = w[6];
+                            c[a] = kF32 ? coord_f32(__uint_as_float(w[a]))
+                                        : coord_f64(__hiloint2double((int)w[2 * a + 1], (int)w[2 * a]));
+                        uint32_t fx, fy, fz;
+                        x = out_coord_frac<kF32>(c[0], op.ax[0], fx);
+                        y = out_coord_frac<kF32>(c[1], op.ax[1], fy);
+                        z = out_coord_frac<kF32>(c[2], op.ax[2], fz);
+                        fw = pack_frac(fx, fy, fz);
                     }
-                    uint32_t fx, fy, fz;
-                    const int32_t x = out_coord_frac<kF32>(c[0], op.ax[0], fx);
-                    const int32_t y = out_coord_frac<kF32>(c[1], op.ax[1], fy);
-                    const int32_t z = out_coord_frac<kF32>(c[2], op.ax[2], fz);
                     if (x == kCoordError || y == kCoordError || z == kCoordError) set_error(err, kErrCoordRange);
-                    if (frac) frac[pos] = pack_frac(fx, fy, fz);
+                    if (frac) frac[pos] = fw;
                     nw[0] = (uint32_t)x;
                     nw[1] = (uint32_t)y;
                     nw[2] = (uint32_t)z;
@@ -798,21 +837,40 @@ int launch_push_tags(uint32_t* pyr, const uint64_t* loff_dev, uint32_t depth, ui
     return 1;
 }
 
+namespace {
+
+template <bool kF32, bool kCells>
+void distribute_on(const uint8_t* cloud, uint64_t n, uint32_t stride, const CloudGrid& g, const OutParams& out,
+                   const FineAxes& fa, const uint32_t* pyr0, const uint64_t* data_idx, uint32_t* fill, uint32_t* lut,
+                   uint8_t* rec, uint32_t* word, uint32_t* err, int num_sms, cudaStream_t stream) {
+    const size_t smem = chunk_smem(stride, g.grid, kF32, kDistTile, !kCells).total;
+    const int grid = chunk_grid_size(k_distribute<kF32, kCells>, kDistThreads, kDistTile, smem, n, num_sms);
+    k_distribute<kF32, kCells><<<grid, kDistThreads, smem, stream>>>(cloud, n, stride, g, out, fa, pyr0, data_idx, fill,
+                                                                     lut, rec, word, err);
+}
+
+}   // namespace
+
 int launch_distribute(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
                       const OutParams& out, const uint32_t* pyr0, const uint64_t* data_idx, uint32_t* fill,
                       uint32_t* lut, uint8_t* rec, uint32_t* frac, uint32_t* err, int num_sms,
                       cudaStream_t stream) {
     if (n == 0) return 0;
-    const size_t smem = chunk_smem(stride, g.grid, float_input, kDistTile).total;
-    if (float_input) {
-        const int grid = chunk_grid_size(k_distribute<true>, kDistThreads, kDistTile, smem, n, num_sms);
-        k_distribute<true><<<grid, kDistThreads, smem, stream>>>(cloud, n, stride, g, out, pyr0, data_idx, fill, lut,
-                                                                  rec, frac, err);
-    } else {
-        const int grid = chunk_grid_size(k_distribute<false>, kDistThreads, kDistTile, smem, n, num_sms);
-        k_distribute<false><<<grid, kDistThreads, smem, stream>>>(cloud, n, stride, g, out, pyr0, data_idx, fill,
-                                                                   lut, rec, frac, err);
-    }
+    const auto go = float_input ? distribute_on<true, false> : distribute_on<false, false>;
+    go(cloud, n, stride, g, out, FineAxes{}, pyr0, data_idx, fill, lut, rec, frac, err, num_sms, stream);
+    return 1;
+}
+
+int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
+                            const OutParams& out, const FineAxis fine[3], const uint32_t* pyr0,
+                            const uint64_t* data_idx, uint32_t* fill, uint32_t* lut, uint8_t* rec, uint32_t* word,
+                            uint32_t* err, int num_sms, cudaStream_t stream) {
+    if (n == 0) return 0;
+    FineAxes fa;
+    for (int a = 0; a < 3; ++a) fa.ax[a] = fine[a];
+    fa.cells = g.grid * 64;   // 2^depth counting cells, each 64 finest cells wide
+    const auto go = float_input ? distribute_on<true, true> : distribute_on<false, true>;
+    go(cloud, n, stride, g, out, fa, pyr0, data_idx, fill, lut, rec, word, err, num_sms, stream);
     return 1;
 }
 

@@ -168,6 +168,16 @@ int launch_leaf_prep(const uint32_t* n_nodes, const uint16_t* info, const uint32
 int launch_push_tags(uint32_t* pyr, const uint64_t* level_off_dev, uint32_t depth, uint32_t grid, const uint8_t* occ,
                      uint32_t* err, cudaStream_t stream);
 
+// Level of a leaf beside its first record in data_idx (launch_leaf_prep).
+constexpr uint32_t kLeafLevelShift = 56;
+
+// Distribution that writes cell words (out_coord_cell) instead of sub-step
+// words: for the octant kernels (launch_units_level).
+int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
+                            const OutParams& out, const FineAxis fine[3], const uint32_t* pyr0,
+                            const uint64_t* data_idx, uint32_t* fill, uint32_t* lut, uint8_t* rec, uint32_t* word,
+                            uint32_t* err, int num_sms, cudaStream_t stream);
+
 int launch_distribute(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
                       const OutParams& out, const uint32_t* pyr0, const uint64_t* data_idx, uint32_t* fill,
                       uint32_t* lut, uint8_t* rec, uint32_t* frac, uint32_t* err, int num_sms,
@@ -278,6 +288,86 @@ int launch_emit_weighted(const SubLevelArgs& a, int num_sms, cudaStream_t stream
 // least `bytes` and never lowers it, so that builders launching the same
 // kernel from several host threads cannot undercut each other's launches.
 void allow_dynamic_smem(const void* kernel, size_t bytes);
+
+// ---- Octant subsampling (k_units.cu): subsampling grids 2^s with s from 3 to 7.
+
+// One unit of a level: the candidates of one child, in the child's octant of
+// the node's grid, or one of the eight parts (again octants) of a large one.
+struct UnitEntry {
+    uint32_t node;    // in the level's node table
+    // bits 0-2 octant, 3-6 part (0 whole, 8 + o part o), 7 staged (the child is
+    // an inner node), 8 / 9 first / last unit of the node, 10-15 its number in
+    // the node, 16-19 first octant whose offset the unit writes
+    uint32_t flags;
+    uint32_t src;     // leaf: first record; inner node: its internal index
+    uint32_t count;   // leaf: points
+};
+
+struct UnitNodeState {
+    uint64_t off1;    // first slot of the node in the level's scratch + 1 (0: not placed yet, ~0: did not fit)
+    uint32_t faces;   // entries of the node's face list
+    uint32_t points;  // candidates of the node (distance weighting)
+};
+
+// Head of the counters a pass starts from zero: level_used (16 x u64), the
+// tickets of the levels' launches (16 x u32), partials per level (16 x u64).
+constexpr size_t kUnitSyncHead = 320;
+
+struct UnitLevelArgs {
+    const SubNode* nodes;
+    const UnitEntry* units;
+    uint32_t n_nodes;
+    uint32_t n_units;
+    uint32_t s;             // log2 of the subsampling grid
+    uint32_t level;
+    uint32_t first_internal;
+    uint32_t smem_words;    // dynamic shared memory, set by the launcher
+    uint64_t seed;
+    const uint8_t* cloud;
+    uint32_t stride;
+    uint32_t float_input;
+    const uint32_t* leaf_lut;
+    const uint32_t* leaf_word;
+    const uint8_t* leaf_rec;
+    uint32_t* stage_lut;    // per staged point: cloud index
+    uint32_t* stage_word;   // cell word
+    uint64_t* stage_col;    // r | g << 16 | b << 32 (averaged modes)
+    // per internal node (level-major index)
+    uint32_t* out_points;
+    uint64_t* stage_off;
+    uint32_t* oct_off;      // first output of each octant
+    UnitNodeState* node_state;   // of this level
+    uint64_t* unit_state;   // of this level: cells + 1 (0: not counted yet), candidates << 32
+    uint64_t* level_used;   // per level: scratch slots taken
+    uint64_t stage_cap, scratch_cap;
+    // per scratch slot
+    uint64_t* best;         // selection key (explicit random)
+    uint64_t* sum;          // inter-cell: packed colour sum; afterwards those of face cells in the order of planes
+    uint2* faces;           // inter-cell and weighted: cells beside other units of their node {rank, word}, node by node
+    uint64_t* face_sum;     // ... their packed colour sum, or the number of their weighted sums in `partial`
+    // distance weighting: the candidates of every cell of a node one after the
+    // other {position in cell units, r | g << 8 | b << 16}
+    uint32_t* csr_count;    // per cell: candidates; afterwards ranks of face cells in the order of planes
+    uint32_t* csr_start;    // per cell: its first candidate in the node
+    float4* csr_pts;
+    uint64_t* partial;      // weighted sums (r, g, b, weight) of face cells over their own unit
+    uint64_t* partials;     // entries taken
+    uint64_t partial_cap;
+    uint32_t* ticket;
+    uint32_t* err;
+};
+
+// any_split: some child of the level is split in parts.  Inter-cell averaging takes two
+// launches: the units, then what their outermost cells get from other units.
+int launch_units_level(const UnitLevelArgs& a, uint32_t mode, bool any_split, int num_sms,
+                       cudaStream_t stream);
+
+// The records of the internal nodes at their post-order positions, made from
+// the cloud points and the staged colours (see k_place_units).
+int launch_place_units(const uint64_t* src_off, const uint64_t* dst_off, const uint32_t* count, uint32_t n_nodes,
+                       uint64_t n, const uint64_t* total, const OutParams& out, const uint8_t* cloud, uint32_t stride,
+                       bool float_input, bool averaged, const uint32_t* stage_lut, const uint64_t* stage_col,
+                       uint8_t* rec, uint32_t* err, int num_sms, cudaStream_t stream);
 
 // Moves staged internal-node records to their final (post-order) positions.
 int launch_place(const uint64_t* src_off, const uint64_t* dst_off, const uint32_t* count, uint32_t n_nodes,

@@ -1,0 +1,114 @@
+"""Octant subsampling (power-of-two grids from 8 to 128) at the sizes where its
+units change shape: the smallest and largest grids, children split in parts,
+leaves of more points than one unit's ranks hold, points without a cell proof,
+and points that two levels put on different sides of an octant boundary.
+Compared with the CPU oracle bit for bit."""
+import numpy as np
+import pytest
+
+from helpers import case_from_points, compare_results, make_case, run_gpu, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+MODES = {
+    "first": dict(),
+    "first_intra": dict(intra=True),
+    "first_inter": dict(inter=True),
+    "first_weighted": dict(inter=True, weighting=True),
+    "random": dict(random=True),
+    "random_intra": dict(random=True, intra=True),
+    "random_inter": dict(random=True, inter=True),
+    "random_weighted": dict(random=True, inter=True, weighting=True),
+}
+
+
+def points(name, n=60_000, seed=3):
+    rng = np.random.default_rng(seed)
+    if name == "volume":        # occupied cells in every direction, every octant
+        xyz = rng.random((n, 3))
+    elif name == "corner":      # most points in one leaf of the smallest tree
+        xyz = rng.random((n, 3))
+        xyz[: n * 4 // 5] *= 0.45
+    elif name == "plane":       # cells along both sides of an octant boundary
+        xyz = rng.random((n, 3))
+        xyz[:, 0] = 0.5 + (xyz[:, 0] - 0.5) * 0.02
+    elif name == "one_octant":  # nodes with a single child
+        xyz = rng.random((n, 3)) * 0.1 + 0.6
+    return xyz, rng.integers(0, 256, (n, 3), dtype=np.uint8)
+
+
+def check(case, cfg, passes=None):
+    ref = run_oracle(case, cfg)
+    s = run_gpu(case, cfg)
+    compare_results(ref, s)
+    # (a staging area that was too small also repeats the pass)
+    assert passes is None or s.stats()["subsample_passes"] == passes
+    s.close()
+
+
+@pytest.mark.parametrize("mode", sorted(MODES))
+@pytest.mark.parametrize("shape,cloud_type,n,chunk,sub,threshold", [
+    ("volume", 0, 60_000, 16, 8, 300), ("volume", 1, 60_000, 16, 128, 300), ("plane", 0, 60_000, 32, 64, 400),
+    ("one_octant", 1, 20_000, 64, 16, 200), ("corner", 0, 200_000, 2, 128, 20_000),
+    ("corner", 1, 150_000, 8, 32, 5_000)])
+def test_units(shape, cloud_type, n, chunk, sub, threshold, mode):
+    xyz, rgb = points(shape, n)
+    case = case_from_points(xyz * 50.0, rgb, cloud_type, scale=0.001, bbox=[0, 0, 0, 50.5, 50.5, 50.5])
+    check(case, dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=threshold, **MODES[mode]))
+
+
+@pytest.mark.parametrize("sub", [4, 100, 256])
+def test_other_grids(sub):
+    """Grids that octant subsampling does not take."""
+    case = make_case(0, 1, 40_000, seed=8)
+    check(case, dict(chunk_grid=32, sub_grid=sub, merge_threshold=600, inter=True))
+
+
+def middle_sides(p, mn, side, sub):
+    """Whether the counting grid (512) and the grid of the root's upper child put x coordinates p in the upper half of
+    that child (the binary64 formula)."""
+    cubic = (mn + side) - mn
+    m1 = mn + cubic / 2
+    count = np.floor((p - mn) / (cubic / 512)) >= 384
+    child = np.floor((p - m1) / (((m1 + cubic / 2) - m1) / sub)) >= sub // 2
+    return count, child
+
+
+@pytest.mark.parametrize("mode", ["first", "first_inter", "random_intra", "random_weighted"])
+def test_points_on_an_octant_boundary(mode):
+    """Points at the middle of a node whose formula puts them on the other side than the counting grid's."""
+    rng = np.random.default_rng(12)
+    side = 100.0
+    for _ in range(4000):
+        mn = float(rng.uniform(-60, 100))
+        p = np.array([mn + side * 0.75])
+        for _ in range(6):
+            p = np.unique(np.concatenate([p, np.nextafter(p, -np.inf), np.nextafter(p, np.inf)]))
+        a, b = middle_sides(p, mn, side, 128)
+        if (a != b).any():
+            break
+    assert (a != b).any()
+    n = 100_000
+    xyz = rng.random((n, 3)) * side
+    xyz[:, 0] += mn
+    xyz[:64, 0] = p[a != b][0]
+    rgb = rng.integers(0, 256, (n, 3), dtype=np.uint8)
+    case = case_from_points(xyz, rgb, 1, scale=0.01, bbox=[mn, 0, 0, mn + side, side, side])
+    check(case, dict(chunk_grid=512, sub_grid=128, merge_threshold=1000, output_factor=12.0, **MODES[mode]), passes=2)
+
+
+def test_grids_in_turn_on_one_session():
+    """One session through grids of both kinds and back: they share the scratch buffers."""
+    from helpers import octree_api
+
+    case = make_case(1, 0, 80_000, seed=31)
+    s = octree_api.OctreeSession(0)
+    s.set_cloud(case.cloud, n=case.n, stride=case.stride, cloud_type=case.cloud_type, scale=case.scale,
+                bb_min=case.bb_min, bb_max=case.bb_max)
+    for sub, mode in ((64, "first_inter"), (100, "random_weighted"), (32, "random_weighted"), (64, "first")):
+        cfg = dict(chunk_grid=64, sub_grid=sub, merge_threshold=1000, **MODES[mode])
+        s.configure(**cfg)
+        s.init()
+        s.generate()
+        compare_results(run_oracle(case, cfg), s)
+    s.close()
