@@ -1075,15 +1075,27 @@ void Builder::subsample() {
     bool octants = leaf_cells_ && octant_subsampling();
     std::vector<UnitEntry> units;
     std::vector<uint32_t> unit_first(depth_ + 2, 0);
-    std::vector<uint8_t> any_split(depth_ + 2, 0);
+    std::vector<uint8_t> any_split(depth_ + 2, 0), spread(depth_ + 2, 0);
+    std::vector<uint32_t> oct_unit;          // spread levels, per node and octant
+    std::vector<size_t> oct_first(depth_ + 2, 0);
+    uint64_t map_words = 0;                  // of the largest spread level
     uint32_t s_log2 = 0;
     while ((1u << s_log2) < S) ++s_log2;
     if (octants) {
+        // the part of the memory estimate that a brick table would take
+        const uint64_t map_room = (uint64_t)num_sms_ * memory_terms(cfg_, num_sms_).slots * 8;
         for (uint32_t l = 1; l <= depth_; ++l) {
             unit_first[l] = (uint32_t)units.size();
             uint64_t whole = 0;
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) whole += table[k].nchild;
             const bool few = S >= 64 && whole < (uint64_t)num_sms_ * 3;
+            // inter-cell colours cost less: the extra launch's lookups in global
+            // memory pay only where a unit has an SM of its own (level of 79
+            // units 123 -> 119 us, of 32 100 -> 76 us, but of 276 228 -> 256 us)
+            spread[l] = few && inter && whole && (weighted || whole <= (uint64_t)num_sms_);
+            oct_first[l] = oct_unit.size();
+            if (spread[l]) oct_unit.resize(oct_unit.size() + 8 * (size_t)(level_first[l + 1] - level_first[l]), ~0u);
+            uint64_t words = 0;
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
                 const NodeHost& v = nodes_[order[k]];
                 uint32_t c = v.child_first, number = 0, q0 = 0;
@@ -1096,13 +1108,20 @@ void Builder::subsample() {
                         any_split[l] = 1;
                         table[k].child_kind |= 1u << (16 + s);
                     }
+                    if (spread[l])
+                        oct_unit[oct_first[l] + (size_t)(k - level_first[l]) * 8 + s] =
+                            ((uint32_t)units.size() - unit_first[l]) | ((uint32_t)split << 31);
                     for (uint32_t part = split ? 8 : 0; part < (split ? 16u : 1u); ++part) {
-                        UnitEntry e;
+                        UnitEntry e{};
                         e.node = k - level_first[l];
                         e.flags = s | (part << 3) | ((uint32_t)ch.internal << 7) | ((uint32_t)(number == 0) << 8) |
                                   (number << 10) | (q0 << 16);
                         e.src = ch.internal ? ii_of[ci] : (uint32_t)ch.data_idx;
                         e.count = ch.internal ? 0 : ch.points;
+                        if (spread[l]) {
+                            e.map = (uint32_t)words;
+                            words += 2 * ((uint64_t)1 << (3 * (s_log2 - (split ? 2 : 1)) - 5)) + 4;
+                        }
                         units.push_back(e);
                         ++number;
                     }
@@ -1110,6 +1129,8 @@ void Builder::subsample() {
                 }
                 units.back().flags |= 1u << 9;
             }
+            if (words * 4 > map_room) spread[l] = 0;
+            if (spread[l]) map_words = std::max(map_words, words);
         }
         unit_first[depth_ + 1] = (uint32_t)units.size();
     }
@@ -1147,12 +1168,17 @@ void Builder::subsample() {
     const size_t table_bytes = (size_t)n_internal * sizeof(SubNode);
     const size_t o_post = (table_bytes + 15) & ~(size_t)15;
     const size_t o_units = (o_post + (size_t)n_internal * 4 + 15) & ~(size_t)15;
-    const size_t units_bytes = units.size() * sizeof(UnitEntry);
+    const size_t o_oct_unit = units.size() * sizeof(UnitEntry);   // units, then octant tables
+    const size_t units_bytes = o_oct_unit + oct_unit.size() * 4;
     table_host_.ensure(o_units + units_bytes + 16);
     if (n_internal) {
         std::memcpy(table_host_.p, table.data(), table_bytes);
         std::memcpy(table_host_.as<uint8_t>(o_post), post.data(), (size_t)n_internal * 4);
-        if (units_bytes) std::memcpy(table_host_.as<uint8_t>(o_units), units.data(), units_bytes);
+        if (octants) {
+            std::memcpy(table_host_.as<uint8_t>(o_units), units.data(), o_oct_unit);
+            if (!oct_unit.empty())
+                std::memcpy(table_host_.as<uint8_t>(o_units + o_oct_unit), oct_unit.data(), oct_unit.size() * 4);
+        }
     }
     post_ii_.ensure(std::max<size_t>((size_t)n_internal * 4, 4));
     sub_nodes_.ensure(std::max<size_t>(table_bytes, sizeof(SubNode)));
@@ -1180,13 +1206,16 @@ void Builder::subsample() {
         // Octant subsampling works in the buffers of the other kernels (a
         // server's lane serves both): staged colours and face sums in the
         // record staging (8 + 8 of its 18 bytes), face lists in key cache and
-        // cell list, weighted sums of face cells in the cell-unit cache.
+        // cell list, weighted sums of face cells in the cell-unit cache, the
+        // bitmaps of spread levels (at most 3 x SMs units, parts of 8 KB or
+        // whole octants of 64 KB) in a brick table.
         if (octants) {
             if (cfg_.random) acc_best_.ensure(scratch_cap * 8);
             if (averaged) stage_rec_.ensure(stage_cap * 18 + 64);
             if (inter) key_cache_.ensure(scratch_cap * 8);
             units_.ensure(std::max<size_t>(units_bytes, sizeof(UnitEntry)));
-            unit_sync_.ensure(kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 8);
+            unit_sync_.ensure(kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 12);
+            if (map_words) g_mask_.ensure(map_words * 4);
             oct_off_.ensure((size_t)n_internal * 32 + 32);
         } else {
             size_brick_tables();
@@ -1302,6 +1331,10 @@ void Builder::subsample() {
                 u.oct_off = oct_off_.as<uint32_t>();
                 u.node_state = node_state + first;
                 u.unit_state = unit_state + unit_first[l];
+                u.unit_rank = reinterpret_cast<uint32_t*>(unit_state + units.size()) + unit_first[l];
+                u.spread = spread[l];
+                u.oct_unit = reinterpret_cast<const uint32_t*>(units_.as<uint8_t>() + o_oct_unit) + oct_first[l];
+                u.maps = g_mask_.as<uint32_t>();
                 u.level_used = reinterpret_cast<uint64_t*>(sync);
                 u.stage_cap = stage_cap;
                 u.scratch_cap = scratch_cap;

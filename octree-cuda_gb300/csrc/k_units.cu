@@ -248,6 +248,7 @@ __device__ __forceinline__ void unit_place(const UnitLevelArgs& a, BlockShared& 
             a.stage_off[ii] = fail ? 0u : sh.level_base + off1 - 1;
             a.node_state[un.node].points = c0 + sh.included;
         }
+        a.unit_rank[ui] = r0;
         sh.rank0 = r0;
         sh.cand0 = c0;
         sh.off = off1 - 1;
@@ -425,6 +426,7 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
             a.stage_lut[oo + r] = (uint32_t)__ldcg(a.best + so + r);
         }
     }
+    if (a.spread) return;
     // ---- emit
     constexpr uint32_t kG = kWeightLanes;
     const uint32_t m0 = box.m0(), b = box.b(), g = lane / kG, s = lane % kG;
@@ -708,40 +710,44 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
     const uint32_t m0 = box.m0(), open = un.open;
     if constexpr (weighted) {
         unit_weighted<kRandom, kB, kLocal, Pre>(a, sh, box, l_key, l_word, l_cnt, cells, keep, so, oo, *ws);
-        return true;
-    }
-    for (uint32_t r0 = warp * 32; r0 < cells; r0 += T) {
-        const uint32_t r = r0 + lane;
-        bool face = false;
-        uint32_t w = 0;
-        if (r < cells) {
-            if (kLocal) w = l_word[r];
-            else if (kColor == 2) w = a.stage_word[oo + r];
-            if (kLocal) {
-                a.stage_word[oo + r] = w;
-                a.stage_lut[oo + r] = kRandom ? (uint32_t)l_key[r] : l_idx[r];
-            } else if (kRandom) {
-                a.stage_lut[oo + r] = (uint32_t)__ldcg(a.best + so + r);
-            }
-            uint64_t e = 0;
-            if (kColor == 1) e = kLocal ? l_packed[r] : __ldcg(a.stage_col + oo + r);
-            if (kColor == 2) {
-                const uint32_t x = w & m0, y = (w >> kFieldBits) & m0, z = (w >> (2 * kFieldBits)) & m0;
-                face = (faces_of(x, y, z, m0) & open) != 0;
-                e = box.sum27(x, y, z, [&](uint32_t q) { return kLocal ? l_packed[q] : __ldcg(g_packed + q); });
-            }
-            if (averaged) {
-                if (!face) {
-                    uint16_t cr, cg, cb;
-                    decode_colors(e, cr, cg, cb);
-                    e = pack_colour(cr, cg, cb);
+    } else {
+        for (uint32_t r0 = warp * 32; r0 < cells; r0 += T) {
+            const uint32_t r = r0 + lane;
+            bool face = false;
+            uint32_t w = 0;
+            if (r < cells) {
+                if (kLocal) w = l_word[r];
+                else if (kColor == 2) w = a.stage_word[oo + r];
+                if (kLocal) {
+                    a.stage_word[oo + r] = w;
+                    a.stage_lut[oo + r] = kRandom ? (uint32_t)l_key[r] : l_idx[r];
+                } else if (kRandom) {
+                    a.stage_lut[oo + r] = (uint32_t)__ldcg(a.best + so + r);
                 }
-                a.stage_col[oo + r] = e;
+                if (kColor == 2 && a.spread) {
+                    if (kLocal) a.sum[so + r] = l_packed[r];
+                    continue;
+                }
+                uint64_t e = 0;
+                if (kColor == 1) e = kLocal ? l_packed[r] : __ldcg(a.stage_col + oo + r);
+                if (kColor == 2) {
+                    const uint32_t x = w & m0, y = (w >> kFieldBits) & m0, z = (w >> (2 * kFieldBits)) & m0;
+                    face = (faces_of(x, y, z, m0) & open) != 0;
+                    e = box.sum27(x, y, z, [&](uint32_t q) { return kLocal ? l_packed[q] : __ldcg(g_packed + q); });
+                }
+                if (averaged) {
+                    if (!face) {
+                        uint16_t cr, cg, cb;
+                        decode_colors(e, cr, cg, cb);
+                        e = pack_colour(cr, cg, cb);
+                    }
+                    a.stage_col[oo + r] = e;
+                }
             }
+            if (kColor == 2 && !a.spread)
+                append_faces(a, un.node, sh.off, sh.rank0 + r, w,
+                             !face ? 0ull : kLocal ? l_packed[r] : __ldcg(g_packed + r), face);
         }
-        if (kColor == 2)
-            append_faces(a, un.node, sh.off, sh.rank0 + r, w,
-                         !face ? 0ull : kLocal ? l_packed[r] : __ldcg(g_packed + r), face);
     }
     return true;
 }
@@ -866,6 +872,15 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                 reinterpret_cast<uint32_t*>(pre)[(tid * kP + q) / 2] =
                     ((run + c[q]) & 0xFFFFu) | ((run + c[q + (kP > 1)]) << 16);
         }
+    }
+    if (kColor >= 2 && a.spread) {
+        __syncthreads();
+        uint32_t* map = a.maps + a.units[ui].map;
+        for (uint32_t i = tid; i < W; i += T) {
+            map[i] = bm[i];
+            map[W + 4 + i] = pre[i];
+        }
+        if (tid == 0) map[W] = 0;
     }
     // (unit_cells starts with a barrier after it cleared the cells)
     const uint32_t room = a.smem_words * 4 - (uint32_t)((pool - bm) * 4);
@@ -1106,6 +1121,165 @@ __global__ void __launch_bounds__(kFaceThreads) k_faces(const __grid_constant__ 
     }
 }
 
+// The colours of a level of few units (the top of the tree, where one unit's
+// cells would keep one SM busy while others idle): `chunks` blocks per unit,
+// each every chunks-th run of its cells.  Neighbours are looked up in the
+// units' bitmaps in global memory, those of other units through the node's
+// octant table, so that no cells are left over for k_faces.
+// Bounded by the weights' instructions.  Root of the 25.8M-point weighted
+// build (115,000 cells, 64 units of very unequal size): 1.27 -> 0.35 ms; levels
+// 8 and 7 1.24 -> 0.54 and 1.15 -> 0.88 ms.
+constexpr int kSpreadThreads = 256;
+
+struct SpreadMap {
+    const uint32_t* map;   // null: no such unit
+    uint32_t b, rank;      // log2 side of its box, rank of its first cell in the node
+};
+
+__device__ __forceinline__ SpreadMap spread_map(const UnitLevelArgs& a, uint32_t node, uint32_t x, uint32_t y,
+                                                uint32_t z) {
+    const uint32_t h = a.s - 1, o = ((x >> h) << 2) | ((y >> h) << 1) | (z >> h);
+    uint32_t u = a.oct_unit[node * 8 + o];
+    SpreadMap m{nullptr, h, 0};
+    if (u == ~0u) return m;
+    if (u >> 31) {
+        m.b = h - 1;
+        u = (u & 0x7FFFFFFFu) +
+            ((((x >> m.b) & 1) << 2) | (((y >> m.b) & 1) << 1) | ((z >> m.b) & 1));
+    }
+    m.map = a.maps + a.units[u].map;
+    m.rank = a.unit_rank[u];
+    return m;
+}
+
+// Occupied cells among the n at (x, y, z), (x + 1, y, z), ... of the unit's
+// box, as bits, and the node rank of the first of them.
+__device__ __forceinline__ uint32_t spread_row(const SpreadMap& m, uint32_t x, uint32_t y, uint32_t z, uint32_t n,
+                                               uint32_t& rank) {
+    if (!m.map) return 0;
+    const uint32_t m0 = (1u << m.b) - 1u, i = (x & m0) | ((y & m0) << m.b) | ((z & m0) << (2 * m.b)), w = i >> 5;
+    const uint32_t lo = m.map[w], t = __funnelshift_r(lo, m.map[w + 1], i) & ((1u << n) - 1u);
+    if (t) rank = m.rank + m.map[(1u << (3 * m.b - 5)) + 4 + w] + __popc(lo & ((1u << (i & 31)) - 1u));
+    return t;
+}
+
+template <int kColor>
+__global__ void __launch_bounds__(kSpreadThreads) k_spread(const __grid_constant__ UnitLevelArgs a, uint32_t chunks) {
+    constexpr uint32_t T = kSpreadThreads, kG = kColor == 3 ? kWeightLanes : 1;
+    __shared__ uint2 s_rows[kColor == 3 ? T / kG : 1][18];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, s = lane % kG;
+    const uint32_t ui = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
+    const uint32_t cells = (uint32_t)a.unit_state[ui] - 1u;
+    const UnitEntry en = a.units[ui];
+    const UnitNodeState st = a.node_state[en.node];
+    if (st.off1 == ~0ull || cells + 1 == 0 || chunk * (T / kG) >= cells) return;
+    uint64_t level_base = 0;
+    for (uint32_t l = 1; l < a.level; ++l) level_base += a.level_used[l];
+    const uint64_t off = st.off1 - 1;
+    const uint32_t rank0 = a.unit_rank[ui], node_cells = a.out_points[a.first_internal + en.node];
+    const uint32_t* words = a.stage_word + level_base + off + rank0;
+    uint64_t* colour = a.stage_col + level_base + off + rank0;
+    const uint32_t S = 1u << a.s;
+    const bool part = (en.flags >> 3) & 15;
+    const SpreadMap own{a.maps + en.map, part ? a.s - 2 : a.s - 1, rank0};
+    for (uint32_t f0 = chunk * (T / kG) + tid / kG; f0 - lane / kG < cells; f0 += chunks * (T / kG)) {
+        const bool act = f0 < cells;
+        const uint32_t w = words[min(f0, cells - 1)];
+        const uint32_t x = w & 127, y = (w >> kFieldBits) & 127, z = (w >> (2 * kFieldBits)) & 127;
+        // a row of up to three cells: those in the box of the cell's own x,
+        // and one more across its side
+        auto row = [&](uint32_t k, uint32_t (&t)[2], uint32_t (&rank)[2]) {
+            const uint32_t yy = y + k % 3 - 1, zz = z + k / 3 - 1;
+            t[0] = t[1] = 0;
+            if (!act || k >= 9 || yy >= S || zz >= S) return;
+            const bool inside = (((yy ^ y) | (zz ^ z)) >> own.b) == 0;
+            const SpreadMap m = inside ? own : spread_map(a, en.node, x, yy, zz);
+            const uint32_t q = (1u << m.b) - 1u, lx = x & q;
+            const uint32_t xa = lx ? x - 1 : x, xb = lx < q ? x + 1 : x;
+            t[0] = spread_row(m, xa, yy, zz, xb - xa + 1, rank[0]);
+            const uint32_t side = lx ? x + 1 : x - 1;   // beyond the box when lx is its first or last cell
+            if ((lx == 0 || lx == q) && side < S)
+                t[1] = spread_row(spread_map(a, en.node, side, yy, zz), side, yy, zz, 1, rank[1]);
+        };
+        if constexpr (kColor == 2) {
+            uint64_t e = 0;
+#pragma unroll 3
+            for (uint32_t k = 0; k < 9; ++k) {
+                uint32_t t[2], rank[2];
+                row(k, t, rank);
+                const uint64_t* p = a.sum + off;
+                if (t[0]) e += p[rank[0]];
+                if (t[0] & (t[0] - 1)) e += p[rank[0] + 1];
+                if (t[0] == 7) e += p[rank[0] + 2];
+                if (t[1]) e += p[rank[1]];
+            }
+            uint16_t cr, cg, cb;
+            decode_colors(e, cr, cg, cb);
+            if (act) colour[f0] = pack_colour(cr, cg, cb);
+        } else {
+            uint2* rows = s_rows[tid / kG];
+            constexpr uint32_t kR = (9 + kG - 1) / kG;
+            uint32_t from[2 * kR], len[2 * kR], sum = 0;
+#pragma unroll
+            for (uint32_t q = 0; q < kR; ++q) {
+                uint32_t t[2], rank[2];
+                row(s + q * kG, t, rank);
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    from[2 * q + d] = len[2 * q + d] = 0;
+                    if (t[d]) {
+                        const uint32_t n = rank[d] + __popc(t[d]);
+                        from[2 * q + d] = a.csr_start[off + rank[d]];
+                        len[2 * q + d] = (n < node_cells ? a.csr_start[off + n] : st.points) - from[2 * q + d];
+                    }
+                    sum += len[2 * q + d];
+                }
+            }
+            uint32_t incl = sum;
+#pragma unroll
+            for (uint32_t o = 1; o < kG; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o, kG);
+                if (s >= o) incl += v;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, kG - 1, kG);
+            uint32_t run = incl - sum;
+#pragma unroll
+            for (uint32_t q = 0; q < 2 * kR; ++q) {
+                const uint32_t slot = 2 * (s * (9 / kG) + min(s, 9 % kG)) + q;
+                if (s + q / 2 * kG < 9) rows[slot] = make_uint2(run + len[q], from[q] - run);
+                run += len[q];
+            }
+            __syncwarp();
+            uint64_t sr = 0, sg = 0, sb = 0, sw = 0;
+            const float cx = __fadd_rn((float)x, 0.5f), cy = __fadd_rn((float)y, 0.5f), cz = __fadd_rn((float)z, 0.5f);
+            uint2 e = rows[0];
+            const float4* pts = a.csr_pts + off;
+            for (uint32_t p = s, k = 0; p < total; p += kG) {
+                while (p >= e.x) e = rows[++k];
+                const float4 v = pts[e.y + p];
+                const uint32_t c = __float_as_uint(v.w);
+                const uint32_t wq = weight_at(v.x, v.y, v.z, cx, cy, cz);
+                sr += (uint64_t)wq * (c & 0xFFu);
+                sg += (uint64_t)wq * ((c >> 8) & 0xFFu);
+                sb += (uint64_t)wq * (c >> 16);
+                sw += wq;
+            }
+#pragma unroll
+            for (uint32_t o = kG / 2; o >= 1; o >>= 1) {
+                sr += __shfl_xor_sync(0xffffffffu, sr, o);
+                sg += __shfl_xor_sync(0xffffffffu, sg, o);
+                sb += __shfl_xor_sync(0xffffffffu, sb, o);
+                sw += __shfl_xor_sync(0xffffffffu, sw, o);
+            }
+            uint32_t c = 0;
+            if (act && s < 3) c = weighted_mean(s == 0 ? sr : s == 1 ? sg : sb, sw);
+            const uint32_t c1 = __shfl_sync(0xffffffffu, c, 1, kG), c2 = __shfl_sync(0xffffffffu, c, 2, kG);
+            if (act && s == 0) colour[f0] = pack_colour((uint16_t)c, (uint16_t)c1, (uint16_t)c2);
+            __syncwarp();   // the rows are written for the next cells
+        }
+    }
+}
+
 // Records of all internal nodes at their final positions (post-order after
 // the n leaf records): output coordinates from the cloud point as in
 // distribution, colours from the staging array (or, raw, the cloud point's).
@@ -1217,6 +1391,18 @@ void launch_faces(const UnitLevelArgs& a, bool any_split, int num_sms, cudaStrea
         a, slices, cut);
 }
 
+template <int kColor>
+void launch_colours(const UnitLevelArgs& a, bool any_split, int num_sms, cudaStream_t stream) {
+    if (!a.spread) {
+        launch_faces<kColor>(a, any_split, num_sms, stream);
+        return;
+    }
+    // about eight blocks per SM, at least one per unit
+    uint32_t chunks = 1;
+    while (chunks < 64 && (uint64_t)a.n_units * chunks < (uint64_t)std::max(num_sms, 1) * 16) chunks <<= 1;
+    k_spread<kColor><<<a.n_units * chunks, kSpreadThreads, 0, stream>>>(a, chunks);
+}
+
 }   // namespace
 
 int launch_units_level(const UnitLevelArgs& a, uint32_t mode, bool any_split, int num_sms,
@@ -1231,13 +1417,13 @@ int launch_units_level(const UnitLevelArgs& a, uint32_t mode, bool any_split, in
     if ((mode & kModeInter) && (mode & kModeWeight)) {
         if (random) launch_units<3, true>(a, num_sms, stream);
         else launch_units<3, false>(a, num_sms, stream);
-        launch_faces<3>(a, any_split, num_sms, stream);
+        launch_colours<3>(a, any_split, num_sms, stream);
         return 2;
     }
     if (mode & kModeInter) {
         if (random) launch_units<2, true>(a, num_sms, stream);
         else launch_units<2, false>(a, num_sms, stream);
-        launch_faces<2>(a, any_split, num_sms, stream);
+        launch_colours<2>(a, any_split, num_sms, stream);
         return 2;
     }
     if (random) launch_units<0, true>(a, num_sms, stream);

@@ -301,6 +301,8 @@ struct UnitEntry {
     uint32_t flags;
     uint32_t src;     // leaf: first record; inner node: its internal index
     uint32_t count;   // leaf: points
+    uint32_t map;     // spread levels: word offset of the unit's bitmap and ranks in `maps`
+    uint32_t pad;
 };
 
 struct UnitNodeState {
@@ -322,6 +324,8 @@ struct UnitLevelArgs {
     uint32_t level;
     uint32_t first_internal;
     uint32_t smem_words;    // dynamic shared memory, set by the launcher
+    uint32_t spread;        // inter-cell and weighted levels of few units: the units leave the
+                            // colours to k_spread, which spreads every unit over many blocks
     uint64_t seed;
     const uint8_t* cloud;
     uint32_t stride;
@@ -338,6 +342,9 @@ struct UnitLevelArgs {
     uint32_t* oct_off;      // first output of each octant
     UnitNodeState* node_state;   // of this level
     uint64_t* unit_state;   // of this level: cells + 1 (0: not counted yet), candidates << 32
+    uint32_t* unit_rank;    // of this level: rank of the unit's first cell in its node
+    const uint32_t* oct_unit;   // spread levels, per node and octant: its first unit | split in parts << 31, or ~0
+    uint32_t* maps;         // spread levels: per unit its bitmap, one word more, and the ranks of its words (32 bits)
     uint64_t* level_used;   // per level: scratch slots taken
     uint64_t stage_cap, scratch_cap;
     // per scratch slot
