@@ -250,6 +250,7 @@ private:
     void size_for_config();
     bool octant_subsampling() const;
     void subsample();
+    void compute_tree_stats();
     void compute_stats();
 
     BuildConfig cfg_;
