@@ -821,8 +821,8 @@ void Builder::generate() {
     launches_ += launch_leaf_prep(n_nodes_.as<uint32_t>(), info_.as<uint16_t>(), count_.as<uint32_t>(),
                                   level_.as<uint8_t>(), key_.as<uint32_t>(), pyr_.as<uint32_t>(), loff_.as<uint64_t>(),
                                   data_idx_.as<uint64_t>(), fill_.as<uint32_t>(), cfg_.n, err_.as<uint32_t>(), stream_);
-    launches_ += launch_push_tags(pyr_.as<uint32_t>(), loff_.as<uint64_t>(), depth_, cfg_.chunk_grid, occ,
-                                  err_.as<uint32_t>(), stream_);
+    launches_ += launch_push_tags(pyr_.as<uint32_t>(), loff_.as<uint64_t>(), depth_, occ, err_.as<uint32_t>(),
+                                  cloud_.as<uint8_t>(), cfg_.n, cfg_.stride, f32, g, stream_);
     leaf_cells_ = octant_subsampling();
     if (leaf_cells_) {
         FineAxis fine[3];

@@ -733,19 +733,22 @@ __device__ __forceinline__ void store_run(uint8_t* dst, uint32_t r0, uint32_t le
     __syncwarp();
 }
 
-// Stores one 18-byte record n = {x, y, z, r | g << 16, b} at slot pos of a
-// 4-byte aligned record array with five stores: four aligned words and one
-// 2-byte store, at the record's end (even slot) or start (odd slot).  The
-// same instructions run for either parity.
-__device__ __forceinline__ void store_record_words(uint8_t* base, uint64_t pos, const uint32_t (&n)[5]) {
-    uint8_t* p = base + pos * 18;
-    const bool odd = (pos & 1) != 0;
+// Stores one 18-byte record n = {x, y, z, r | g << 16, b} at an even address
+// (or at slot pos of a 4-byte aligned record array) with five stores: four
+// aligned words and one 2-byte store, at the record's end or start.  The same
+// instructions run for either parity.
+__device__ __forceinline__ void store_record_at(uint8_t* p, const uint32_t (&n)[5]) {
+    const bool odd = (reinterpret_cast<uintptr_t>(p) & 2u) != 0;
     *reinterpret_cast<uint16_t*>(p + (odd ? 0 : 16)) = (uint16_t)(odd ? n[0] : n[4]);
     uint32_t* q = reinterpret_cast<uint32_t*>(p + (odd ? 2 : 0));
     q[0] = odd ? __funnelshift_r(n[0], n[1], 16) : n[0];
     q[1] = odd ? __funnelshift_r(n[1], n[2], 16) : n[1];
     q[2] = odd ? __funnelshift_r(n[2], n[3], 16) : n[2];
     q[3] = odd ? __funnelshift_r(n[3], n[4], 16) : n[3];
+}
+
+__device__ __forceinline__ void store_record_words(uint8_t* base, uint64_t pos, const uint32_t (&n)[5]) {
+    store_record_at(base + pos * 18, n);
 }
 
 #endif   // __CUDACC__

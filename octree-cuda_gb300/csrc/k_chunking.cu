@@ -28,6 +28,11 @@ namespace {
 constexpr uint32_t kLeafTag = 0x80000000u;
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;   // run key of lanes without a point
 
+// Sample of the cloud's order in the words after the error word: runs and
+// points (order_sample).
+constexpr uint32_t kOrderWord = 4;
+constexpr uint32_t kOrderWarps = 64;
+
 __device__ __forceinline__ void set_error(uint32_t* err, uint32_t bit) {
     atomicOr(err, bit);
 }
@@ -41,10 +46,50 @@ __device__ __forceinline__ void set_error(uint32_t* err, uint32_t bit) {
 // counting: 1024-record tiles, 512 threads
 constexpr uint32_t kCountTile = 1024;
 constexpr uint32_t kCountThreads = 512;
-// distribution: 896-record tiles, 448 threads (three blocks fit one SM's
-// registers)
-constexpr uint32_t kDistTile = 896;
-constexpr uint32_t kDistThreads = 448;
+// Distribution stores each record from its own lane where a leaf's points
+// follow each other in the cloud, and brings a leaf's records of a tile
+// together in shared memory first where they do not (25.8M-point planes, whose
+// points jump between leaves: 1.39 -> 0.88 ms; grouping everything costs the
+// 119.7M-point terrain 2.38 -> 3.4 ms).
+//   kDirect     896-record tiles, 448 threads (three blocks fit one SM's registers)
+//   kGrouped    768-record tiles, one record per thread
+//   kByTile     as kDirect; a round of 448 records is grouped when the runs of
+//               the tile before were short (float records: with 27-byte tiles
+//               its shared memory would take the L1 cache the leaf tags live
+//               in, 2.38 -> 2.76 ms)
+// A sample of the cloud's order (order_sample) chooses kGrouped or the
+// other kernel of the record type.
+enum DistMode : int { kDirect, kGrouped, kByTile };
+__host__ __device__ constexpr uint32_t dist_threads(int mode) { return mode == kGrouped ? 768 : 448; }
+__host__ __device__ constexpr uint32_t dist_tile(int mode) { return mode == kGrouped ? 768 : 896; }
+constexpr uint32_t kGroupRun = 4;   // runs of equal leaves shorter than this on average: grouped
+constexpr uint64_t kGroupMinPoints = 1 << 18;
+constexpr uint32_t kGroupMaxStride = 64;
+
+// Grouping of a round of records (one per thread) by leaf: a hash of the
+// leaves, the byte image of the records in leaf order, and per record in that
+// order its position and word.
+template <int kMode>
+struct GroupSmem {
+    static constexpr uint32_t kRecords = dist_threads(kMode);
+    static constexpr uint32_t kSlots = kMode == kGrouped ? 1024 : 512;
+    static constexpr uint32_t kHashShift = kMode == kGrouped ? 22 : 23;
+    static constexpr uint32_t kImage = kMode == kGrouped ? 20 * 1024 : 11 * 1024;
+    uint32_t key[kSlots];       // leaf + 1, 0 = empty
+    uint32_t count[kSlots];     // records
+    uint32_t first[kSlots];     // their first position
+    uint32_t at[kSlots];        // ... in the image (bytes) << 16 | in leaf order
+    uint8_t level[kSlots];      // the leaf's level
+    uint32_t pos[kRecords];     // in leaf order
+    uint32_t word[kRecords];
+    uint16_t rec[kRecords];
+    uint16_t runs[kRecords];    // slots in use
+    uint32_t warp[32];
+    uint32_t n_runs, bytes, bad;   // bytes: of the whole image
+    uint32_t lead[3];           // runs of the tile (by tile), the one before, the one after
+    uint32_t pad[2];
+    uint8_t image[kImage];      // 16-byte aligned
+};
 
 __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) {
     return (x + a - 1) / a * a;
@@ -470,11 +515,43 @@ __global__ void __launch_bounds__(1024) k_leaf_prep(const uint32_t* __restrict__
     if (threadIdx.x == 0 && running != n_points) set_error(err, kErrTag);
 }
 
+// How far the cloud's order keeps leaves together: runs of points in one block
+// of 16^3 finest cells, about a leaf's size, among 32 consecutive points at
+// kOrderWarps places of the cloud.  Approximate cells do.
+template <bool kF32>
+__device__ __forceinline__ void order_sample(const uint8_t* __restrict__ cloud, uint64_t n, uint32_t stride,
+                                             const CloudGrid& g, uint32_t sample, uint32_t* order) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (n < 32 || sample >= kOrderWarps) return;
+    const uint64_t p = (n - 32) * sample / (kOrderWarps - 1) + lane;
+    constexpr int kWords = kF32 ? 3 : 6;
+    uint32_t w[kWords], block = 0;
+    record_words<kWords>(cloud + p * stride, w);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float v = kF32 ? __uint_as_float(w[a]) : approx_f64(w[kF32 ? 0 : 2 * a], w[kF32 ? 0 : 2 * a + 1]);
+        const float u = fminf(fmaxf(__fmaf_rn(v, g.r[a], g.c[a]), 0.0f), (float)(g.grid - 1));
+        block = (block << 10) | ((uint32_t)u >> 4);
+    }
+    const uint32_t runs = __popc(run_starts(block));
+    if (lane == 0) {
+        atomicAdd(order, runs);
+        atomicAdd(order + 1, 32u);
+    }
+}
+
 // Writes the leaf tag of every occupied finest cell into the cell: one
 // thread per level-1 cell reads its 8 children and, when some of them are
 // occupied and untagged, the nearest tagged ancestor.
 __global__ void k_push_tags(uint32_t* __restrict__ pyr, const uint64_t* __restrict__ loff, uint32_t depth, uint64_t n1,
-                            const uint8_t* __restrict__ occ, uint32_t* err) {
+                            const uint8_t* __restrict__ occ, uint32_t* err, const uint8_t* __restrict__ cloud,
+                            uint64_t n, uint32_t stride, uint32_t float_input, CloudGrid g, uint32_t tag_blocks) {
+    if (blockIdx.x >= tag_blocks) {   // the blocks after those of the tags sample the cloud's order
+        const uint32_t sample = (blockIdx.x - tag_blocks) * (blockDim.x / 32) + threadIdx.x / 32;
+        if (float_input) order_sample<true>(cloud, n, stride, g, sample, err + kOrderWord);
+        else order_sample<false>(cloud, n, stride, g, sample, err + kOrderWord);
+        return;
+    }
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= n1) return;
     if (occ && occ[i >> 3] == 0) return;   // no point in this 64-cell block
@@ -505,6 +582,92 @@ __global__ void k_push_tags(uint32_t* __restrict__ pyr, const uint64_t* __restri
     c[1] = make_uint4(v[4], v[5], v[6], v[7]);
 }
 
+// Reserves every leaf's records of the round with one atomic and lays out the
+// image: a leaf's part starts at the 16-byte phase of its destination.  All
+// threads; starts after a barrier, ends with one.
+template <int kMode>
+__device__ __forceinline__ void group_place(GroupSmem<kMode>& gs, const uint64_t* __restrict__ data_idx, uint32_t* fill,
+                                            uint64_t n) {
+    constexpr uint32_t kGroupSlots = GroupSmem<kMode>::kSlots;
+    static_assert(kGroupSlots <= 2 * dist_threads(kMode), "two slots per thread");
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    uint32_t c[2] = {0, 0}, v[2] = {0, 0}, f[2];
+    if (t < kGroupSlots / 2) {
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j) {
+            c[j] = gs.count[2 * t + j];
+            f[j] = c[j] ? atomicAdd(&fill[gs.key[2 * t + j] - 1], c[j]) : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j) {
+            if (!c[j]) continue;
+            const uint32_t s = 2 * t + j;
+            const uint64_t d = data_idx[gs.key[s] - 1];
+            f[j] += (uint32_t)d;
+            if ((uint64_t)f[j] + c[j] > n) gs.bad = 1;   // only reachable with corrupted input tags
+            gs.first[s] = f[j];
+            gs.level[s] = (uint8_t)(d >> kLeafLevelShift);
+            v[j] = ((((f[j] * 18u) & 15u) + c[j] * 18u + 15u) & ~15u) << 16 | c[j];
+            gs.runs[atomicAdd(&gs.n_runs, 1u)] = (uint16_t)s;
+        }
+    }
+    const uint32_t sum = v[0] + v[1];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) gs.warp[warp] = incl;
+    __syncthreads();
+    uint32_t run = incl - sum;
+    for (uint32_t q = 0; q < kGroupSlots / 64; ++q) run += q < warp ? gs.warp[q] : 0u;
+    if (t < kGroupSlots / 2) {
+        gs.at[2 * t] = run + (((f[0] * 18u) & 15u) << 16);
+        gs.at[2 * t + 1] = run + v[0] + (((f[1] * 18u) & 15u) << 16);
+        if (t == kGroupSlots / 2 - 1) gs.bytes = (run + sum) >> 16;
+    }
+    __syncthreads();
+}
+
+// Copies the image out, a warp per leaf: 16-byte words, and 2-byte words at
+// both ends; then indices and words, neighbouring lanes to neighbouring
+// positions.
+template <int kMode>
+__device__ __forceinline__ void group_store(const GroupSmem<kMode>& gs, uint64_t p0, uint32_t* __restrict__ lut,
+                                            uint32_t* __restrict__ word, uint8_t* __restrict__ rec) {
+    constexpr uint32_t kGroupSlots = GroupSmem<kMode>::kSlots;
+    const uint32_t t = threadIdx.x, lane = t & 31;
+    for (uint32_t r = t >> 5; r < gs.n_runs; r += dist_threads(kMode) / 32) {
+        const uint32_t s = gs.runs[r], a0 = gs.at[s] >> 16, a1 = a0 + gs.count[s] * 18u;
+        uint8_t* out = rec + (uint64_t)gs.first[s] * 18 - a0;   // of image byte 0
+        const uint32_t b0 = (a0 + 15u) & ~15u, b1 = a1 & ~15u;
+        if (b0 < b1) {
+            for (uint32_t i = b0 + 16 * lane; i < b1; i += 512)
+                *reinterpret_cast<uint4*>(out + i) = *reinterpret_cast<const uint4*>(gs.image + i);
+            // up to seven 2-byte words before, up to seven after
+            const uint32_t i = lane < 8 ? a0 + 2 * lane : b1 + 2 * (lane - 8);
+            if (lane < 16 && i < (lane < 8 ? b0 : a1))
+                *reinterpret_cast<uint16_t*>(out + i) = *reinterpret_cast<const uint16_t*>(gs.image + i);
+        } else {
+            const uint32_t i = a0 + 2 * lane;   // at most 30 bytes
+            if (i < a1) *reinterpret_cast<uint16_t*>(out + i) = *reinterpret_cast<const uint16_t*>(gs.image + i);
+        }
+    }
+    const uint32_t last = gs.at[kGroupSlots - 1], total = (last & 0xFFFFu) + gs.count[kGroupSlots - 1];
+    if (t < total) {
+        const uint32_t pos = gs.pos[t];
+        lut[pos] = (uint32_t)(p0 + gs.rec[t]);
+        word[pos] = gs.word[t];
+    }
+}
+
+template <int kMode>
+__device__ __forceinline__ void group_clear(GroupSmem<kMode>& gs) {
+    for (uint32_t i = threadIdx.x; i < GroupSmem<kMode>::kSlots; i += dist_threads(kMode)) gs.key[i] = gs.count[i] = 0;
+    if (threadIdx.x == 0) gs.n_runs = gs.bad = 0;
+}
+
 // K5 (point_distributing.cuh:30-75): every point goes to its leaf's bucket
 // with its LUT entry and 18-byte output record.  The first lane of each run
 // of equal cells reads the cell's leaf tag; the first lane of each run of
@@ -519,20 +682,38 @@ struct FineAxes {
     uint32_t cells;   // finest cells per axis
 };
 
-template <bool kF32, bool kCells>
-__global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* __restrict__ cloud, uint64_t n,
+template <bool kF32, bool kCells, int kMode>
+__global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3)
+    k_distribute(const uint8_t* __restrict__ cloud, uint64_t n,
                                                               uint32_t stride, CloudGrid g, OutParams op, FineAxes fa,
                                                               const uint32_t* __restrict__ pyr0,
                                                               const uint64_t* __restrict__ data_idx, uint32_t* fill,
                                                               uint32_t* __restrict__ lut, uint8_t* __restrict__ rec,
-                                                              uint32_t* __restrict__ frac, uint32_t* err) {
+                                                              uint32_t* __restrict__ frac, uint32_t* err,
+                                                              const uint32_t* __restrict__ order) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const ChunkSmem L = chunk_smem(stride, g.grid, kF32, kDistTile, !kCells);
+    // of the two kernels launched, the one for the order of the points runs
+    if (order && (order[0] * kGroupRun > order[1]) != (kMode == kGrouped)) return;
+    constexpr uint32_t kTile = dist_tile(kMode), kThreads = dist_threads(kMode);
+    const ChunkSmem L = chunk_smem(stride, g.grid, kF32, kTile, !kCells);
     load_tables<kF32>(g, smem, L, !kCells);
+    GroupSmem<kMode>* gs = reinterpret_cast<GroupSmem<kMode>*>(smem + align_up(L.total, 16));
+    if (kMode != kDirect) {   // (tile_loop starts with a barrier)
+        group_clear(*gs);
+        if (threadIdx.x < 3) gs->lead[threadIdx.x] = 0;
+    }
+    uint32_t next_turn = 0;
     const uint32_t lane = threadIdx.x & 31;
-    tile_loop<kDistTile>(cloud, n, stride, smem, L, err, [&](const uint8_t* recs, uint64_t p0, uint32_t cnt) {
+    tile_loop<kTile>(cloud, n, stride, smem, L, err, [&](const uint8_t* recs, uint64_t p0, uint32_t cnt) {
+        bool group = kMode == kGrouped;
+        const uint32_t turn = next_turn;
+        if (kMode == kByTile) {
+            next_turn = turn == 2 ? 0 : turn + 1;
+            group = gs->lead[turn == 0 ? 2 : turn - 1] * kGroupRun > kTile;
+            if (threadIdx.x == 0) gs->lead[next_turn] = 0;
+        }
 #pragma unroll 1
-        for (uint32_t base = 0; base < kDistTile; base += kDistThreads) {
+        for (uint32_t base = 0; base < kTile; base += kThreads) {
             const uint32_t k = base + threadIdx.x;
             constexpr int kWords = kF32 ? 4 : 7;
             uint32_t w[kWords];
@@ -574,24 +755,47 @@ __global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* _
             }
             starts = run_starts(node);
             leader = run_leader(starts);
+            const bool lead = node != kNoKey && lane == leader;
             uint64_t first = 0;   // the leaf's level above kLeafLevelShift
-            if (node != kNoKey && lane == leader) first = data_idx[node] + atomicAdd(&fill[node], run_end(starts) - lane);
-            first = ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(first >> 32), leader) << 32) |
-                    __shfl_sync(0xffffffffu, (uint32_t)first, leader);
+            uint32_t slot = 0, rank = lane - leader;
+            if (kMode == kByTile) {
+                const uint32_t leads = __popc(__ballot_sync(0xffffffffu, lead));
+                if (lane == 0) atomicAdd(&gs->lead[turn], leads);
+            }
+            if (!group) {
+                if (lead) first = data_idx[node] + atomicAdd(&fill[node], run_end(starts) - lane);
+                first = ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(first >> 32), leader) << 32) |
+                        __shfl_sync(0xffffffffu, (uint32_t)first, leader);
+            } else {
+                if (lead) {
+                    slot = (node * 2654435761u) >> GroupSmem<kMode>::kHashShift;
+                    for (uint32_t probe = 0; probe < GroupSmem<kMode>::kSlots; ++probe) {   // fewer leaves than slots
+                        const uint32_t old = atomicCAS(&gs->key[slot], 0u, node + 1);
+                        if (old == 0 || old == node + 1) break;
+                        slot = (slot + 1) % GroupSmem<kMode>::kSlots;
+                    }
+                    rank = atomicAdd(&gs->count[slot], run_end(starts) - lane);
+                }
+                slot = __shfl_sync(0xffffffffu, slot, leader);
+                rank = __shfl_sync(0xffffffffu, rank, leader) + lane - leader;
+                __syncthreads();
+                group_place(*gs, data_idx, fill, n);
+                first = gs->first[slot] | ((uint64_t)gs->level[slot] << kLeafLevelShift);
+            }
             const uint32_t lv = (uint32_t)(first >> kLeafLevelShift);
             first &= (1ull << kLeafLevelShift) - 1;
+            const bool image = group && gs->bytes <= GroupSmem<kMode>::kImage && !gs->bad;
             uint32_t nw[5] = {0, 0, 0, 0, 0};
             bool ok = false;
+            const uint64_t pos = first + rank;
+            uint32_t fw = 0;
             if (node != kNoKey) {
-                const uint64_t pos = first + (lane - leader);
                 if (pos >= n) {   // only reachable with corrupted input tags
                     set_error(err, kErrTag);
                 } else {
                     ok = true;
-                    lut[pos] = (uint32_t)(p0 + k);
                     const uint32_t col = w[kF32 ? 3 : 6];
                     int32_t x, y, z;
-                    uint32_t fw;
                     if (kCells) {
                         x = q[0];
                         y = q[1];
@@ -611,7 +815,6 @@ __global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* _
                         fw = pack_frac(fx, fy, fz);
                     }
                     if (x == kCoordError || y == kCoordError || z == kCoordError) set_error(err, kErrCoordRange);
-                    if (frac) frac[pos] = fw;
                     nw[0] = (uint32_t)x;
                     nw[1] = (uint32_t)y;
                     nw[2] = (uint32_t)z;
@@ -619,11 +822,31 @@ __global__ void __launch_bounds__(kDistThreads, 3) k_distribute(const uint8_t* _
                     nw[4] = (col >> 16) & 0xFFu;
                 }
             }
-            // each lane stores its own record with five stores (staging the
-            // runs of a leaf through shared memory for coalesced stores was
-            // slower: 119.7M-point build 3.00 -> 2.73 ms, 25.8M-point random
-            // planes 2.25 -> 1.32 ms)
-            if (ok) store_record_words(rec, first + (lane - leader), nw);
+            if (!image) {
+                // each lane stores its own record with five stores (staging the
+                // runs of a warp through shared memory for coalesced stores was
+                // slower: 119.7M-point build 3.00 -> 2.73 ms)
+                if (ok) {
+                    lut[pos] = (uint32_t)(p0 + k);
+                    frac[pos] = fw;
+                    store_record_words(rec, pos, nw);
+                }
+            } else {
+                if (ok) {
+                    const uint32_t at = gs->at[slot], i = (at & 0xFFFFu) + rank;
+                    gs->pos[i] = (uint32_t)pos;
+                    gs->word[i] = fw;
+                    gs->rec[i] = (uint16_t)k;
+                    store_record_at(gs->image + (at >> 16) + rank * 18, nw);
+                }
+                __syncthreads();
+                group_store(*gs, p0, lut, frac, rec);
+            }
+            if (group) {
+                __syncthreads();
+                group_clear(*gs);
+                if (kMode == kByTile) __syncthreads();   // another round may follow
+            }
         }
     });
 }
@@ -829,24 +1052,30 @@ int launch_leaf_prep(const uint32_t* n_nodes, const uint16_t* info, const uint32
     return 1;
 }
 
-int launch_push_tags(uint32_t* pyr, const uint64_t* loff_dev, uint32_t depth, uint32_t grid, const uint8_t* occ,
-                     uint32_t* err, cudaStream_t stream) {
-    const uint64_t n1 = (uint64_t)(grid / 2) * (grid / 2) * (grid / 2);
+int launch_push_tags(uint32_t* pyr, const uint64_t* loff_dev, uint32_t depth, const uint8_t* occ, uint32_t* err,
+                     const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
+                     cudaStream_t stream) {
+    const uint64_t n1 = (uint64_t)(g.grid / 2) * (g.grid / 2) * (g.grid / 2);
     if (!n1) return 0;
-    k_push_tags<<<(unsigned)((n1 + 255) / 256), 256, 0, stream>>>(pyr, loff_dev, depth, n1, occ, err);
+    const uint32_t blocks = (uint32_t)((n1 + 255) / 256);
+    k_push_tags<<<blocks + kOrderWarps / 8, 256, 0, stream>>>(pyr, loff_dev, depth, n1, occ, err, cloud, n, stride,
+                                                              float_input, g, blocks);
     return 1;
 }
 
 namespace {
 
-template <bool kF32, bool kCells>
+template <bool kF32, bool kCells, int kMode>
 void distribute_on(const uint8_t* cloud, uint64_t n, uint32_t stride, const CloudGrid& g, const OutParams& out,
                    const FineAxes& fa, const uint32_t* pyr0, const uint64_t* data_idx, uint32_t* fill, uint32_t* lut,
-                   uint8_t* rec, uint32_t* word, uint32_t* err, int num_sms, cudaStream_t stream) {
-    const size_t smem = chunk_smem(stride, g.grid, kF32, kDistTile, !kCells).total;
-    const int grid = chunk_grid_size(k_distribute<kF32, kCells>, kDistThreads, kDistTile, smem, n, num_sms);
-    k_distribute<kF32, kCells><<<grid, kDistThreads, smem, stream>>>(cloud, n, stride, g, out, fa, pyr0, data_idx, fill,
-                                                                     lut, rec, word, err);
+                   uint8_t* rec, uint32_t* word, uint32_t* err, const uint32_t* order, int num_sms,
+                   cudaStream_t stream) {
+    constexpr uint32_t kTile = dist_tile(kMode), kThreads = dist_threads(kMode);
+    const size_t smem = align_up(chunk_smem(stride, g.grid, kF32, kTile, !kCells).total, 16) +
+                        (kMode != kDirect ? sizeof(GroupSmem<kMode>) : 0);
+    const int grid = chunk_grid_size(k_distribute<kF32, kCells, kMode>, kThreads, kTile, smem, n, num_sms);
+    k_distribute<kF32, kCells, kMode><<<grid, kThreads, smem, stream>>>(cloud, n, stride, g, out, fa, pyr0, data_idx,
+                                                                         fill, lut, rec, word, err, order);
 }
 
 }   // namespace
@@ -856,8 +1085,8 @@ int launch_distribute(const uint8_t* cloud, uint64_t n, uint32_t stride, bool fl
                       uint32_t* lut, uint8_t* rec, uint32_t* frac, uint32_t* err, int num_sms,
                       cudaStream_t stream) {
     if (n == 0) return 0;
-    const auto go = float_input ? distribute_on<true, false> : distribute_on<false, false>;
-    go(cloud, n, stride, g, out, FineAxes{}, pyr0, data_idx, fill, lut, rec, frac, err, num_sms, stream);
+    const auto go = float_input ? distribute_on<true, false, kDirect> : distribute_on<false, false, kDirect>;
+    go(cloud, n, stride, g, out, FineAxes{}, pyr0, data_idx, fill, lut, rec, frac, err, nullptr, num_sms, stream);
     return 1;
 }
 
@@ -869,9 +1098,18 @@ int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, b
     FineAxes fa;
     for (int a = 0; a < 3; ++a) fa.ax[a] = fine[a];
     fa.cells = g.grid * 64;   // 2^depth counting cells, each 64 finest cells wide
-    const auto go = float_input ? distribute_on<true, true> : distribute_on<false, true>;
-    go(cloud, n, stride, g, out, fa, pyr0, data_idx, fill, lut, rec, word, err, num_sms, stream);
-    return 1;
+    // records too long for the grouped kernels' shared memory are stored lane
+    // by lane; on a small cloud the second launch costs more than it can give
+    const bool fits = stride <= kGroupMaxStride, both = fits && n >= kGroupMinPoints;
+    const uint32_t* order = both ? err + kOrderWord : nullptr;
+    const auto by_lane = !float_input ? distribute_on<false, true, kDirect>
+                         : fits       ? distribute_on<true, true, kByTile>
+                                      : distribute_on<true, true, kDirect>;
+    by_lane(cloud, n, stride, g, out, fa, pyr0, data_idx, fill, lut, rec, word, err, order, num_sms, stream);
+    if (!both) return 1;
+    const auto grouped = float_input ? distribute_on<true, true, kGrouped> : distribute_on<false, true, kGrouped>;
+    grouped(cloud, n, stride, g, out, fa, pyr0, data_idx, fill, lut, rec, word, err, order, num_sms, stream);
+    return 2;
 }
 
 int launch_place(const uint64_t* src_off, const uint64_t* dst_off, const uint32_t* count, uint32_t n_nodes,

@@ -164,9 +164,11 @@ int launch_leaf_prep(const uint32_t* n_nodes, const uint16_t* info, const uint32
                      uint64_t n_points, uint32_t* err, cudaStream_t stream);
 
 // Writes each occupied finest-level cell's leaf tag into the cell (after
-// launch_leaf_prep), so that distribution finds a point's leaf in one read.
-int launch_push_tags(uint32_t* pyr, const uint64_t* level_off_dev, uint32_t depth, uint32_t grid, const uint8_t* occ,
-                     uint32_t* err, cudaStream_t stream);
+// launch_leaf_prep), so that distribution finds a point's leaf in one read;
+// samples the order of the cloud's points for launch_distribute_cells.
+int launch_push_tags(uint32_t* pyr, const uint64_t* level_off_dev, uint32_t depth, const uint8_t* occ, uint32_t* err,
+                     const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
+                     cudaStream_t stream);
 
 // Level of a leaf beside its first record in data_idx (launch_leaf_prep).
 constexpr uint32_t kLeafLevelShift = 56;
