@@ -1079,6 +1079,7 @@ void Builder::subsample() {
     std::vector<uint32_t> oct_unit;          // spread levels, per node and octant
     std::vector<size_t> oct_first(depth_ + 2, 0);
     uint64_t map_words = 0;                  // of the largest spread level
+    std::vector<uint32_t> mean_candidates(depth_ + 2, 0);   // per unit, inner children taken at 16384 points at most
     uint32_t s_log2 = 0;
     while ((1u << s_log2) < S) ++s_log2;
     if (octants) {
@@ -1095,7 +1096,7 @@ void Builder::subsample() {
             spread[l] = few && inter && whole && (weighted || whole <= (uint64_t)num_sms_);
             oct_first[l] = oct_unit.size();
             if (spread[l]) oct_unit.resize(oct_unit.size() + 8 * (size_t)(level_first[l + 1] - level_first[l]), ~0u);
-            uint64_t words = 0;
+            uint64_t words = 0, candidates = 0;
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
                 const NodeHost& v = nodes_[order[k]];
                 uint32_t c = v.child_first, number = 0, q0 = 0;
@@ -1104,6 +1105,7 @@ void Builder::subsample() {
                     const uint32_t ci = c++;
                     const NodeHost& ch = nodes_[ci];
                     const bool split = few && ch.internal && out_bound[ci] > 4096;
+                    candidates += ch.internal ? std::min<uint64_t>(out_bound[ci], 16384) : ch.points;
                     if (split) {
                         any_split[l] = 1;
                         table[k].child_kind |= 1u << (16 + s);
@@ -1129,6 +1131,8 @@ void Builder::subsample() {
                 }
                 units.back().flags |= 1u << 9;
             }
+            const uint64_t count = units.size() - unit_first[l];
+            if (count) mean_candidates[l] = (uint32_t)(candidates / count);
             if (words * 4 > map_room) spread[l] = 0;
             if (spread[l]) map_words = std::max(map_words, words);
         }
@@ -1350,7 +1354,7 @@ void Builder::subsample() {
                 u.csr_pts = csr_pts_.as<float4>();
                 u.ticket = reinterpret_cast<uint32_t*>(sync + 128) + l;
                 u.err = err_.as<uint32_t>();
-                launches_ += launch_units_level(u, mode, any_split[l], num_sms_, stream_);
+                launches_ += launch_units_level(u, mode, mean_candidates[l], any_split[l], num_sms_, stream_);
                 char mark[32];
                 std::snprintf(mark, sizeof mark, "sub_l%u", l);
                 stage_mark(mark);

@@ -44,12 +44,10 @@ namespace oc {
 
 namespace {
 
-#ifndef OC_UNIT_THREADS
-#define OC_UNIT_THREADS 512
-#define OC_UNIT_BLOCKS 2
-#endif
-constexpr int kUnitThreads = OC_UNIT_THREADS;
-constexpr int kUnitBlocks = OC_UNIT_BLOCKS;   // per SM
+// Blocks of a level (T threads): two of 512 per SM hide each other's barriers;
+// one of 1024 has the whole shared memory for its unit's cells; two of 768 for
+// distance weighting, whose emit runs on instructions and loads alone.
+constexpr int unit_blocks(int T) { return T == 1024 ? 1 : 2; }
 constexpr uint32_t kFieldBits = 7;   // coordinates of a cell word: x | y << 7 | z << 14
 
 __device__ __forceinline__ uint32_t fields(uint32_t x, uint32_t y, uint32_t z) {
@@ -194,12 +192,10 @@ __host__ __device__ constexpr uint32_t cell_bytes(int color, bool random) {
 }
 
 // Distance weighting: the point ranges a group of lanes walks for its cell, as {end in the cell's list, first point - begin in the list}.
-#ifndef OC_WEIGHT_LANES
-#define OC_WEIGHT_LANES 4
-#endif
-constexpr uint32_t kWeightLanes = OC_WEIGHT_LANES;   // per cell
+constexpr uint32_t kWeightLanes = 4;   // per cell
+constexpr int kWeightThreads = 768;
 struct WeightShared {
-    uint2 rows[kUnitThreads / kWeightLanes][9];
+    uint2 rows[kWeightThreads / kWeightLanes][9];
 };
 
 // Node-grid cell of a candidate without the proof, as coordinates; ~0 when
@@ -323,12 +319,11 @@ __device__ __forceinline__ uint32_t weighted_mean(uint64_t sum, uint64_t weight)
 // hold.  (A lane per cell, or lanes sharing each neighbour's points, waits
 // for the longest list: the weight of a pair costs about 45 instructions.)
 // Colours are of 8 bits here: the cloud's, or means of those.
-template <bool kRandom, int kB, bool kLocal, class Pre>
+template <int T, bool kRandom, int kB, bool kLocal, class Pre>
 __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box,
                                               const uint64_t* l_key, const uint32_t* l_word, uint32_t* l_cnt,
                                               uint32_t cells, const int (&keep)[4], uint64_t so, uint64_t oo,
                                               WeightShared& ws) {
-    constexpr int T = kUnitThreads;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Unit& un = sh.un;
     const uint32_t* l_idx = reinterpret_cast<const uint32_t*>(l_key);
@@ -533,11 +528,10 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
 // sums beyond 16 bits) in the staging arrays and the level's scratch, reached
 // by reductions.  keep: the cells of this thread's first four candidates.
 // Returns false (every thread alike) when a local unit has to be redone.
-template <int kColor, bool kRandom, int kB, bool kLocal, class Pre>
+template <int T, int kColor, bool kRandom, int kB, bool kLocal, class Pre>
 __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box, uint32_t* pool,
                                            uint32_t ui, uint32_t cells, const int (&keep)[4], uint32_t claim,
                                            uint32_t included, bool placed, WeightShared* ws) {
-    constexpr int T = kUnitThreads;
     constexpr bool averaged = kColor == 1 || kColor == 2, weighted = kColor == 3;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Unit& un = sh.un;
@@ -709,7 +703,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
     const uint64_t* g_packed = a.sum + so;
     const uint32_t m0 = box.m0(), open = un.open;
     if constexpr (weighted) {
-        unit_weighted<kRandom, kB, kLocal, Pre>(a, sh, box, l_key, l_word, l_cnt, cells, keep, so, oo, *ws);
+        unit_weighted<T, kRandom, kB, kLocal, Pre>(a, sh, box, l_key, l_word, l_cnt, cells, keep, so, oo, *ws);
     } else {
         for (uint32_t r0 = warp * 32; r0 < cells; r0 += T) {
             const uint32_t r = r0 + lane;
@@ -752,11 +746,24 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
     return true;
 }
 
+// unit_cells on global memory out of line, for blocks of 1024 threads, which
+// seldom need it: inlined, its registers weigh on the other variant's (level
+// 4 of the 119.7M-point build 1.34 -> 1.27 ms; two blocks of 512, which
+// need it often, lose by it: level 1 0.84 -> 1.13 ms).
+template <int T, int kColor, bool kRandom, int kB, class Pre>
+__device__ __noinline__ void unit_cells_global(const UnitLevelArgs& a, BlockShared& sh, const uint32_t* bm,
+                                               const Pre* pre, uint32_t b, uint32_t ui, uint32_t cells, int4 keep4,
+                                               uint32_t claim, uint32_t included, bool placed) {
+    const int keep[4] = {keep4.x, keep4.y, keep4.z, keep4.w};
+    const Box<kB, Pre> box{bm, pre, b};
+    unit_cells<T, kColor, kRandom, kB, false, Pre>(a, sh, box, nullptr, ui, cells, keep, claim, included, placed,
+                                                   nullptr);
+}
+
 // One unit: pass A, ranks, then its cells.
-template <int kColor, bool kRandom, int kB, class Pre>
+template <int T, int kColor, bool kRandom, int kB, class Pre>
 __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh, uint32_t* bm, uint32_t ui,
                                          WeightShared* ws) {
-    constexpr int T = kUnitThreads;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Unit& un = sh.un;
     const uint32_t b = kB ? (uint32_t)kB : un.b;
@@ -886,18 +893,33 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
     const uint32_t room = a.smem_words * 4 - (uint32_t)((pool - bm) * 4);
     bool placed = false;
     if (sizeof(Pre) == 2 && cells * cell_bytes(kColor, kRandom) <= room) {
-        if (unit_cells<kColor, kRandom, kB, true, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, false, ws)) return;
+        if (unit_cells<T, kColor, kRandom, kB, true, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, false, ws)) return;
         placed = true;
         __syncthreads();
     }
-    unit_cells<kColor, kRandom, kB, false, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, placed, ws);
+    if constexpr (T == 1024)
+        unit_cells_global<T, kColor, kRandom, kB, Pre>(a, sh, bm, pre, b, ui, cells,
+                                                       make_int4(keep[0], keep[1], keep[2], keep[3]), claim, included,
+                                                       placed);
+    else
+        unit_cells<T, kColor, kRandom, kB, false, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, placed, ws);
+}
+
+// Units of other kinds than the most frequent one, out of line for blocks of
+// 1024 (levels 1 and 4 of 119.7M points 822 -> 778 and 1378 -> 1256 us).
+template <int T, int kColor, bool kRandom>
+__device__ __noinline__ void unit_run_other(const UnitLevelArgs& a, BlockShared& sh, uint32_t* bm, uint32_t ui,
+                                            WeightShared* ws) {
+    if (sh.un.b == 6) unit_run<T, kColor, kRandom, 6, uint32_t>(a, sh, bm, ui, ws);
+    else if (sh.un.b == 5) unit_run<T, kColor, kRandom, 5, uint16_t>(a, sh, bm, ui, ws);
+    else unit_run<T, kColor, kRandom, 0, uint16_t>(a, sh, bm, ui, ws);
 }
 
 // kColor: 0 raw colour, 1 intra-cell, 2 inter-cell, 3 distance-weighted.  An
 // inter-cell or weighted colour whose neighbourhood reaches into other units keeps its sum and goes to its
 // node's face list (k_faces).
-template <int kColor, bool kRandom>
-__global__ void __launch_bounds__(kUnitThreads, kUnitBlocks) k_units(const __grid_constant__ UnitLevelArgs a) {
+template <int T, int kColor, bool kRandom>
+__global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_constant__ UnitLevelArgs a) {
     extern __shared__ __align__(16) uint32_t dyn[];
     __shared__ BlockShared sh;
     const uint32_t tid = threadIdx.x;
@@ -920,10 +942,15 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitBlocks) k_units(const __gri
         if (ui >= a.n_units) break;
         // (the weighted lists follow the pool)
         WeightShared* ws = reinterpret_cast<WeightShared*>(dyn + a.smem_words);
-        if (sh.un.b == 6 && sh.un.cnt > 65535) unit_run<kColor, kRandom, 6, uint32_t>(a, sh, dyn, ui, ws);
-        else if (sh.un.b == 6) unit_run<kColor, kRandom, 6, uint16_t>(a, sh, dyn, ui, ws);
-        else if (sh.un.b == 5) unit_run<kColor, kRandom, 5, uint16_t>(a, sh, dyn, ui, ws);
-        else unit_run<kColor, kRandom, 0, uint16_t>(a, sh, dyn, ui, ws);
+        if constexpr (T == 1024) {
+            if (sh.un.b == 6 && sh.un.cnt <= 65535) unit_run<T, kColor, kRandom, 6, uint16_t>(a, sh, dyn, ui, ws);
+            else unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
+            continue;
+        }
+        if (sh.un.b == 6 && sh.un.cnt > 65535) unit_run<T, kColor, kRandom, 6, uint32_t>(a, sh, dyn, ui, ws);
+        else if (sh.un.b == 6) unit_run<T, kColor, kRandom, 6, uint16_t>(a, sh, dyn, ui, ws);
+        else if (sh.un.b == 5) unit_run<T, kColor, kRandom, 5, uint16_t>(a, sh, dyn, ui, ws);
+        else unit_run<T, kColor, kRandom, 0, uint16_t>(a, sh, dyn, ui, ws);
     }
 }
 
@@ -1359,15 +1386,36 @@ int blocks_per_sm(const void* kernel, int threads, size_t smem) {
 
 // Shared memory of a unit block: an equal share of an SM's 227 KB, less the
 // static part and the 1 KB the system takes per block.
-template <int kColor, bool kRandom>
-void launch_units(UnitLevelArgs a, int num_sms, cudaStream_t stream) {
-    const size_t smem = (227 * 1024 / kUnitBlocks - 1024 - sizeof(BlockShared)) & ~(size_t)127;
+template <int T, int kColor, bool kRandom>
+void launch_units_of(UnitLevelArgs a, int num_sms, cudaStream_t stream) {
+    const size_t smem = (227 * 1024 / unit_blocks(T) - 1024 - sizeof(BlockShared)) & ~(size_t)127;
     a.smem_words = (uint32_t)((smem - (kColor == 3 ? sizeof(WeightShared) : 0)) / 4) & ~3u;
-    auto kern = k_units<kColor, kRandom>;
+    auto kern = k_units<T, kColor, kRandom>;
     allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
-    const uint64_t fit = (uint64_t)std::max(num_sms, 1) *
-                         blocks_per_sm(reinterpret_cast<const void*>(kern), kUnitThreads, smem);
-    kern<<<(unsigned)std::min<uint64_t>(a.n_units, fit), kUnitThreads, smem, stream>>>(a);
+    const uint64_t fit =
+        (uint64_t)std::max(num_sms, 1) * blocks_per_sm(reinterpret_cast<const void*>(kern), T, smem);
+    kern<<<(unsigned)std::min<uint64_t>(a.n_units, fit), T, smem, stream>>>(a);
+}
+
+// Blocks of 1024 where every unit has an SM of its own, and on levels of many
+// units whose cells would mostly not fit in half an SM's shared memory
+// (candidates x bytes per cell; a unit that does not fit works in global
+// memory).  Levels 8 and 9 of the 25.8M-point random planes 106 -> 86 and
+// 115 -> 68 us, level 5 (104 KB) 481 -> 453; 12.3M-point terrain, level 4
+// (140 KB) 330 -> 278 us; but 119.7M points, level 3 (74 KB): 2.42 ms with two
+// blocks, 2.82 with one.  With 1 to 3 units per SM two blocks are the better
+// balance (level of 294 units: 135 us against 172).
+template <int kColor, bool kRandom>
+void launch_units(const UnitLevelArgs& a, uint32_t mean_candidates, int num_sms, cudaStream_t stream) {
+    if constexpr (kColor == 3) {
+        launch_units_of<kWeightThreads, kColor, kRandom>(a, num_sms, stream);
+    } else {
+        const uint64_t sms = (uint64_t)std::max(num_sms, 1);
+        const bool wide = a.n_units <= sms ||
+                          (a.n_units >= 3 * sms && (uint64_t)mean_candidates * cell_bytes(kColor, kRandom) > 78 * 1024);
+        if (wide) launch_units_of<1024, kColor, kRandom>(a, num_sms, stream);
+        else launch_units_of<512, kColor, kRandom>(a, num_sms, stream);
+    }
 }
 
 }   // namespace
@@ -1405,29 +1453,29 @@ void launch_colours(const UnitLevelArgs& a, bool any_split, int num_sms, cudaStr
 
 }   // namespace
 
-int launch_units_level(const UnitLevelArgs& a, uint32_t mode, bool any_split, int num_sms,
+int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_candidates, bool any_split, int num_sms,
                        cudaStream_t stream) {
     if (!a.n_units) return 0;
     const bool random = (mode & kModeRandom) != 0;
     if (mode & kModeIntra) {
-        if (random) launch_units<1, true>(a, num_sms, stream);
-        else launch_units<1, false>(a, num_sms, stream);
+        if (random) launch_units<1, true>(a, mean_candidates, num_sms, stream);
+        else launch_units<1, false>(a, mean_candidates, num_sms, stream);
         return 1;
     }
     if ((mode & kModeInter) && (mode & kModeWeight)) {
-        if (random) launch_units<3, true>(a, num_sms, stream);
-        else launch_units<3, false>(a, num_sms, stream);
+        if (random) launch_units<3, true>(a, mean_candidates, num_sms, stream);
+        else launch_units<3, false>(a, mean_candidates, num_sms, stream);
         launch_colours<3>(a, any_split, num_sms, stream);
         return 2;
     }
     if (mode & kModeInter) {
-        if (random) launch_units<2, true>(a, num_sms, stream);
-        else launch_units<2, false>(a, num_sms, stream);
+        if (random) launch_units<2, true>(a, mean_candidates, num_sms, stream);
+        else launch_units<2, false>(a, mean_candidates, num_sms, stream);
         launch_colours<2>(a, any_split, num_sms, stream);
         return 2;
     }
-    if (random) launch_units<0, true>(a, num_sms, stream);
-    else launch_units<0, false>(a, num_sms, stream);
+    if (random) launch_units<0, true>(a, mean_candidates, num_sms, stream);
+    else launch_units<0, false>(a, mean_candidates, num_sms, stream);
     return 1;
 }
 

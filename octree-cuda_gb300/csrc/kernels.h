@@ -366,9 +366,9 @@ struct UnitLevelArgs {
     uint32_t* err;
 };
 
-// any_split: some child of the level is split in parts.  Inter-cell averaging takes two
+// mean_candidates: about, per unit.  any_split: some child of the level is split in parts.  Inter-cell averaging takes two
 // launches: the units, then what their outermost cells get from other units.
-int launch_units_level(const UnitLevelArgs& a, uint32_t mode, bool any_split, int num_sms,
+int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_candidates, bool any_split, int num_sms,
                        cudaStream_t stream);
 
 // The records of the internal nodes at their post-order positions, made from
