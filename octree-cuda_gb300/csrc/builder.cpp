@@ -718,6 +718,14 @@ CloudGrid Builder::cloud_grid() const {
     return g;
 }
 
+FixedGrid Builder::fixed_grid() const {
+    FixedGrid f;
+    for (int a = 0; a < 3; ++a)
+        f.ax[a] = make_fixed_axis(cfg_.bb_min[a], cfg_.bb_max[0] - cfg_.bb_min[0], 1.0 / cfg_.scale[a], depth_);
+    f.cells = 64u << depth_;
+    return f;
+}
+
 // Sparse clouds (at most one point per 16 finest cells) flag the 64-cell
 // blocks of the finest level they touch (one byte per block): counting sets
 // the flags, the pyramid and the tag push skip unflagged blocks, and the build
@@ -825,9 +833,7 @@ void Builder::generate() {
                                   cloud_.as<uint8_t>(), cfg_.n, cfg_.stride, f32, g, stream_);
     leaf_cells_ = octant_subsampling();
     if (leaf_cells_) {
-        FineAxis fine[3];
-        for (int a = 0; a < 3; ++a) fine[a] = make_fine_axis(cfg_.bb_min[a], cfg_.bb_max[0] - cfg_.bb_min[0], depth_);
-        launches_ += launch_distribute_cells(cloud_.as<uint8_t>(), cfg_.n, cfg_.stride, f32, g, op, fine,
+        launches_ += launch_distribute_cells(cloud_.as<uint8_t>(), cfg_.n, cfg_.stride, f32, g, op, fixed_grid(),
                                              pyr_.as<uint32_t>(), data_idx_.as<uint64_t>(), fill_.as<uint32_t>(),
                                              lut_.as<uint32_t>(), rec_.as<uint8_t>(), leaf_frac_.as<uint32_t>(),
                                              err_.as<uint32_t>(), num_sms_, stream_);
@@ -1421,7 +1427,7 @@ void Builder::subsample() {
         if (octants)
             launches_ += launch_place_units(place_src_.as<uint64_t>(), place_dst_.as<uint64_t>(),
                                             place_cnt_.as<uint32_t>(), n_internal, cfg_.n, out_total_.as<uint64_t>(),
-                                            op, cloud_.as<uint8_t>(), cfg_.stride, cfg_.cloud_type == 0, averaged,
+                                            op, fixed_grid(), cloud_.as<uint8_t>(), cfg_.stride, cfg_.cloud_type == 0, averaged,
                                             stage_lut_.as<uint32_t>(), stage_rec_.as<uint64_t>(), rec_.as<uint8_t>(),
                                             err_.as<uint32_t>(), num_sms_, stream_);
         else

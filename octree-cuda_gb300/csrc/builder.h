@@ -243,6 +243,7 @@ private:
     void build_tree_host();
     void fill_cell_tables();
     CloudGrid cloud_grid() const;
+    FixedGrid fixed_grid() const;
     bool sparse_cloud() const;
     void clear_for_count(bool sparse);
     void params_writable();

@@ -5,7 +5,7 @@
 // kernel_helpers.cuh:10-25) and quantises output coordinates the same way
 // (point_distributing.cuh:245-247).  GB300's binary64 issue rate is a small
 // fraction of its binary32 rate, so every stage evaluates those formulas with
-// an fp32 (or float-float) estimate plus a rigorous error bound, and only
+// an fp32 estimate or in fixed point (fixed_axis.h) with a rigorous error bound, and only
 // falls back to the binary64 expression when the estimate lies within that
 // bound of a cell boundary.  The result is always the binary64 result.
 #pragma once
@@ -14,6 +14,8 @@
 
 #include <cstdint>
 #include <cstring>
+
+#include "fixed_axis.h"
 
 namespace oc {
 
@@ -66,30 +68,6 @@ __host__ __device__ inline OutAxis make_out_axis(double mn, double sf) {
 }
 
 constexpr int32_t kCoordError = (int32_t)0x80000000;
-
-// Finest subsampling cells along one axis of the cloud's cube: those of a
-// 128^3 grid in a node of level 1 (see out_coord_cell).
-struct FineAxis {
-    float b_hi, b_lo;   // cells per coordinate unit
-    float e;            // 2^-22 + what binary64 rounding at any level is worth, in cells
-};
-
-// mn: box minimum, side: cube side, depth: tree depth.  A node's box minimum
-// comes from at most `depth` additions of binary64, its cell size from two more
-// roundings of numbers up to M = max(|mn|, |mn + side|, side), and the formula
-// adds the rounding of p - min and of the quotient: together under
-// (depth + 8) * 2^-52 * M in coordinate units; twice that is allowed for.
-inline FineAxis make_fine_axis(double mn, double side, uint32_t depth) {
-    FineAxis f;
-    const double cells = (double)(64ull << depth);
-    const double B = cells / side;
-    f.b_hi = (float)B;
-    f.b_lo = (float)(B - (double)f.b_hi);
-    const double a = mn < 0 ? -mn : mn, z = mn + side < 0 ? -(mn + side) : mn + side;
-    const double M = a > z ? (a > side ? a : side) : (z > side ? z : side);
-    f.e = (float)((2.384185791015625e-07 + (depth + 8.0) * 4.440892098500626e-16 * M * B) * 1.000001);   // 2^-22, 2^-51
-    return f;
-}
 
 // ---------------------------------------------------------------------------
 // Morton order with x as the most significant bit of every triple: the child
@@ -332,12 +310,6 @@ __device__ __forceinline__ int32_t out_coord_frac(const Coord& c, const OutAxis&
     return exact_out_coord(exact_value<kFloatInput>(c), o.mn, o.sf);
 }
 
-template <bool kFloatInput>
-__device__ __forceinline__ int32_t out_coord(const Coord& c, const OutAxis& o) {
-    uint32_t unused;
-    return out_coord_frac<kFloatInput>(c, o, unused);
-}
-
 // Sub-step word of an output record: bits 0-9, 10-19, 20-29 the x, y, z
 // fraction bins of out_coord_frac, bit 31 set when all three are known.
 __device__ __forceinline__ uint32_t pack_frac(uint32_t fx, uint32_t fy, uint32_t fz) {
@@ -351,52 +323,36 @@ __device__ __forceinline__ uint32_t pack_frac(uint32_t fx, uint32_t fy, uint32_t
 
 constexpr uint32_t kSafeWord = 0x80000000u;
 
-// Quantised output coordinate (as out_coord) and cell of the finest grid of
-// one axis, which share the exact difference to the box minimum.  `safe` is
-// set when the cell-unit position U = (p - min) * B lies at least E from every
-// integer and inside [0, cells): E covers the rounding of this evaluation
-// (the first two terms, as in out_coord_frac) and, in f.e, what the binary64
-// formula of any level can differ from U, so that every level's formula and
-// the counting grid's give the cell (int)U or an ancestor of it.
-template <bool kFloatInput>
-__device__ __forceinline__ int32_t out_coord_cell(const Coord& c, const OutAxis& o, const FineAxis& f, uint32_t cells,
-                                                  uint32_t& cell, bool& safe) {
-    safe = false;
-    cell = 0;
-    if (kFloatInput || c.ok) {
-        // s + e1 = hi - m_hi exactly (Knuth TwoSum)
-        const float nm = -o.m_hi;
-        const float s = __fadd_rn(c.hi, nm);
-        const float bb = __fsub_rn(s, c.hi);
-        const float e1 = __fadd_rn(__fsub_rn(c.hi, __fsub_rn(s, bb)), __fsub_rn(nm, bb));
-        const float lo2 = __fsub_rn(__fadd_rn(e1, c.lo), o.m_lo);
-        const float reach = __fadd_rn(fabsf(c.hi), fabsf(o.m_hi));
-        {
-            const float ph = __fmul_rn(s, f.b_hi);
-            const float pl = __fmaf_rn(s, f.b_lo, __fmaf_rn(lo2, f.b_hi, __fmaf_rn(s, f.b_hi, -ph)));
-            const float fl = floorf(ph);
-            const float frac = __fadd_rn(__fsub_rn(ph, fl), pl);
-            const float g = floorf(frac);
-            const float rem = __fsub_rn(frac, g);
-            const float E = __fmaf_rn(__fmaf_rn(reach, f.b_hi, fabsf(ph)), 2.2737367544323206e-13f, f.e);   // 2^-42
-            if (fabsf(ph) < 1.0e9f && rem >= E && rem <= __fsub_rn(1.0f, E)) {
-                cell = (uint32_t)((int32_t)fl + (int32_t)g);
-                safe = cell < cells;
-            }
-        }
-        const float ph = __fmul_rn(s, o.sf_hi);
-        const float pl = __fmaf_rn(s, o.sf_lo, __fmaf_rn(lo2, o.sf_hi, __fmaf_rn(s, o.sf_hi, -ph)));
-        if (fabsf(ph) < 1.0e9f) {
-            const float fl = floorf(ph);
-            const float frac = __fadd_rn(__fsub_rn(ph, fl), pl);
-            const float g = floorf(frac);
-            const float rem = __fsub_rn(frac, g);
-            const float E = __fmaf_rn(__fmaf_rn(reach, fabsf(o.sf_hi), fabsf(ph)), 2.2737367544323206e-13f,
-                                      2.384185791015625e-07f);   // 2^-42, 2^-22
-            if (rem >= E && rem <= __fsub_rn(1.0f, E)) return (int32_t)fl + (int32_t)g;
-        }
+// Axis k of a cloud point from its words, as binary64.
+template <bool kFloatInput, int kWords>
+__device__ __forceinline__ double word_coord(const uint32_t (&w)[kWords], int k) {
+    return kFloatInput ? widen_bits(w[k]) : __hiloint2double((int)w[2 * k + 1], (int)w[2 * k]);
+}
+
+// The same where the value itself matters (denormals, infinity, NaN).
+template <bool kFloatInput, int kWords>
+__device__ __forceinline__ double word_coord_exact(const uint32_t (&w)[kWords], int k) {
+    return kFloatInput ? (double)__uint_as_float(w[k]) : __hiloint2double((int)w[2 * k + 1], (int)w[2 * k]);
+}
+
+// Quantised output coordinates of a cloud point: (int32_t)floor((p - min) * sf)
+// in binary64, kCoordError outside int32.
+template <bool kFloatInput, int kWords>
+__device__ __forceinline__ void fixed_out_coords(const uint32_t (&w)[kWords], const FixedGrid& f, const OutAxis (&o)[3],
+                                                 uint32_t* out) {
+    bool all = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        uint64_t d;
+        bool proven;
+        all &= fixed_difference(word_coord<kFloatInput>(w, k), f.ax[k].o, d);
+        out[k] = fixed_units(d, f.ax[k].out, proven);
+        all &= proven && (int32_t)out[k] >= 0;
     }
-    return exact_out_coord(exact_value<kFloatInput>(c), o.mn, o.sf);
+    if (all) return;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        out[k] = (uint32_t)exact_out_coord(word_coord_exact<kFloatInput>(w, k), o[k].mn, o[k].sf);
 }
 
 // ---------------------------------------------------------------------------
@@ -529,7 +485,7 @@ __device__ __forceinline__ void load_point(const uint8_t* rec, Coord c[3], uint3
 // where the lanes of a warp read records far apart, the load units work per
 // word and lane (a 27-byte record by load_point takes five).
 template <bool kFloatInput, bool kColour>
-__device__ __forceinline__ void gather_point(const uint8_t* rec, Coord c[3], uint32_t col[3]) {
+__device__ __forceinline__ void gather_words(const uint8_t* rec, uint32_t (&r)[kFloatInput ? 4 : 7]) {
     constexpr uint32_t kBytes = (kFloatInput ? 12u : 24u) + (kColour ? 3u : 0u);
     constexpr int kWords = kFloatInput ? 4 : 7;
     const uintptr_t addr = reinterpret_cast<uintptr_t>(rec);
@@ -539,7 +495,7 @@ __device__ __forceinline__ void gather_point(const uint8_t* rec, Coord c[3], uin
     const uint4 v1 = o + kBytes > 16 ? q[1] : make_uint4(0, 0, 0, 0);
     const uint4 v2 = o + kBytes > 32 ? q[2] : make_uint4(0, 0, 0, 0);
     const uint32_t w[12] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w};
-    uint32_t a[kWords + 2], r[kWords];   // shifted by two words, then one, then bytes
+    uint32_t a[kWords + 2];   // shifted by two words, then one, then bytes
 #pragma unroll
     for (int j = 0; j < kWords + 2; ++j) a[j] = (o & 8) ? w[j + 2 < 12 ? j + 2 : 11] : w[j];
 #pragma unroll
@@ -547,6 +503,13 @@ __device__ __forceinline__ void gather_point(const uint8_t* rec, Coord c[3], uin
         const uint32_t lo = (o & 4) ? a[j + 1] : a[j], hi = (o & 4) ? a[j + 2] : a[j + 1];
         r[j] = __funnelshift_r(lo, hi, (o & 3u) * 8u);
     }
+}
+
+template <bool kFloatInput, bool kColour>
+__device__ __forceinline__ void gather_point(const uint8_t* rec, Coord c[3], uint32_t col[3]) {
+    constexpr int kWords = kFloatInput ? 4 : 7;
+    uint32_t r[kWords];
+    gather_words<kFloatInput, kColour>(rec, r);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
         c[k] = kFloatInput ? coord_f32(__uint_as_float(r[k]))

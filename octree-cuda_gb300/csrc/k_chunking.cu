@@ -676,16 +676,17 @@ __device__ __forceinline__ void group_clear(GroupSmem<kMode>& gs) {
 // room for two: 119.7M-point build 2.73 -> 2.56 ms).
 // kCells: the cell words of octant subsampling instead of sub-step words.  The
 // proven finest cell gives the counting cell as well (its upper bits), so the
-// boundary-key lookup is left out; an unproven axis is evaluated in binary64.
-struct FineAxes {
-    FineAxis ax[3];
-    uint32_t cells;   // finest cells per axis
-};
-
+// boundary-key lookup is left out; an unproven point is evaluated in binary64.
+// Positions are in fixed point: the kernel is bound by the issue of
+// instructions (70% of the slots), and with float-float positions a third of
+// its 490 per point were these (119.7M binary64 points 2.42 -> 2.05 ms, 12.3M
+// 0.263 -> 0.229 ms).  Counting, which waits for its atomics, gains nothing by
+// them and keeps the boundary keys (0.90 ms either way).
 template <bool kF32, bool kCells, int kMode>
 __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3)
     k_distribute(const uint8_t* __restrict__ cloud, uint64_t n,
-                                                              uint32_t stride, CloudGrid g, OutParams op, FineAxes fa,
+                                                              uint32_t stride, CloudGrid g, OutParams op,
+                                                              const __grid_constant__ FixedGrid fg,
                                                               const uint32_t* __restrict__ pyr0,
                                                               const uint64_t* __restrict__ data_idx, uint32_t* fill,
                                                               uint32_t* __restrict__ lut, uint8_t* __restrict__ rec,
@@ -720,22 +721,31 @@ __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3
             uint32_t m = kNoKey;
             int32_t q[3];      // kCells: output coordinates, finest cells, colour
             uint32_t fine[3];
-            bool proven = true;
+            bool proven = true, known = true;   // cells, output coordinates
             if (k < cnt) {
                 record_words<kWords>(recs + (uint64_t)k * stride, w);
                 int cell[3];
                 if (kCells) {
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        const Coord c = kF32 ? coord_f32(__uint_as_float(w[a]))
-                                             : coord_f64(__hiloint2double((int)w[2 * a + 1], (int)w[2 * a]));
-                        bool safe;
-                        q[a] = out_coord_cell<kF32>(c, op.ax[a], fa.ax[a], fa.cells, fine[a], safe);
+                        uint64_t d;
+                        bool exact_cell, exact_out;
+                        const bool in = fixed_difference(word_coord<kF32>(w, a), fg.ax[a].o, d);
+                        fine[a] = fixed_units(d, fg.ax[a].cell, exact_cell);
+                        q[a] = (int32_t)fixed_units(d, fg.ax[a].out, exact_out);
                         cell[a] = (int)(fine[a] >> 6);
-                        if (!safe) {
-                            proven = false;
-                            cell[a] = exact_axis_cell(exact_value<kF32>(c), g.ax[a].mn, g.ax[a].t, g.grid);
-                        }
+                        proven &= in && exact_cell && fine[a] < fg.cells;
+                        known &= in && exact_out && q[a] >= 0;
+                    }
+                    if (!proven) {
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+                            cell[a] = exact_axis_cell(word_coord_exact<kF32>(w, a), g.ax[a].mn, g.ax[a].t, g.grid);
+                    }
+                    if (!known) {
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+                            q[a] = exact_out_coord(word_coord_exact<kF32>(w, a), op.ax[a].mn, op.ax[a].sf);
                     }
                     if ((cell[0] | cell[1] | cell[2]) >= 0) m = cell_morton(cell, smem, L);
                     else set_error(err, kErrBelowBox);
@@ -1067,14 +1077,14 @@ namespace {
 
 template <bool kF32, bool kCells, int kMode>
 void distribute_on(const uint8_t* cloud, uint64_t n, uint32_t stride, const CloudGrid& g, const OutParams& out,
-                   const FineAxes& fa, const uint32_t* pyr0, const uint64_t* data_idx, uint32_t* fill, uint32_t* lut,
+                   const FixedGrid& fg, const uint32_t* pyr0, const uint64_t* data_idx, uint32_t* fill, uint32_t* lut,
                    uint8_t* rec, uint32_t* word, uint32_t* err, const uint32_t* order, int num_sms,
                    cudaStream_t stream) {
     constexpr uint32_t kTile = dist_tile(kMode), kThreads = dist_threads(kMode);
     const size_t smem = align_up(chunk_smem(stride, g.grid, kF32, kTile, !kCells).total, 16) +
                         (kMode != kDirect ? sizeof(GroupSmem<kMode>) : 0);
     const int grid = chunk_grid_size(k_distribute<kF32, kCells, kMode>, kThreads, kTile, smem, n, num_sms);
-    k_distribute<kF32, kCells, kMode><<<grid, kThreads, smem, stream>>>(cloud, n, stride, g, out, fa, pyr0, data_idx,
+    k_distribute<kF32, kCells, kMode><<<grid, kThreads, smem, stream>>>(cloud, n, stride, g, out, fg, pyr0, data_idx,
                                                                          fill, lut, rec, word, err, order);
 }
 
@@ -1086,18 +1096,15 @@ int launch_distribute(const uint8_t* cloud, uint64_t n, uint32_t stride, bool fl
                       cudaStream_t stream) {
     if (n == 0) return 0;
     const auto go = float_input ? distribute_on<true, false, kDirect> : distribute_on<false, false, kDirect>;
-    go(cloud, n, stride, g, out, FineAxes{}, pyr0, data_idx, fill, lut, rec, frac, err, nullptr, num_sms, stream);
+    go(cloud, n, stride, g, out, FixedGrid{}, pyr0, data_idx, fill, lut, rec, frac, err, nullptr, num_sms, stream);
     return 1;
 }
 
 int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
-                            const OutParams& out, const FineAxis fine[3], const uint32_t* pyr0,
+                            const OutParams& out, const FixedGrid& fixed, const uint32_t* pyr0,
                             const uint64_t* data_idx, uint32_t* fill, uint32_t* lut, uint8_t* rec, uint32_t* word,
                             uint32_t* err, int num_sms, cudaStream_t stream) {
     if (n == 0) return 0;
-    FineAxes fa;
-    for (int a = 0; a < 3; ++a) fa.ax[a] = fine[a];
-    fa.cells = g.grid * 64;   // 2^depth counting cells, each 64 finest cells wide
     // records too long for the grouped kernels' shared memory are stored lane
     // by lane; on a small cloud the second launch costs more than it can give
     const bool fits = stride <= kGroupMaxStride, both = fits && n >= kGroupMinPoints;
@@ -1105,10 +1112,10 @@ int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, b
     const auto by_lane = !float_input ? distribute_on<false, true, kDirect>
                          : fits       ? distribute_on<true, true, kByTile>
                                       : distribute_on<true, true, kDirect>;
-    by_lane(cloud, n, stride, g, out, fa, pyr0, data_idx, fill, lut, rec, word, err, order, num_sms, stream);
+    by_lane(cloud, n, stride, g, out, fixed, pyr0, data_idx, fill, lut, rec, word, err, order, num_sms, stream);
     if (!both) return 1;
     const auto grouped = float_input ? distribute_on<true, true, kGrouped> : distribute_on<false, true, kGrouped>;
-    grouped(cloud, n, stride, g, out, fa, pyr0, data_idx, fill, lut, rec, word, err, order, num_sms, stream);
+    grouped(cloud, n, stride, g, out, fixed, pyr0, data_idx, fill, lut, rec, word, err, order, num_sms, stream);
     return 2;
 }
 

@@ -18,7 +18,7 @@
 // Cell words.  A candidate's cell in a node is the cell its position in the
 // cloud's cube gives at that node's resolution, unless rounding of the
 // reference's binary64 formula could decide otherwise: distribution proves the
-// former for almost every point (fine_cell) and stores the point's cell in its
+// former for almost every point (fixed_units) and stores the point's cell in its
 // leaf's parent; each level's output stores its own cell, and the parent's is
 // that, halved.  Bit 31 of a word says that the proof holds at every level;
 // without it the cell is evaluated from the cloud point in binary64.  When that
@@ -1310,6 +1310,9 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread(const __grid_constant
 // Records of all internal nodes at their final positions (post-order after
 // the n leaf records): output coordinates from the cloud point as in
 // distribution, colours from the staging array (or, raw, the cloud point's).
+// Bound by the reads of cloud points all over the cloud, 44 bytes of DRAM
+// traffic per point for 24 (115M records 2.19 -> 1.88 ms with coordinates in
+// fixed point instead of float-float, which left more registers for loads).
 // A warp takes runs of 128 records; the node of its first record comes from a
 // search over the nodes' first positions.
 template <bool kF32, bool kAveraged>
@@ -1317,6 +1320,7 @@ __global__ void __launch_bounds__(256) k_place_units(const uint64_t* __restrict_
                                                      const uint64_t* __restrict__ dst_off,
                                                      const uint32_t* __restrict__ count, uint32_t n_nodes, uint64_t n,
                                                      const uint64_t* __restrict__ total, OutParams op,
+                                                     const __grid_constant__ FixedGrid fg,
                                                      const uint8_t* __restrict__ cloud, uint32_t stride,
                                                      const uint32_t* __restrict__ stage_lut,
                                                      const uint64_t* __restrict__ stage_col, uint8_t* __restrict__ rec,
@@ -1343,18 +1347,17 @@ __global__ void __launch_bounds__(256) k_place_units(const uint64_t* __restrict_
                 while (p >= dst_off[v] + count[v] && v + 1 < n_nodes) ++v;
                 const uint64_t s = src_off[v] + (p - dst_off[v]);
                 const uint32_t idx = min(stage_lut[s], (uint32_t)n - 1u);   // a failed pass may leave any value
-                Coord c[3];
-                uint32_t col[3];
-                gather_point<kF32, !kAveraged>(cloud + (uint64_t)idx * stride, c, col);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) nw[k] = (uint32_t)out_coord<kF32>(c[k], op.ax[k]);
+                uint32_t w[kF32 ? 4 : 7];
+                gather_words<kF32, !kAveraged>(cloud + (uint64_t)idx * stride, w);
+                fixed_out_coords<kF32>(w, fg, op.ax, nw);
                 if (kAveraged) {
                     const uint2 e = *reinterpret_cast<const uint2*>(stage_col + s);
                     nw[3] = e.x;
                     nw[4] = e.y;
                 } else {
-                    nw[3] = col[0] | (col[1] << 16);
-                    nw[4] = col[2];
+                    const uint32_t col = w[kF32 ? 3 : 6];
+                    nw[3] = (col & 0xFFu) | (((col >> 8) & 0xFFu) << 16);
+                    nw[4] = (col >> 16) & 0xFFu;
                 }
             }
             store_run(rec + (p0 + q) * 18, 0, (uint32_t)min((unsigned long long)32, (unsigned long long)(end - p0 - q)),
@@ -1480,7 +1483,8 @@ int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_cand
 }
 
 int launch_place_units(const uint64_t* src_off, const uint64_t* dst_off, const uint32_t* count, uint32_t n_nodes,
-                       uint64_t n, const uint64_t* total, const OutParams& out, const uint8_t* cloud, uint32_t stride,
+                       uint64_t n, const uint64_t* total, const OutParams& out, const FixedGrid& fixed,
+                       const uint8_t* cloud, uint32_t stride,
                        bool float_input, bool averaged, const uint32_t* stage_lut, const uint64_t* stage_col,
                        uint8_t* rec, uint32_t* err, int num_sms, cudaStream_t stream) {
     if (!n_nodes) return 0;
@@ -1489,7 +1493,7 @@ int launch_place_units(const uint64_t* src_off, const uint64_t* dst_off, const u
         const uint64_t fit = (uint64_t)std::max(num_sms, 1) *
                              blocks_per_sm(reinterpret_cast<const void*>(kern), 256, 0);
         const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(fit, (n + 1023) / 1024));
-        kern<<<grid, 256, 0, stream>>>(src_off, dst_off, count, n_nodes, n, total, out, cloud, stride, stage_lut,
+        kern<<<grid, 256, 0, stream>>>(src_off, dst_off, count, n_nodes, n, total, out, fixed, cloud, stride, stage_lut,
                                        stage_col, rec, err);
     };
     if (float_input) averaged ? go(k_place_units<true, true>) : go(k_place_units<true, false>);

@@ -173,10 +173,10 @@ int launch_push_tags(uint32_t* pyr, const uint64_t* level_off_dev, uint32_t dept
 // Level of a leaf beside its first record in data_idx (launch_leaf_prep).
 constexpr uint32_t kLeafLevelShift = 56;
 
-// Distribution that writes cell words (out_coord_cell) instead of sub-step
+// Distribution that writes cell words (kSafeWord) instead of sub-step
 // words: for the octant kernels (launch_units_level).
 int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
-                            const OutParams& out, const FineAxis fine[3], const uint32_t* pyr0,
+                            const OutParams& out, const FixedGrid& fixed, const uint32_t* pyr0,
                             const uint64_t* data_idx, uint32_t* fill, uint32_t* lut, uint8_t* rec, uint32_t* word,
                             uint32_t* err, int num_sms, cudaStream_t stream);
 
@@ -374,7 +374,8 @@ int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_cand
 // The records of the internal nodes at their post-order positions, made from
 // the cloud points and the staged colours (see k_place_units).
 int launch_place_units(const uint64_t* src_off, const uint64_t* dst_off, const uint32_t* count, uint32_t n_nodes,
-                       uint64_t n, const uint64_t* total, const OutParams& out, const uint8_t* cloud, uint32_t stride,
+                       uint64_t n, const uint64_t* total, const OutParams& out, const FixedGrid& fixed,
+                       const uint8_t* cloud, uint32_t stride,
                        bool float_input, bool averaged, const uint32_t* stage_lut, const uint64_t* stage_col,
                        uint8_t* rec, uint32_t* err, int num_sms, cudaStream_t stream);
 
