@@ -244,8 +244,10 @@ private:
     void fill_cell_tables();
     CloudGrid cloud_grid() const;
     FixedGrid fixed_grid() const;
+    bool leaves_pyramid_zero() const;
+    void clean_pyramid();
     bool sparse_cloud() const;
-    void clear_for_count(bool sparse);
+    void clear_for_count();
     void params_writable();
     void record_params();
     void size_for_config();
@@ -270,7 +272,7 @@ private:
     const uint8_t* prefetched_ = nullptr;   // host cloud in flight to spare_ (nullptr: none)
     uint64_t prefetched_bytes_ = 0;
     DevBuf occ_;                        // sparse clouds: one flag byte per 64-cell block of the finest level
-    bool pyr_zero_ = false;             // the pyramid and the flags are all zero (sparse clean-up ran)
+    bool pyr_zero_ = false;             // the pyramid and the flags are all zero (clean_pyramid ran)
     DevBuf key_, count_, level_, info_, child_first_, level_start_, n_nodes_;
     DevBuf data_idx_, fill_;
     DevBuf lut_, rec_;                  // final outputs (N + P_out records)

@@ -112,3 +112,25 @@ def test_grids_in_turn_on_one_session():
         s.generate()
         compare_results(run_oracle(case, cfg), s)
     s.close()
+
+
+def test_pyramid_left_zero_between_builds():
+    """Builds in turn that find the count pyramid zero, or not: a dense one with a pyramid large enough to be zeroed
+    beside subsampling, again on the same state, a small dense grid, the sparse kind, and back."""
+    from helpers import octree_api
+
+    case = make_case(1, 1, 1_100_000, seed=41)
+    s = octree_api.OctreeSession(0)
+    s.set_cloud(case.cloud, n=case.n, stride=case.stride, cloud_type=case.cloud_type, scale=case.scale,
+                bb_min=case.bb_min, bb_max=case.bb_max)
+    want = {}
+    for grid in (256, 256, 64, 512, 256, 64):
+        cfg = dict(chunk_grid=grid, sub_grid=64, merge_threshold=20_000)
+        s.configure(**cfg)
+        s.init()
+        for _ in range(2):
+            s.generate()
+            if grid not in want:
+                want[grid] = run_oracle(case, cfg)
+            compare_results(want[grid], s)
+    s.close()
