@@ -141,15 +141,17 @@ int launch_count(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_i
 // flags themselves.
 int launch_sparse_zero(uint32_t* pyr0, uint8_t* occ, uint64_t blocks, cudaStream_t stream);
 
-// Builds levels 1..depth of the Morton count pyramid from level 0 and counts
-// occupied cells per level into `nonzero[level]`.  With occ, finest-level
-// blocks whose bit is clear are not read.
+// Builds the large levels of the Morton count pyramid from level 0 and counts
+// their occupied cells into `nonzero[level]`; launch_enumerate does the small
+// ones.  With occ (every level above the finest is zero), finest-level blocks
+// whose flag is clear are not read.
 int launch_pyramid(uint32_t* pyr, const uint64_t* level_off_host, uint32_t depth, uint32_t* nonzero,
                     const uint8_t* occ, cudaStream_t stream);
 
-int launch_enumerate(const uint32_t* pyr, const uint64_t* level_off_dev, uint32_t depth, uint32_t threshold,
-                      uint32_t* key, uint32_t* count, uint8_t* level, uint16_t* info, uint32_t* child_first,
-                      uint32_t cap, uint32_t* level_start, uint32_t* n_nodes, uint32_t* err, cudaStream_t stream);
+int launch_enumerate(uint32_t* pyr, const uint64_t* level_off_dev, uint32_t depth, uint32_t* nonzero,
+                     uint32_t threshold, uint32_t* key, uint32_t* count, uint8_t* level, uint16_t* info,
+                     uint32_t* child_first, uint32_t cap, uint32_t* level_start, uint32_t* n_nodes, uint32_t* err,
+                     cudaStream_t stream);
 
 // Ordered keys of the coordinate minima (keys[0..2]) and maxima (keys[3..5])
 // of the cloud, NaN coordinates skipped (float keys widened to 64 bits);

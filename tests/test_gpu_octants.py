@@ -134,3 +134,21 @@ def test_pyramid_left_zero_between_builds():
                 want[grid] = run_oracle(case, cfg)
             compare_results(want[grid], s)
     s.close()
+
+
+@pytest.mark.parametrize("n", [500, 60_000])
+@pytest.mark.parametrize("grid", [2, 4, 8, 16, 32, 64, 128, 256])
+def test_pyramid_levels(grid, n):
+    """Counts of every level and the number of occupied cells, where the pyramid's top (32^3 cells and fewer) is the
+    whole of it, starts after one or two launches, and for sparse and dense clouds."""
+    xyz, rgb = points("volume", n)
+    case = case_from_points(xyz * 50.0, rgb, 1, scale=0.001, bbox=[0, 0, 0, 50.5, 50.5, 50.5])
+    cfg = dict(chunk_grid=grid, sub_grid=32, merge_threshold=300)
+    ref = run_oracle(case, cfg, keep_levels=True)
+    s = run_gpu(case, dict(cfg, debug=1))
+    assert s.stats()["sparse_nodes"] == ref.stats["sparse_nodes"]
+    level, g = 0, grid
+    while g >= 1:
+        np.testing.assert_array_equal(s.level_counts(level, g), ref.level_counts[level])
+        level, g = level + 1, g // 2
+    s.close()
