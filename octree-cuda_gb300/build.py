@@ -18,7 +18,9 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-CU_SOURCES = ["k_chunking.cu", "k_subsample.cu", "k_units.cu", "noalloc.cu"]
+# (k_units.cu is compiled in three parts, side by side)
+CU_SOURCES = ["k_chunking.cu", "k_subsample.cu", "k_units.cu", "k_units.cu:OC_UNITS_PART=1", "k_units.cu:OC_UNITS_PART=2",
+              "noalloc.cu"]
 CPP_SOURCES = ["builder.cpp", "export.cpp", "octree_api.cpp", "serve.cpp", "wave.cpp"]
 HEADERS = ["device_common.cuh", "fixed_axis.h", "kernels.h", "builder.h", "wave.h"]
 
@@ -44,14 +46,15 @@ EXTRA_NVCC = os.environ.get("OC_EXTRA_NVCC", "").split()
 
 
 def _compile(src, verbose_ptxas=False):
+    src, _, define = src.partition(":")
     path = os.path.join(CSRC, src)
-    obj = os.path.join(BUILD, src + ".o")
+    obj = os.path.join(BUILD, src + ("." + define if define else "") + ".o")
     deps = [path] + [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(HERE, "..", "include", "octreeApi.h")]
     if _newer(obj, deps) and not verbose_ptxas:
         return obj, ""
     if src.endswith(".cu"):
         cmd = [NVCC, *ARCH, *EXTRA_NVCC, "-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
-               "-Xcompiler", "-fvisibility=hidden", "-c", path, "-o", obj]
+               "-Xcompiler", "-fvisibility=hidden", *(["-D" + define] if define else []), "-c", path, "-o", obj]
         if verbose_ptxas:
             cmd.insert(1, "-Xptxas=-v")
     else:

@@ -40,11 +40,15 @@
 #include "device_common.cuh"
 #include "kernels.h"
 
+#ifndef OC_UNITS_PART
+#define OC_UNITS_PART 0
+#endif
+
 namespace oc {
 
 namespace {
 
-// Blocks of a level (T threads): two of 512 per SM hide each other's barriers;
+// Blocks of a level (T threads): two of 640 per SM hide each other's barriers;
 // one of 1024 has the whole shared memory for its unit's cells; two of 768 for
 // distance weighting, whose emit runs on instructions and loads alone.
 constexpr int unit_blocks(int T) { return T == 1024 ? 1 : 2; }
@@ -748,7 +752,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
 
 // unit_cells on global memory out of line, for blocks of 1024 threads, which
 // seldom need it: inlined, its registers weigh on the other variant's (level
-// 4 of the 119.7M-point build 1.34 -> 1.27 ms; two blocks of 512, which
+// 4 of the 119.7M-point build 1.34 -> 1.27 ms; two blocks per SM, which
 // need it often, lose by it: level 1 0.84 -> 1.13 ms).
 template <int T, int kColor, bool kRandom, int kB, class Pre>
 __device__ __noinline__ void unit_cells_global(const UnitLevelArgs& a, BlockShared& sh, const uint32_t* bm,
@@ -905,8 +909,8 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
         unit_cells<T, kColor, kRandom, kB, false, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, placed, ws);
 }
 
-// Units of other kinds than the most frequent one, out of line for blocks of
-// 1024 (levels 1 and 4 of 119.7M points 822 -> 778 and 1378 -> 1256 us).
+// Units of other kinds than the level's frequent ones, out of line, so that
+// their registers do not weigh on those (see launch_units).
 template <int T, int kColor, bool kRandom>
 __device__ __noinline__ void unit_run_other(const UnitLevelArgs& a, BlockShared& sh, uint32_t* bm, uint32_t ui,
                                             WeightShared* ws) {
@@ -918,7 +922,8 @@ __device__ __noinline__ void unit_run_other(const UnitLevelArgs& a, BlockShared&
 // kColor: 0 raw colour, 1 intra-cell, 2 inter-cell, 3 distance-weighted.  An
 // inter-cell or weighted colour whose neighbourhood reaches into other units keeps its sum and goes to its
 // node's face list (k_faces).
-template <int T, int kColor, bool kRandom>
+// kHalf: units of half the side (parts of split children, or a grid of 64) are frequent too.
+template <int T, int kColor, bool kRandom, bool kHalf>
 __global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_constant__ UnitLevelArgs a) {
     extern __shared__ __align__(16) uint32_t dyn[];
     __shared__ BlockShared sh;
@@ -942,15 +947,9 @@ __global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_consta
         if (ui >= a.n_units) break;
         // (the weighted lists follow the pool)
         WeightShared* ws = reinterpret_cast<WeightShared*>(dyn + a.smem_words);
-        if constexpr (T == 1024) {
-            if (sh.un.b == 6 && sh.un.cnt <= 65535) unit_run<T, kColor, kRandom, 6, uint16_t>(a, sh, dyn, ui, ws);
-            else unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
-            continue;
-        }
-        if (sh.un.b == 6 && sh.un.cnt > 65535) unit_run<T, kColor, kRandom, 6, uint32_t>(a, sh, dyn, ui, ws);
-        else if (sh.un.b == 6) unit_run<T, kColor, kRandom, 6, uint16_t>(a, sh, dyn, ui, ws);
-        else if (sh.un.b == 5) unit_run<T, kColor, kRandom, 5, uint16_t>(a, sh, dyn, ui, ws);
-        else unit_run<T, kColor, kRandom, 0, uint16_t>(a, sh, dyn, ui, ws);
+        if (sh.un.b == 6 && sh.un.cnt <= 65535) unit_run<T, kColor, kRandom, 6, uint16_t>(a, sh, dyn, ui, ws);
+        else if (kHalf && sh.un.b == 5) unit_run<T, kColor, kRandom, 5, uint16_t>(a, sh, dyn, ui, ws);
+        else unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
     }
 }
 
@@ -1389,11 +1388,11 @@ int blocks_per_sm(const void* kernel, int threads, size_t smem) {
 
 // Shared memory of a unit block: an equal share of an SM's 227 KB, less the
 // static part and the 1 KB the system takes per block.
-template <int T, int kColor, bool kRandom>
+template <int T, int kColor, bool kRandom, bool kHalf>
 void launch_units_of(UnitLevelArgs a, int num_sms, cudaStream_t stream) {
     const size_t smem = (227 * 1024 / unit_blocks(T) - 1024 - sizeof(BlockShared)) & ~(size_t)127;
     a.smem_words = (uint32_t)((smem - (kColor == 3 ? sizeof(WeightShared) : 0)) / 4) & ~3u;
-    auto kern = k_units<T, kColor, kRandom>;
+    auto kern = k_units<T, kColor, kRandom, kHalf>;
     allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     const uint64_t fit =
         (uint64_t)std::max(num_sms, 1) * blocks_per_sm(reinterpret_cast<const void*>(kern), T, smem);
@@ -1408,22 +1407,37 @@ void launch_units_of(UnitLevelArgs a, int num_sms, cudaStream_t stream) {
 // (140 KB) 330 -> 278 us; but 119.7M points, level 3 (74 KB): 2.42 ms with two
 // blocks, 2.82 with one.  With 1 to 3 units per SM two blocks are the better
 // balance (level of 294 units: 135 us against 172).
+//
+// `half`: units of half the side are frequent.  Only the frequent kinds are in
+// line in a kernel, and two blocks of 640 then have registers enough (with all
+// kinds in line 640 threads gained nothing over 512; 704 and 768 gain less).
+// 119.7M points, levels 2 and 3, 0.96 -> 0.87 and 2.31 -> 2.07 ms; 5.1M points
+// 1.10 -> 1.03; 25.8M, level 4, 0.34 -> 0.30.  Both kinds in line everywhere:
+// level 3 2.20; out of line where they are frequent: level 8 of 25.8M points
+// 80 -> 106 us, weighted 0.51 -> 0.53 ms.
 template <int kColor, bool kRandom>
-void launch_units(const UnitLevelArgs& a, uint32_t mean_candidates, int num_sms, cudaStream_t stream) {
+void launch_units(const UnitLevelArgs& a, uint32_t mean_candidates, bool half, int num_sms, cudaStream_t stream) {
     if constexpr (kColor == 3) {
-        launch_units_of<kWeightThreads, kColor, kRandom>(a, num_sms, stream);
+        if (half) launch_units_of<kWeightThreads, kColor, kRandom, true>(a, num_sms, stream);
+        else launch_units_of<kWeightThreads, kColor, kRandom, false>(a, num_sms, stream);
     } else {
         const uint64_t sms = (uint64_t)std::max(num_sms, 1);
         const bool wide = a.n_units <= sms ||
                           (a.n_units >= 3 * sms && (uint64_t)mean_candidates * cell_bytes(kColor, kRandom) > 78 * 1024);
-        if (wide) launch_units_of<1024, kColor, kRandom>(a, num_sms, stream);
-        else launch_units_of<512, kColor, kRandom>(a, num_sms, stream);
+        if (wide) launch_units_of<1024, kColor, kRandom, false>(a, num_sms, stream);
+        else if (half) launch_units_of<640, kColor, kRandom, true>(a, num_sms, stream);
+        else launch_units_of<640, kColor, kRandom, false>(a, num_sms, stream);
     }
 }
 
-}   // namespace
-
-namespace {
+// Half-size units are frequent where children are split and on grids up to 64.
+template <int kColor>
+void launch_units_as(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                     cudaStream_t stream) {
+    const bool half = any_split || a.s <= 6;
+    if (random) launch_units<kColor, true>(a, mean_candidates, half, num_sms, stream);
+    else launch_units<kColor, false>(a, mean_candidates, half, num_sms, stream);
+}
 
 template <int kColor>
 void launch_faces(const UnitLevelArgs& a, bool any_split, int num_sms, cudaStream_t stream) {
@@ -1456,30 +1470,52 @@ void launch_colours(const UnitLevelArgs& a, bool any_split, int num_sms, cudaStr
 
 }   // namespace
 
+// The colours' kernels, compiled apart: OC_UNITS_PART 0 raw and averaged in the
+// cell, 1 inter-cell, 2 distance-weighted.
+int launch_units_raw(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                     cudaStream_t stream);
+int launch_units_intra(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                       cudaStream_t stream);
+int launch_units_inter(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                       cudaStream_t stream);
+int launch_units_weighted(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                          cudaStream_t stream);
+
+#if OC_UNITS_PART == 1
+int launch_units_inter(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                       cudaStream_t stream) {
+    launch_units_as<2>(a, random, mean_candidates, any_split, num_sms, stream);
+    launch_colours<2>(a, any_split, num_sms, stream);
+    return 2;
+}
+#elif OC_UNITS_PART == 2
+int launch_units_weighted(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                          cudaStream_t stream) {
+    launch_units_as<3>(a, random, mean_candidates, any_split, num_sms, stream);
+    launch_colours<3>(a, any_split, num_sms, stream);
+    return 2;
+}
+#else
+int launch_units_raw(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                     cudaStream_t stream) {
+    launch_units_as<0>(a, random, mean_candidates, any_split, num_sms, stream);
+    return 1;
+}
+
+int launch_units_intra(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                       cudaStream_t stream) {
+    launch_units_as<1>(a, random, mean_candidates, any_split, num_sms, stream);
+    return 1;
+}
+
 int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_candidates, bool any_split, int num_sms,
                        cudaStream_t stream) {
     if (!a.n_units) return 0;
-    const bool random = (mode & kModeRandom) != 0;
-    if (mode & kModeIntra) {
-        if (random) launch_units<1, true>(a, mean_candidates, num_sms, stream);
-        else launch_units<1, false>(a, mean_candidates, num_sms, stream);
-        return 1;
-    }
-    if ((mode & kModeInter) && (mode & kModeWeight)) {
-        if (random) launch_units<3, true>(a, mean_candidates, num_sms, stream);
-        else launch_units<3, false>(a, mean_candidates, num_sms, stream);
-        launch_colours<3>(a, any_split, num_sms, stream);
-        return 2;
-    }
-    if (mode & kModeInter) {
-        if (random) launch_units<2, true>(a, mean_candidates, num_sms, stream);
-        else launch_units<2, false>(a, mean_candidates, num_sms, stream);
-        launch_colours<2>(a, any_split, num_sms, stream);
-        return 2;
-    }
-    if (random) launch_units<0, true>(a, mean_candidates, num_sms, stream);
-    else launch_units<0, false>(a, mean_candidates, num_sms, stream);
-    return 1;
+    const auto go = (mode & kModeIntra)                                ? launch_units_intra
+                    : (mode & kModeInter) && (mode & kModeWeight) ? launch_units_weighted
+                    : (mode & kModeInter)                              ? launch_units_inter
+                                                                       : launch_units_raw;
+    return go(a, (mode & kModeRandom) != 0, mean_candidates, any_split, num_sms, stream);
 }
 
 int launch_place_units(const uint64_t* src_off, const uint64_t* dst_off, const uint32_t* count, uint32_t n_nodes,
@@ -1500,5 +1536,7 @@ int launch_place_units(const uint64_t* src_off, const uint64_t* dst_off, const u
     else averaged ? go(k_place_units<false, true>) : go(k_place_units<false, false>);
     return 1;
 }
+
+#endif   // OC_UNITS_PART
 
 }   // namespace oc
