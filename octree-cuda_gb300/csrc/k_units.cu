@@ -1332,9 +1332,11 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread(const __grid_constant
 // Records of all internal nodes at their final positions (post-order after
 // the n leaf records): output coordinates from the cloud point as in
 // distribution, colours from the staging array (or, raw, the cloud point's).
-// Bound by the reads of cloud points all over the cloud, 44 bytes of DRAM
-// traffic per point for 24 (115M records 2.19 -> 1.88 ms with coordinates in
-// fixed point instead of float-float, which left more registers for loads).
+// Bound by the reads of cloud points all over the cloud, 57 bytes of DRAM
+// traffic per point for 24: 86 in all, at 5.3 TB/s (115M records 2.19 -> 1.88
+// ms with coordinates in fixed point instead of float-float, which left more
+// registers for loads; two or four gathers per lane in flight leave too few
+// warps: 3.1 and 2.05 ms).
 // A warp takes runs of 128 records; the node of its first record comes from a
 // search over the nodes' first positions.
 template <bool kF32, bool kAveraged>
