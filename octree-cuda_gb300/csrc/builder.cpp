@@ -694,13 +694,7 @@ void Builder::check_device_errors(const char* stage) {
 }
 
 void throw_device_errors(uint32_t e, const char* stage) {
-    if (e & kErrBelowBox) throw Error(std::string(stage) + ": a point lies below the bounding box");
-    if (e & kErrCoordRange) throw Error(std::string(stage) + ": an output coordinate does not fit int32");
-    if (e & kErrProbe) throw Error(std::string(stage) + ": subsampling brick table overflow");
-    if (e & kErrNodeCap) throw Error(std::string(stage) + ": node capacity exceeded");
-    if (e & kErrCapacity) throw Error(std::string(stage) + ": output capacity exceeded");
-    if (e & kErrTag) throw Error(std::string(stage) + ": a point found no leaf");
-    if (e & kErrTimeout) throw Error(std::string(stage) + ": a bulk copy did not complete in time");
+    if (const char* message = device_error_message(e)) throw Error(std::string(stage) + ": " + message);
 }
 
 CloudGrid Builder::cloud_grid() const {

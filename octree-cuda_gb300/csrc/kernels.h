@@ -368,6 +368,19 @@ struct UnitLevelArgs {
     uint32_t* err;
 };
 
+// Message of a device error word's first bit; null when no bit is set.
+inline const char* device_error_message(uint32_t e) {
+    if (e & kErrBelowBox) return "a point lies below the bounding box";
+    if (e & kErrCoordRange) return "an output coordinate does not fit int32";
+    if (e & kErrProbe) return "subsampling brick table overflow";
+    if (e & kErrNodeCap) return "node capacity exceeded";
+    if (e & kErrCapacity) return "output capacity exceeded";
+    if (e & kErrTag) return "a point found no leaf";
+    if (e & kErrTimeout) return "a wait on the device (for a bulk copy or for another block) gave up";
+    if (e & kErrForeign) return "points outside their octants were left over";
+    return e ? "unknown device error" : nullptr;
+}
+
 // mean_candidates: about, per unit.  any_split: some child of the level is split in parts.  Inter-cell averaging takes two
 // launches: the units, then what their outermost cells get from other units.
 int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_candidates, bool any_split, int num_sms,
