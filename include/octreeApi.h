@@ -80,7 +80,9 @@ OCPI_EXPORT const char* ocpi_last_error(void);
 /* Seed of the explicit-random subsampling priorities (default 0x5EED). */
 OCPI_EXPORT int ocpi_set_random_seed(void* session, uint64_t seed);
 /* Debug switches: bit 0 keeps a copy of the count pyramid (dense per level,
- * z-major order) for ocpi_get_level_counts. */
+ * z-major order) for ocpi_get_level_counts; bit 1 makes the device's waits for
+ * the earlier parts of a node give up at once, so that the build fails with
+ * the error of a wait that ran out (for tests of that error). */
 OCPI_EXPORT int ocpi_set_debug_flags(void* session, uint32_t flags);
 
 typedef struct OcpiStats {

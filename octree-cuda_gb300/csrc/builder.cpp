@@ -1331,6 +1331,8 @@ void Builder::subsample() {
                                        kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 8,
                                        stream_),
                        "memset");
+            uint64_t largest_unit = S3;
+            for (const UnitEntry& e : units) largest_unit = std::max<uint64_t>(largest_unit, e.count);
             uint8_t* sync = unit_sync_.as<uint8_t>();
             UnitNodeState* node_state = reinterpret_cast<UnitNodeState*>(sync + kUnitSyncHead);
             uint64_t* unit_state = reinterpret_cast<uint64_t*>(node_state + n_internal);
@@ -1378,6 +1380,7 @@ void Builder::subsample() {
                 u.csr_start = csr_start_.as<uint32_t>();
                 u.csr_pts = csr_pts_.as<float4>();
                 u.ticket = reinterpret_cast<uint32_t*>(sync + 128) + l;
+                u.wait_limit = unit_wait_limit(cfg_.debug, largest_unit);
                 u.err = err_.as<uint32_t>();
                 launches_ += launch_units_level(u, mode, mean_candidates[l], any_split[l], num_sms_, stream_);
                 char mark[32];
@@ -1475,6 +1478,11 @@ void Builder::subsample() {
         if (attempt == 0) compute_tree_stats();
         check_cuda(cudaStreamSynchronize(stream_), "subsample");
         const uint32_t e = *back_host_.as<uint32_t>(0);
+        if (e & ~(kErrCapacity | kErrForeign)) {
+            // the tables behind the results may not agree: nothing is taken from them
+            if (copy_stream_) check_cuda(cudaStreamSynchronize(copy_stream_), "output copies");
+            throw_device_errors(e, (e & kErrCapacity) ? "subsample" : "generate");
+        }
         p_out_ = *back_host_.as<uint64_t>(16);
         if ((e & kErrForeign) && attempt < 6 && !(e & ~(kErrForeign | kErrCapacity))) {
             // a point that two levels' formulas put on different sides of an

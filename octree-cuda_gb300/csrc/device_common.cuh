@@ -126,10 +126,14 @@ enum : uint32_t {
     kErrProbe = 1u << 2,         // a hash probe exceeded its bound
     kErrCapacity = 1u << 3,      // a scratch buffer was too small
     kErrTag = 1u << 4,           // a point found no leaf
-    kErrTimeout = 1u << 5,       // a bounded wait on a bulk copy gave up
+    kErrTimeout = 1u << 5,       // a bounded wait (on a bulk copy, on an earlier unit) gave up
     kErrNodeCap = 1u << 6,       // the tree has more nodes than the node table holds
     kErrForeign = 1u << 7,       // a candidate's cell lies outside its child's octant (the pass is repeated)
 };
+
+// Any of these leaves a level without whole outputs: what reads them does not
+// run (the pass is repeated or the build fails).
+constexpr uint32_t kErrStop = kErrCapacity | kErrTimeout | kErrForeign;
 
 // ---------------------------------------------------------------------------
 // Ordered keys: monotone maps of IEEE bit patterns onto signed integers, so

@@ -68,13 +68,14 @@ __device__ __forceinline__ void store_release(uint64_t* p, uint64_t v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Waits until *p is not 0; gives up after about 2^31 clock cycles and returns 0.
-__device__ __forceinline__ uint64_t wait_nonzero(const uint64_t* p) {
-    uint64_t v = load_acquire(p);
-    if (v) return v;
+// Waits until *p is not 0; gives up after `limit` clock cycles (a negative
+// limit: at once) and returns 0.
+__device__ __forceinline__ uint64_t wait_nonzero(const uint64_t* p, long long limit) {
+    uint64_t v = limit < 0 ? 0 : load_acquire(p);
+    if (v || limit < 0) return v;
     const long long t0 = clock64();
     while (!(v = load_acquire(p)))
-        if (clock64() - t0 > (1ll << 31)) return 0;
+        if (clock64() - t0 > limit) return 0;
     return v;
 }
 
@@ -206,7 +207,7 @@ __device__ __forceinline__ void append_faces(const UnitLevelArgs& a, uint32_t no
 struct BlockShared {
     Unit un;
     uint32_t warp[32];
-    uint32_t unit, unsafe, rank0, cand0, included, next, fail, redo;
+    uint32_t unit, unsafe, rank0, cand0, included, next, fail, redo, stop;
     int32_t delta;
     uint64_t off, level_base;
 };
@@ -245,13 +246,13 @@ __device__ __forceinline__ void unit_place(const UnitLevelArgs& a, BlockShared& 
     uint32_t r0 = 0, c0 = 0;
     bool ok = true;
     for (uint32_t q = lane; q < un.index; q += 32) {
-        const uint64_t v = wait_nonzero(&a.unit_state[ui - 1 - q]);
+        const uint64_t v = wait_nonzero(&a.unit_state[ui - 1 - q], a.wait_limit);
         ok = ok && v != 0;
         r0 += (uint32_t)v - 1;
         c0 += (uint32_t)(v >> 32);
     }
     uint64_t off1 = 0;
-    if (lane == 0) off1 = wait_nonzero(&a.node_state[un.node].off1);
+    if (lane == 0) off1 = wait_nonzero(&a.node_state[un.node].off1, a.wait_limit);
     ok = ok && (lane != 0 || off1 != 0);
     r0 = __reduce_add_sync(0xffffffffu, r0);
     c0 = __reduce_add_sync(0xffffffffu, c0);
@@ -954,7 +955,13 @@ __global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_consta
         uint64_t b = 0;
         for (uint32_t l = 1; l < a.level; ++l) b += a.level_used[l];
         sh.level_base = b;
+        sh.stop = *(volatile uint32_t*)a.err;
     }
+    __syncthreads();
+    // after an error the tables of the levels below may not agree with each
+    // other: nothing is read by them (a unit that gave up leaves cells without
+    // points, and octants whose ends lie before their starts)
+    if (sh.stop) return;
     for (;;) {
         __syncthreads();   // the previous unit is done with the shared state
         if (tid == 0) {
@@ -1014,6 +1021,7 @@ __global__ void __launch_bounds__(kFaceThreads) k_faces(const __grid_constant__ 
     const uint32_t W = max((3 * pl.np) << (2 * a.s) >> 5, 1u);
     uint32_t* bits = dyn;
     uint32_t* pre = dyn + W;
+    if (*a.err) return;   // (set by earlier launches alone, as in k_spread)
     uint64_t level_base = 0;
     for (uint32_t l = 1; l < a.level; ++l) level_base += a.level_used[l];
     for (uint32_t item = blockIdx.x; item < a.n_nodes * slices; item += gridDim.x) {
@@ -1218,6 +1226,7 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread(const __grid_constant
     __shared__ uint2 s_rows[kColor == 3 ? T / kG : 1][18];
     const uint32_t tid = threadIdx.x, lane = tid & 31, s = lane % kG;
     const uint32_t ui = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
+    if (*a.err) return;
     const uint32_t cells = (uint32_t)a.unit_state[ui] - 1u;
     const UnitEntry en = a.units[ui];
     const UnitNodeState st = a.node_state[en.node];
@@ -1353,7 +1362,7 @@ __global__ void __launch_bounds__(256) k_place_units(const uint64_t* __restrict_
     constexpr uint32_t kRun = 128;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint8_t* stage = s_stage + warp * kStageBytes;
-    if (*err & kErrCapacity) return;   // nothing was placed; the pass is repeated
+    if (*err & kErrStop) return;   // nothing was placed
     const uint64_t end = n + *total;
     const uint64_t step = (uint64_t)gridDim.x * 8 * kRun;
     for (uint64_t p0 = n + ((uint64_t)blockIdx.x * 8 + warp) * kRun; p0 < end; p0 += step) {

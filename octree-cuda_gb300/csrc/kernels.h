@@ -365,6 +365,7 @@ struct UnitLevelArgs {
     uint64_t* partials;     // entries taken
     uint64_t partial_cap;
     uint32_t* ticket;
+    int64_t wait_limit;     // clock cycles a unit waits for the node's earlier ones (negative: none, every wait fails)
     uint32_t* err;
 };
 
@@ -379,6 +380,17 @@ inline const char* device_error_message(uint32_t e) {
     if (e & kErrTimeout) return "a wait on the device (for a bulk copy or for another block) gave up";
     if (e & kErrForeign) return "points outside their octants were left over";
     return e ? "unknown device error" : nullptr;
+}
+
+// Debug flag (ocpi_set_debug_flags): the waits between units give up at once.
+constexpr uint32_t kDebugNoWait = 2;
+
+// How long a unit waits for the node's earlier units: 2^31 cycles (a second),
+// and 1024 for each candidate of the largest unit, which covers a unit whose
+// every candidate is evaluated in binary64 (about 100 cycles each in a block
+// of its own).
+inline int64_t unit_wait_limit(uint32_t debug, uint64_t largest_unit) {
+    return (debug & kDebugNoWait) ? -1 : (int64_t)((1ull << 31) + (largest_unit << 10));
 }
 
 // mean_candidates: about, per unit.  any_split: some child of the level is split in parts.  Inter-cell averaging takes two

@@ -1,4 +1,4 @@
-"""The messages of device error words (octree-cuda_gb300/csrc/kernels.h, compiled with the host
+"""The messages of device error words and the wait limit (octree-cuda_gb300/csrc/kernels.h, compiled with the host
 compiler): every bit has a message, so that no failed build is taken for a good one."""
 import os
 import shutil
@@ -18,7 +18,9 @@ int main() {
         if (!m || !*m) return 1 + k;
     }
     if (oc::device_error_message(0)) return 40;
-    return 0;
+    // no unit is given less than a second; the largest cloud's limit does not wrap
+    if (oc::unit_wait_limit(0, 0) < (1ll << 31) || oc::unit_wait_limit(0, 0xFFFFFFFFull) < (1ll << 41)) return 41;
+    return oc::unit_wait_limit(oc::kDebugNoWait, 1000) < 0 ? 0 : 42;
 }
 """
 

@@ -152,3 +152,30 @@ def test_pyramid_levels(grid, n):
         np.testing.assert_array_equal(s.level_counts(level, g), ref.level_counts[level])
         level, g = level + 1, g // 2
     s.close()
+
+
+@pytest.mark.parametrize("mode", sorted(MODES))
+@pytest.mark.parametrize("n,chunk,sub", [(60_000, 16, 32), (150_000, 64, 128)])
+def test_wait_that_runs_out(n, chunk, sub, mode):
+    """A unit that gives up waiting for its node's earlier ones ends the call with an error, and nothing after it reads
+    what it left (levels of both kinds: with colours spread over blocks, and not); the session goes on."""
+    from helpers import octree_api
+
+    xyz, rgb = points("volume", n)
+    case = case_from_points(xyz * 50.0, rgb, 1, scale=0.001, bbox=[0, 0, 0, 50.5, 50.5, 50.5])
+    cfg = dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=300, output_factor=12.0, **MODES[mode])
+    s = octree_api.OctreeSession(0)
+    s.set_cloud(case.cloud, n=case.n, stride=case.stride, cloud_type=case.cloud_type, scale=case.scale,
+                bb_min=case.bb_min, bb_max=case.bb_max)
+    out = np.zeros(12 * n * 18, np.uint8), np.zeros(12 * n, np.uint32)
+    s.set_output_host(*out)
+    s.configure(debug=2, **cfg)
+    s.init()
+    for _ in range(2):
+        with pytest.raises(octree_api.OctreeError, match="wait on the device"):
+            s.generate()
+    s.configure(**cfg)
+    s.init()
+    s.generate()
+    compare_results(run_oracle(case, cfg), s)
+    s.close()
