@@ -320,15 +320,12 @@ void Builder::size_for_config() {
     }
     node_cap_ = (uint32_t)std::min<uint64_t>(cap, level_off_[depth_ + 1]);
 
-    {
-        // a new pyramid or bitmap allocation holds garbage: the next build
-        // clears it in full
-        const void* old_pyr = pyr_.p;
-        const void* old_occ = occ_.p;
-        pyr_.ensure(level_off_[depth_ + 1] * 4);
-        occ_.ensure(std::max<uint64_t>(level_off_[1] >> 6, 1));
-        if (pyr_.p != old_pyr || occ_.p != old_occ) pyr_zero_ = false;
-    }
+    // a new pyramid or flag allocation holds garbage: the next build clears it
+    // in full (the address says nothing: a larger one may come back at the old)
+    const uint64_t pyr_bytes = level_off_[depth_ + 1] * 4, occ_bytes = std::max<uint64_t>(level_off_[1] >> 6, 1);
+    if (pyr_bytes > pyr_.bytes || occ_bytes > occ_.bytes) pyr_zero_ = false;
+    pyr_.ensure(pyr_bytes);
+    occ_.ensure(occ_bytes);
     loff_.ensure(level_off_.size() * 8);
     params_writable();
     loff_host_.ensure(level_off_.size() * 8);
