@@ -104,7 +104,9 @@ typedef struct OcpiStats {
     uint32_t kernel_launches; /* kernels launched by the last ocpi_generate_octree */
     uint32_t subsample_passes; /* subsampling passes of the last build: 1, or more when a level's
                                   candidates or the final records outgrew their buffers and the
-                                  pass was repeated with larger ones */
+                                  pass was repeated with larger ones, or when points on the
+                                  boundary of an octant were met and the levels from there on
+                                  were repeated (timings: "repeat_octants", "repeat_nodes") */
 } OcpiStats;
 
 OCPI_EXPORT int ocpi_get_stats(void* session, OcpiStats* out);

@@ -1104,11 +1104,17 @@ void Builder::subsample() {
     std::vector<uint32_t> mean_candidates(depth_ + 2, 0);   // per unit, inner children taken at 16384 points at most
     uint32_t s_log2 = 0;
     while ((1u << s_log2) < S) ++s_log2;
-    if (octants) {
+    // every_octant: octants without a child get a unit too, for points of other
+    // octants whose cell lies there (a repeat with those, see k_foreign).
+    auto lay_out_units = [&](bool every_octant) {
+        units.clear();
+        oct_unit.clear();
+        map_words = 0;
         // the part of the memory estimate that a brick table would take
         const uint64_t map_room = (uint64_t)num_sms_ * memory_terms(cfg_, num_sms_).slots * 8;
         for (uint32_t l = 1; l <= depth_; ++l) {
             unit_first[l] = (uint32_t)units.size();
+            any_split[l] = 0;
             uint64_t whole = 0;
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) whole += table[k].nchild;
             const bool few = S >= 64 && whole < (uint64_t)num_sms_ * 3;
@@ -1122,12 +1128,22 @@ void Builder::subsample() {
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
                 const NodeHost& v = nodes_[order[k]];
                 uint32_t c = v.child_first, number = 0, q0 = 0;
+                table[k].child_kind &= 0xFFFFu;
                 for (uint32_t s = 0; s < 8; ++s) {
-                    if (!(v.mask & (1u << s))) continue;
-                    const uint32_t ci = c++;
-                    const NodeHost& ch = nodes_[ci];
-                    const bool split = few && ch.internal && out_bound[ci] > 4096;
-                    candidates += ch.internal ? std::min<uint64_t>(out_bound[ci], 16384) : ch.points;
+                    UnitEntry e{};
+                    e.node = k - level_first[l];
+                    bool split = false;
+                    if (v.mask & (1u << s)) {
+                        const uint32_t ci = c++;
+                        const NodeHost& ch = nodes_[ci];
+                        split = few && ch.internal && out_bound[ci] > 4096;
+                        candidates += ch.internal ? std::min<uint64_t>(out_bound[ci], 16384) : ch.points;
+                        e.flags = (uint32_t)ch.internal << 7;
+                        e.src = ch.internal ? ii_of[ci] : (uint32_t)ch.data_idx;
+                        e.count = ch.internal ? 0 : ch.points;
+                    } else if (!every_octant) {
+                        continue;
+                    }
                     if (split) {
                         any_split[l] = 1;
                         table[k].child_kind |= 1u << (16 + s);
@@ -1136,17 +1152,13 @@ void Builder::subsample() {
                         oct_unit[oct_first[l] + (size_t)(k - level_first[l]) * 8 + s] =
                             ((uint32_t)units.size() - unit_first[l]) | ((uint32_t)split << 31);
                     for (uint32_t part = split ? 8 : 0; part < (split ? 16u : 1u); ++part) {
-                        UnitEntry e{};
-                        e.node = k - level_first[l];
-                        e.flags = s | (part << 3) | ((uint32_t)ch.internal << 7) | ((uint32_t)(number == 0) << 8) |
-                                  (number << 10) | (q0 << 16);
-                        e.src = ch.internal ? ii_of[ci] : (uint32_t)ch.data_idx;
-                        e.count = ch.internal ? 0 : ch.points;
+                        UnitEntry u = e;
+                        u.flags |= s | (part << 3) | ((uint32_t)(number == 0) << 8) | (number << 10) | (q0 << 16);
                         if (spread[l]) {
-                            e.map = (uint32_t)words;
+                            u.map = (uint32_t)words;
                             words += 2 * ((uint64_t)1 << (3 * (s_log2 - (split ? 2 : 1)) - 5)) + 4;
                         }
-                        units.push_back(e);
+                        units.push_back(u);
                         ++number;
                     }
                     q0 = s + 1;
@@ -1154,12 +1166,13 @@ void Builder::subsample() {
                 units.back().flags |= 1u << 9;
             }
             const uint64_t count = units.size() - unit_first[l];
-            if (count) mean_candidates[l] = (uint32_t)(candidates / count);
+            mean_candidates[l] = count ? (uint32_t)(candidates / count) : 0;
             if (words * 4 > map_room) spread[l] = 0;
             if (spread[l]) map_words = std::max(map_words, words);
         }
         unit_first[depth_ + 1] = (uint32_t)units.size();
-    }
+    };
+    if (octants) lay_out_units(false);
 
     // ---- capacities: the staging arrays hold every level's candidates
     // (N + P_out at most, bounded by the reference's output capacity) and the
@@ -1194,18 +1207,20 @@ void Builder::subsample() {
     const size_t table_bytes = (size_t)n_internal * sizeof(SubNode);
     const size_t o_post = (table_bytes + 15) & ~(size_t)15;
     const size_t o_units = (o_post + (size_t)n_internal * 4 + 15) & ~(size_t)15;
-    const size_t o_oct_unit = units.size() * sizeof(UnitEntry);   // units, then octant tables
-    const size_t units_bytes = o_oct_unit + oct_unit.size() * 4;
-    table_host_.ensure(o_units + units_bytes + 16);
-    if (n_internal) {
+    size_t o_oct_unit = 0, units_bytes = 0;   // units, then octant tables
+    auto stage_tables = [&]() {
+        o_oct_unit = units.size() * sizeof(UnitEntry);
+        units_bytes = o_oct_unit + oct_unit.size() * 4;
+        table_host_.ensure(o_units + units_bytes + 16);
+        if (!n_internal) return;
         std::memcpy(table_host_.p, table.data(), table_bytes);
         std::memcpy(table_host_.as<uint8_t>(o_post), post.data(), (size_t)n_internal * 4);
-        if (octants) {
-            std::memcpy(table_host_.as<uint8_t>(o_units), units.data(), o_oct_unit);
-            if (!oct_unit.empty())
-                std::memcpy(table_host_.as<uint8_t>(o_units + o_oct_unit), oct_unit.data(), oct_unit.size() * 4);
-        }
-    }
+        if (!octants) return;
+        std::memcpy(table_host_.as<uint8_t>(o_units), units.data(), o_oct_unit);
+        if (!oct_unit.empty())
+            std::memcpy(table_host_.as<uint8_t>(o_units + o_oct_unit), oct_unit.data(), oct_unit.size() * 4);
+    };
+    stage_tables();
     post_ii_.ensure(std::max<size_t>((size_t)n_internal * 4, 4));
     sub_nodes_.ensure(std::max<size_t>(table_bytes, sizeof(SubNode)));
     if (n_internal)
@@ -1228,20 +1243,28 @@ void Builder::subsample() {
     level_base_.ensure(8);
     work_.ensure(4);
 
-    for (int attempt = 0;; ++attempt) {
+    // Octants: whether the pass looks for points outside their octants before
+    // each level (k_foreign), and the first level that it has to do.
+    bool foreign = false;
+    uint32_t from_level = 1;
+    for (int attempt = 0, grown = 0;; ++attempt) {
         // Octant subsampling works in the buffers of the other kernels (a
         // server's lane serves both): staged colours and face sums in the
         // record staging (8 + 8 of its 18 bytes), face lists in key cache and
         // cell list, weighted sums of face cells in the cell-unit cache, the
         // bitmaps of spread levels (at most 3 x SMs units, parts of 8 KB or
-        // whole octants of 64 KB) in a brick table.
+        // whole octants of 64 KB) and the list of points outside their octants
+        // in a brick table.
         if (octants) {
             if (cfg_.random) acc_best_.ensure(scratch_cap * 8);
             if (averaged) stage_rec_.ensure(stage_cap * 18 + 64);
             if (inter) key_cache_.ensure(scratch_cap * 8);
             units_.ensure(std::max<size_t>(units_bytes, sizeof(UnitEntry)));
-            unit_sync_.ensure(kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 12);
+            unit_sync_.ensure_keep(kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 12 +
+                                       (foreign ? (size_t)n_internal * 32 : 0),
+                                   kUnitSyncHead, stream_);
             if (map_words) g_mask_.ensure(map_words * 4);
+            if (foreign) g_key_.ensure((size_t)num_sms_ * memory_terms(cfg_, num_sms_).slots * 4);
             oct_off_.ensure((size_t)n_internal * 32 + 32);
         } else {
             size_brick_tables();
@@ -1266,7 +1289,7 @@ void Builder::subsample() {
         if (copy_stream_) check_cuda(cudaStreamSynchronize(copy_stream_), "output copies");
         lut_.ensure_keep(rec_cap * 4, (size_t)cfg_.n * 4, stream_);
         rec_.ensure_keep(rec_cap * 18 + 16, (size_t)cfg_.n * 18, stream_);
-        if (host_rec_) {
+        if (host_rec_ && attempt == 0) {
             // leaf records (and LUT entries) are final: stream them to the
             // caller's arrays while the levels are subsampled
             check_cuda(cudaEventRecord(leaf_ready_, stream_), "event");
@@ -1324,8 +1347,10 @@ void Builder::subsample() {
                 check_cuda(cudaMemcpyAsync(units_.p, table_host_.as<uint8_t>(o_units), units_bytes,
                                            cudaMemcpyHostToDevice, stream_),
                            "H2D units");
-            check_cuda(cudaMemsetAsync(unit_sync_.p, 0,
-                                       kUnitSyncHead + (size_t)n_internal * sizeof(UnitNodeState) + units.size() * 8,
+            // (the slots that levels below from_level took stay)
+            check_cuda(cudaMemsetAsync(unit_sync_.as<uint64_t>() + from_level, 0,
+                                       kUnitSyncHead - from_level * 8 + (size_t)n_internal * sizeof(UnitNodeState) +
+                                           units.size() * 8,
                                        stream_),
                        "memset");
             uint64_t largest_unit = S3;
@@ -1333,7 +1358,10 @@ void Builder::subsample() {
             uint8_t* sync = unit_sync_.as<uint8_t>();
             UnitNodeState* node_state = reinterpret_cast<UnitNodeState*>(sync + kUnitSyncHead);
             uint64_t* unit_state = reinterpret_cast<uint64_t*>(node_state + n_internal);
-            for (uint32_t l = 1; l <= depth_; ++l) {
+            uint32_t* unit_rank = reinterpret_cast<uint32_t*>(unit_state + units.size());
+            uint32_t* heads = unit_rank + units.size();
+            if (foreign) check_cuda(cudaMemsetAsync(heads, 0, (size_t)n_internal * 32, stream_), "memset");
+            for (uint32_t l = from_level; l <= depth_; ++l) {
                 const uint32_t first = level_first[l], cnt = level_first[l + 1] - first;
                 if (!cnt) continue;
                 UnitLevelArgs u{};
@@ -1359,7 +1387,7 @@ void Builder::subsample() {
                 u.oct_off = oct_off_.as<uint32_t>();
                 u.node_state = node_state + first;
                 u.unit_state = unit_state + unit_first[l];
-                u.unit_rank = reinterpret_cast<uint32_t*>(unit_state + units.size()) + unit_first[l];
+                u.unit_rank = unit_rank + unit_first[l];
                 u.spread = spread[l];
                 u.oct_unit = reinterpret_cast<const uint32_t*>(units_.as<uint8_t>() + o_oct_unit) + oct_first[l];
                 u.maps = g_mask_.as<uint32_t>();
@@ -1379,6 +1407,13 @@ void Builder::subsample() {
                 u.ticket = reinterpret_cast<uint32_t*>(sync + 128) + l;
                 u.wait_limit = unit_wait_limit(cfg_.debug, largest_unit);
                 u.err = err_.as<uint32_t>();
+                if (foreign) {
+                    u.foreign_head = heads + (size_t)first * 8;
+                    u.foreign = g_key_.as<uint4>();
+                    u.foreign_used = reinterpret_cast<uint32_t*>(sync + 320);
+                    u.foreign_cap = (uint32_t)std::min<uint64_t>(g_key_.bytes / sizeof(uint4), 0x7FFFFFFF);
+                    launches_ += launch_foreign(u, averaged, num_sms_, stream_);
+                }
                 launches_ += launch_units_level(u, mode, mean_candidates[l], any_split[l], num_sms_, stream_);
                 char mark[32];
                 std::snprintf(mark, sizeof mark, "sub_l%u", l);
@@ -1454,7 +1489,7 @@ void Builder::subsample() {
                                       n_internal, stage_rec_.as<uint8_t>(), rec_.as<uint8_t>(), stream_);
         stage_mark("place");
         check_cuda(cudaGetLastError(), "subsample launch");
-        check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(0), err_.p, 4, cudaMemcpyDeviceToHost, stream_), "D2H err");
+        check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(0), err_.p, 8, cudaMemcpyDeviceToHost, stream_), "D2H err");
         check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(8), level_base_.p, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
         check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(16), out_total_.p, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
         if (n_internal) {
@@ -1481,12 +1516,21 @@ void Builder::subsample() {
             throw_device_errors(e, (e & kErrCapacity) ? "subsample" : "generate");
         }
         p_out_ = *back_host_.as<uint64_t>(16);
-        if ((e & kErrForeign) && attempt < 6 && !(e & ~(kErrForeign | kErrCapacity))) {
-            // a point that two levels' formulas put on different sides of an
-            // octant boundary: the pass is repeated by the kernels of whole nodes
-            octants = false;
-            const uint32_t none = 0;
-            check_cuda(cudaMemcpyAsync(err_.p, &none, 4, cudaMemcpyHostToDevice, stream_), "H2D err");
+        if (e & kErrForeign) {
+            // Points that two levels' formulas put on different sides of an
+            // octant boundary: the level that met them and those above it are
+            // done again with such points handed to the units their cells are
+            // in.  More of them than the list holds: the kernels of whole nodes.
+            if (!foreign) {
+                foreign = true;
+                from_level = std::max(back_host_.as<uint32_t>(0)[1], 1u);
+                lay_out_units(true);
+            } else {
+                octants = false;
+            }
+            stage_tables();
+            check_cuda(cudaMemsetAsync(err_.p, 0, 8, stream_), "memset");
+            stage_mark(octants ? "repeat_octants" : "repeat_nodes");
             continue;
         }
         if (!(e & kErrCapacity)) {
@@ -1500,7 +1544,8 @@ void Builder::subsample() {
             stats_.subsample_passes = (uint32_t)attempt + 1;
             break;
         }
-        if (attempt >= 6 || (e & ~kErrCapacity)) check_device_errors("subsample");
+        if (++grown > 6) check_device_errors("subsample");
+        from_level = 1;
         // a level or the final records did not fit: grow and repeat the pass
         stage_cap *= 2;
         scratch_cap = std::min<uint64_t>(scratch_cap * 2, std::max(max_level_bound, scratch_cap));

@@ -128,7 +128,7 @@ enum : uint32_t {
     kErrTag = 1u << 4,           // a point found no leaf
     kErrTimeout = 1u << 5,       // a bounded wait (on a bulk copy, on an earlier unit) gave up
     kErrNodeCap = 1u << 6,       // the tree has more nodes than the node table holds
-    kErrForeign = 1u << 7,       // a candidate's cell lies outside its child's octant (the pass is repeated)
+    kErrForeign = 1u << 7,       // a candidate's cell lies outside its child's octant (word 1: the level; the pass is repeated)
 };
 
 // Any of these leaves a level without whole outputs: what reads them does not

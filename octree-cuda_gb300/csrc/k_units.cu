@@ -23,8 +23,9 @@
 // that, halved.  Bit 31 of a word says that the proof holds at every level;
 // without it the cell is evaluated from the cloud point in binary64.  When that
 // lands outside the unit (a point on an octant boundary that the two levels
-// round differently) kErrForeign is set and the build subsamples again with the
-// kernels of k_subsample.cu.
+// round differently; common where coordinates are multiples of a scale and the
+// box is too) kErrForeign is set, and the levels from this one on are done again
+// with such points handed to the units of their cells (k_foreign).
 //
 // What a level writes per output point: cloud index, cell word and (averaged
 // modes) colour, 8 to 16 bytes instead of the 18-byte record; k_place_units
@@ -207,7 +208,7 @@ __device__ __forceinline__ void append_faces(const UnitLevelArgs& a, uint32_t no
 struct BlockShared {
     Unit un;
     uint32_t warp[32];
-    uint32_t unit, unsafe, rank0, cand0, included, next, fail, redo, stop;
+    uint32_t unit, unsafe, foreign, rank0, cand0, included, next, fail, redo, stop;
     int32_t delta;
     uint64_t off, level_base;
 };
@@ -225,16 +226,46 @@ struct WeightShared {
     uint2 rows[kWeightThreads / kWeightLanes][9];
 };
 
-// Node-grid cell of a candidate without the proof, as coordinates; ~0 when
-// it is not the unit's.
-__device__ __noinline__ uint32_t unproven_cell(const UnitLevelArgs& a, const Unit& un, uint32_t idx) {
+// Node-grid cell of a candidate without the proof, as coordinates; foreign
+// when it is not the unit's.
+__device__ __noinline__ uint32_t node_cell(const UnitLevelArgs& a, const Unit& un, uint32_t idx, bool& foreign) {
     const uint32_t f = exact_cell(a, a.nodes[un.node], idx);
     const uint32_t x = f & 127, y = (f >> kFieldBits) & 127, z = f >> (2 * kFieldBits), b = un.b;
     const uint32_t h = a.s - 1;
     const bool other = (((x >> h) << 2) | ((y >> h) << 1) | (z >> h)) != un.octant;
     const bool part = un.part && ((((x >> b) & 1) << 2) | (((y >> b) & 1) << 1) | ((z >> b) & 1)) != un.part - 8;
-    if (other || part) atomicOr(a.err, kErrForeign);
-    return other || part ? ~0u : f;
+    foreign = other || part;
+    return f;
+}
+
+// The same with ~0 for a foreign candidate: k_foreign has handed it to the unit
+// its cell is in, or the pass is repeated with that, from this level.
+__device__ __forceinline__ uint32_t unproven_cell(const UnitLevelArgs& a, const Unit& un, uint32_t idx) {
+    bool foreign;
+    const uint32_t f = node_cell(a, un, idx, foreign);
+    if (!foreign) return f;
+    if (!a.foreign_head) {
+        a.err[1] = a.level;
+        atomicOr(a.err, kErrForeign);
+    }
+    return ~0u;
+}
+
+// Calls get(cell in the unit's box as Box::cell takes it, cloud index, r | g <<
+// 16, b) for the points of other units whose cell lies in this one: the block's
+// threads take the points of one segment after the other.
+template <class Get>
+__device__ __forceinline__ void foreign_points(const UnitLevelArgs& a, const Unit& un, uint32_t head, Get&& get) {
+    for (uint32_t seg = head; seg;) {
+        const uint4 h = a.foreign[seg - 1];
+        for (uint32_t k = threadIdx.x; k < h.y; k += blockDim.x) {
+            const uint4 e = a.foreign[seg + k];
+            const uint32_t b = un.b, x = e.x & 127, y = (e.x >> kFieldBits) & 127, z = e.x >> (2 * kFieldBits);
+            if (un.part && ((((x >> b) & 1) << 2) | (((y >> b) & 1) << 1) | ((z >> b) & 1)) != un.part - 8) continue;
+            get(e.x, e.y, e.z, e.w);
+        }
+        seg = h.x;
+    }
 }
 
 // Waits for the counts of the node's earlier units and the node's place
@@ -346,7 +377,7 @@ __device__ __forceinline__ uint32_t weighted_mean(uint64_t sum, uint64_t weight)
 // hold.  (A lane per cell, or lanes sharing each neighbour's points, waits
 // for the longest list: the weight of a pair costs about 45 instructions.)
 // Colours are of 8 bits here: the cloud's, or means of those.
-template <int T, bool kRandom, int kB, bool kLocal, class Pre>
+template <int T, bool kRandom, int kB, bool kLocal, bool kForeign, class Pre>
 __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box,
                                               const uint64_t* l_key, const uint32_t* l_word, uint32_t* l_cnt,
                                               uint32_t cells, const int (&keep)[4], uint64_t so, uint64_t oo,
@@ -388,6 +419,26 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
         const uint64_t start = un.start;
         const uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
         const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
+        // the weight measures the distance from the point itself to each
+        // neighbour cell centre (kernel_inter_cell_filtering.cuh:171-176)
+        auto cell_units = [&](uint32_t idx) {
+            Coord co[3];
+            uint32_t col[3];
+            float4 v;
+            const uint8_t* p = a.cloud + (uint64_t)idx * a.stride;
+            if (a.float_input) {
+                gather_point<true, false>(p, co, col);
+                v.x = point_units<true>(co[0], nd.ax[0]);
+                v.y = point_units<true>(co[1], nd.ax[1]);
+                v.z = point_units<true>(co[2], nd.ax[2]);
+            } else {
+                gather_point<false, false>(p, co, col);
+                v.x = point_units<false>(co[0], nd.ax[0]);
+                v.y = point_units<false>(co[1], nd.ax[1]);
+                v.z = point_units<false>(co[2], nd.ax[2]);
+            }
+            return v;
+        };
         for (uint32_t k0 = tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -407,23 +458,7 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
                     if (mine) i = (int)box.cell(f);
                 }
                 if (i < 0) continue;
-                // the weight measures the distance from the point itself to
-                // each neighbour cell centre (kernel_inter_cell_filtering.cuh:171-176)
-                Coord co[3];
-                uint32_t col[3];
-                float4 v;
-                const uint8_t* p = a.cloud + (uint64_t)idx * a.stride;
-                if (a.float_input) {
-                    gather_point<true, false>(p, co, col);
-                    v.x = point_units<true>(co[0], nd.ax[0]);
-                    v.y = point_units<true>(co[1], nd.ax[1]);
-                    v.z = point_units<true>(co[2], nd.ax[2]);
-                } else {
-                    gather_point<false, false>(p, co, col);
-                    v.x = point_units<false>(co[0], nd.ax[0]);
-                    v.y = point_units<false>(co[1], nd.ax[1]);
-                    v.z = point_units<false>(co[2], nd.ax[2]);
-                }
+                float4 v = cell_units(idx);
                 uint32_t c;
                 if (staged) {
                     const uint2 q = *reinterpret_cast<const uint2*>(a.stage_col + start + k);
@@ -436,6 +471,12 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
                 a.csr_pts[c0 + atomicAdd(cur + box.rank((uint32_t)i), 1u)] = v;
             }
         }
+        if (kForeign && sh.foreign)
+            foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t rg, uint32_t bl) {
+                float4 v = cell_units(idx);
+                v.w = __uint_as_float((rg & 0xFFu) | ((rg >> 8) & 0xFF00u) | (bl << 16));
+                a.csr_pts[c0 + atomicAdd(cur + box.rank(box.cell(f)), 1u)] = v;
+            });
     }
     __syncthreads();
     auto cell_end = [&](uint32_t r) { return kLocal ? cur[r] : __ldcg(cur + r); };
@@ -555,7 +596,7 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
 // sums beyond 16 bits) in the staging arrays and the level's scratch, reached
 // by reductions.  keep: the cells of this thread's first four candidates.
 // Returns false (every thread alike) when a local unit has to be redone.
-template <int T, int kColor, bool kRandom, int kB, bool kLocal, class Pre>
+template <int T, int kColor, bool kRandom, int kB, bool kLocal, bool kForeign, class Pre>
 __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box, uint32_t* pool,
                                            uint32_t ui, uint32_t cells, const int (&keep)[4], uint32_t claim,
                                            uint32_t included, bool placed, WeightShared* ws) {
@@ -607,6 +648,34 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
         const uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
         const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
         uint32_t wide = 0;   // colour bits above 8
+        auto add = [&](uint32_t rank, uint32_t idx, uint32_t c0, uint32_t c1) {
+            if (kRandom) {
+                const SubNode& nd = a.nodes[un.node];
+                const unsigned long long key =
+                    ((unsigned long long)rp_priority(a.seed, nd.level, nd.morton, idx) << 32) | idx;
+                if (!kLocal) atomicMin(reinterpret_cast<unsigned long long*>(a.best + so + rank), key);
+                else if (key < *(volatile uint64_t*)&l_key[rank])
+                    atomicMin(reinterpret_cast<unsigned long long*>(l_key + rank), key);
+            } else if (kLocal) {
+                atomicMin(l_idx + rank, idx);
+            } else {
+                atomicMin(a.stage_lut + oo + rank, idx);
+            }
+            if (averaged) {
+                if (kLocal) {
+                    // r | g << 16 and b | 1 << 20: exact while the cell has at
+                    // most 257 candidates with colours of 8 bits (checked below)
+                    atomicAdd(&l_sum[rank].x, c0);
+                    atomicAdd(&l_sum[rank].y, c1 | (1u << 20));
+                    wide |= (c0 & 0xFF00FF00u) | (c1 & 0xFF00u);
+                } else {
+                    atomicAdd(reinterpret_cast<unsigned long long*>(kColor == 1 ? a.stage_col + oo + rank
+                                                                                : a.sum + so + rank),
+                              (unsigned long long)encode_colors(c0 & 0xFFFFu, c0 >> 16, c1));
+                }
+            }
+            if (weighted) atomicAdd(kLocal ? l_cnt + rank : a.csr_count + so + rank, 1u);
+        };
         for (uint32_t k0 = tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
             uint32_t idx[4], c0[4], c1[4];
             int i[4];
@@ -650,32 +719,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
             for (int j = 0; j < 4; ++j) {
                 if (i[j] < 0) continue;
                 const uint32_t rank = box.rank((uint32_t)i[j]);
-                if (kRandom) {
-                    const SubNode& nd = a.nodes[un.node];
-                    const unsigned long long key =
-                        ((unsigned long long)rp_priority(a.seed, nd.level, nd.morton, idx[j]) << 32) | idx[j];
-                    if (!kLocal) atomicMin(reinterpret_cast<unsigned long long*>(a.best + so + rank), key);
-                    else if (key < *(volatile uint64_t*)&l_key[rank])
-                        atomicMin(reinterpret_cast<unsigned long long*>(l_key + rank), key);
-                } else if (kLocal) {
-                    atomicMin(l_idx + rank, idx[j]);
-                } else {
-                    atomicMin(a.stage_lut + oo + rank, idx[j]);
-                }
-                if (averaged) {
-                    if (kLocal) {
-                        // r | g << 16 and b | 1 << 20: exact while the cell has at
-                        // most 257 candidates with colours of 8 bits (checked below)
-                        atomicAdd(&l_sum[rank].x, c0[j]);
-                        atomicAdd(&l_sum[rank].y, c1[j] | (1u << 20));
-                        wide |= (c0[j] & 0xFF00FF00u) | (c1[j] & 0xFF00u);
-                    } else {
-                        atomicAdd(reinterpret_cast<unsigned long long*>(kColor == 1 ? a.stage_col + oo + rank
-                                                                                    : a.sum + so + rank),
-                                  (unsigned long long)encode_colors(c0[j] & 0xFFFFu, c0[j] >> 16, c1[j]));
-                    }
-                }
-                if (weighted) atomicAdd(kLocal ? l_cnt + rank : a.csr_count + so + rank, 1u);
+                add(rank, idx[j], c0[j], c1[j]);
                 if (it + j >= 32 || (claim >> (it + j)) & 1u) {
                     const uint32_t wd = (kSafeWord | base) + box.coordinates((uint32_t)i[j]);
                     if (kLocal) l_word[rank] = wd;
@@ -683,6 +727,10 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                 }
             }
         }
+        if (kForeign && sh.foreign)
+            foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t c0, uint32_t c1) {
+                add(box.rank(box.cell(f)), idx, c0, c1);
+            });
         if (kLocal && averaged && wide) sh.redo = 1;
         __syncthreads();
         // a cell that any candidate without the proof falls in loses it
@@ -695,6 +743,12 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                 if (kLocal) l_word[box.rank(i)] = base + box.coordinates(i);
                 else a.stage_word[oo + box.rank(i)] = base + box.coordinates(i);
             }
+            if (kForeign && sh.foreign)
+                foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t, uint32_t, uint32_t) {
+                    const uint32_t i = box.cell(f);
+                    if (kLocal) l_word[box.rank(i)] = base + box.coordinates(i);
+                    else a.stage_word[oo + box.rank(i)] = base + box.coordinates(i);
+                });
         }
     }
     // ---- the sums as the packed words of the reference; a count field that
@@ -730,7 +784,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
     const uint64_t* g_packed = a.sum + so;
     const uint32_t m0 = box.m0(), open = un.open;
     if constexpr (weighted) {
-        unit_weighted<T, kRandom, kB, kLocal, Pre>(a, sh, box, l_key, l_word, l_cnt, cells, keep, so, oo, *ws);
+        unit_weighted<T, kRandom, kB, kLocal, kForeign, Pre>(a, sh, box, l_key, l_word, l_cnt, cells, keep, so, oo, *ws);
     } else {
         for (uint32_t r0 = warp * 32; r0 < cells; r0 += T) {
             const uint32_t r = r0 + lane;
@@ -777,18 +831,19 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
 // seldom need it: inlined, its registers weigh on the other variant's (level
 // 4 of the 119.7M-point build 1.34 -> 1.27 ms; two blocks per SM, which
 // need it often, lose by it: level 1 0.84 -> 1.13 ms).
-template <int T, int kColor, bool kRandom, int kB, class Pre>
+template <int T, int kColor, bool kRandom, int kB, bool kForeign, class Pre>
 __device__ __noinline__ void unit_cells_global(const UnitLevelArgs& a, BlockShared& sh, const uint32_t* bm,
                                                const Pre* pre, uint32_t b, uint32_t ui, uint32_t cells, int4 keep4,
                                                uint32_t claim, uint32_t included, bool placed) {
     const int keep[4] = {keep4.x, keep4.y, keep4.z, keep4.w};
     const Box<kB, Pre> box{bm, pre, b};
-    unit_cells<T, kColor, kRandom, kB, false, Pre>(a, sh, box, nullptr, ui, cells, keep, claim, included, placed,
-                                                   nullptr);
+    unit_cells<T, kColor, kRandom, kB, false, kForeign, Pre>(a, sh, box, nullptr, ui, cells, keep, claim, included,
+                                                             placed, nullptr);
 }
 
-// One unit: pass A, ranks, then its cells.
-template <int T, int kColor, bool kRandom, int kB, class Pre>
+// One unit: pass A, ranks, then its cells.  kForeign: points of other units
+// may have their cells here.
+template <int T, int kColor, bool kRandom, int kB, bool kForeign, class Pre>
 __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh, uint32_t* bm, uint32_t ui,
                                          WeightShared* ws) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -856,6 +911,14 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                 if (!(old & bit) && it + j < 32) claim |= 1u << (it + j);
             }
         }
+        if (kForeign && sh.foreign) {
+            unsafe = true;
+            foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t, uint32_t, uint32_t) {
+                const uint32_t i = box.cell(f);
+                ++included;
+                atomicOr(&bm[i >> 5], 1u << (i & 31));
+            });
+        }
         if (unsafe) sh.unsafe = 1;
         if (kColor == 3) {
             const uint32_t n = __reduce_add_sync(0xffffffffu, included);
@@ -920,26 +983,96 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
     const uint32_t room = a.smem_words * 4 - (uint32_t)((pool - bm) * 4);
     bool placed = false;
     if (sizeof(Pre) == 2 && cells * cell_bytes(kColor, kRandom) <= room) {
-        if (unit_cells<T, kColor, kRandom, kB, true, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, false, ws)) return;
+        if (unit_cells<T, kColor, kRandom, kB, true, kForeign, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, false, ws))
+            return;
         placed = true;
         __syncthreads();
     }
     if constexpr (T == 1024)
-        unit_cells_global<T, kColor, kRandom, kB, Pre>(a, sh, bm, pre, b, ui, cells,
+        unit_cells_global<T, kColor, kRandom, kB, kForeign, Pre>(a, sh, bm, pre, b, ui, cells,
                                                        make_int4(keep[0], keep[1], keep[2], keep[3]), claim, included,
                                                        placed);
     else
-        unit_cells<T, kColor, kRandom, kB, false, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, placed, ws);
+        unit_cells<T, kColor, kRandom, kB, false, kForeign, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, placed,
+                                                                 ws);
 }
 
-// Units of other kinds than the level's frequent ones, out of line, so that
+// Units of other kinds than the level's frequent ones (among them those with
+// points from other units), out of line, so that
 // their registers do not weigh on those (see launch_units).
 template <int T, int kColor, bool kRandom>
 __device__ __noinline__ void unit_run_other(const UnitLevelArgs& a, BlockShared& sh, uint32_t* bm, uint32_t ui,
                                             WeightShared* ws) {
-    if (sh.un.b == 6) unit_run<T, kColor, kRandom, 6, uint32_t>(a, sh, bm, ui, ws);
-    else if (sh.un.b == 5) unit_run<T, kColor, kRandom, 5, uint16_t>(a, sh, bm, ui, ws);
-    else unit_run<T, kColor, kRandom, 0, uint16_t>(a, sh, bm, ui, ws);
+    if (sh.un.b == 6) unit_run<T, kColor, kRandom, 6, true, uint32_t>(a, sh, bm, ui, ws);
+    else if (sh.un.b == 5) unit_run<T, kColor, kRandom, 5, true, uint16_t>(a, sh, bm, ui, ws);
+    else unit_run<T, kColor, kRandom, 0, true, uint16_t>(a, sh, bm, ui, ws);
+}
+
+// The level's points whose cell lies outside their unit, as a segment per unit
+// (or chunk of one) and octant they belong to.  Reads the words of all
+// candidates, for builds that were found to have such points.
+constexpr int kForeignThreads = 256;
+
+__global__ void __launch_bounds__(kForeignThreads) k_foreign(const __grid_constant__ UnitLevelArgs a, uint32_t chunks,
+                                                             uint32_t colour) {
+    __shared__ uint32_t s_count[8], s_at[8], s_stop;
+    constexpr uint32_t T = kForeignThreads;
+    const uint32_t tid = threadIdx.x;
+    if (tid == 0) s_stop = *(volatile uint32_t*)a.err;
+    __syncthreads();
+    if (s_stop) return;
+    for (uint32_t item = blockIdx.x; item < a.n_units * chunks; item += gridDim.x) {
+        const Unit un = load_unit(a, item / chunks);
+        const uint32_t per = un.cnt / chunks + 1, first = min(item % chunks * per, un.cnt), end = min(first + per, un.cnt);
+        const uint32_t* word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
+        const uint32_t* lut = (un.staged ? a.stage_lut : a.leaf_lut) + un.start;
+        auto points = [&](auto&& get) {
+            for (uint32_t k0 = first + tid; k0 < end; k0 += 4 * T) {
+                uint32_t w[4];
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) w[j] = k0 + j * T < end ? word[k0 + j * T] : kSafeWord;
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    if (w[j] >> 31) continue;
+                    bool foreign;
+                    const uint32_t f = node_cell(a, un, lut[k0 + j * T], foreign), h = a.s - 1;
+                    const uint32_t x = f & 127, y = (f >> kFieldBits) & 127, z = f >> (2 * kFieldBits);
+                    if (foreign) get(k0 + j * T, f, ((x >> h) << 2) | ((y >> h) << 1) | (z >> h));
+                }
+            }
+        };
+        if (tid < 8) s_count[tid] = 0;
+        __syncthreads();
+        points([&](uint32_t, uint32_t, uint32_t o) { atomicAdd(&s_count[o], 1u); });
+        __syncthreads();
+        if (tid < 8 && s_count[tid]) {
+            const uint32_t n = s_count[tid], at = atomicAdd(a.foreign_used, n + 1);
+            if ((uint64_t)at + n + 1 > a.foreign_cap) {
+                atomicOr(a.err, kErrForeign);   // no room: the kernels of whole nodes
+                s_at[tid] = ~0u;
+            } else {
+                a.foreign[at] = make_uint4(atomicExch(&a.foreign_head[un.node * 8 + tid], at + 1), n, 0, 0);
+                s_at[tid] = at + 1;
+            }
+        }
+        const bool any = __syncthreads_or(tid < 8 && s_count[tid]);
+        if (any)
+            points([&](uint32_t k, uint32_t f, uint32_t o) {
+                if (s_at[o] == ~0u) return;
+                uint32_t c0 = 0, c1 = 0;
+                if (colour && un.staged) {
+                    const uint2 v = *reinterpret_cast<const uint2*>(a.stage_col + un.start + k);
+                    c0 = v.x;
+                    c1 = v.y;
+                } else if (colour) {
+                    const uint16_t* v = reinterpret_cast<const uint16_t*>(a.leaf_rec + (un.start + k) * 18 + 12);
+                    c0 = v[0] | ((uint32_t)v[1] << 16);
+                    c1 = v[2];
+                }
+                a.foreign[atomicAdd(&s_at[o], 1u)] = make_uint4(f, lut[k], c0, c1);
+            });
+        __syncthreads();
+    }
 }
 
 // kColor: 0 raw colour, 1 intra-cell, 2 inter-cell, 3 distance-weighted.  An
@@ -969,7 +1102,10 @@ __global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_consta
             sh.unit = u;
             sh.unsafe = 0;
             sh.included = 0;
-            if (u < a.n_units) sh.un = load_unit(a, u);
+            if (u < a.n_units) {
+                sh.un = load_unit(a, u);
+                sh.foreign = a.foreign_head ? a.foreign_head[sh.un.node * 8 + sh.un.octant] : 0u;
+            }
         }
         __syncthreads();
         const uint32_t ui = sh.unit;
@@ -977,8 +1113,9 @@ __global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_consta
         if (kColor != 3 && tid == T - 33 && a.n_units - ui > gridDim.x) prefetch_unit<kColor>(a, ui + gridDim.x);
         // (the weighted lists follow the pool)
         WeightShared* ws = reinterpret_cast<WeightShared*>(dyn + a.smem_words);
-        if (sh.un.b == 6 && sh.un.cnt <= 65535) unit_run<T, kColor, kRandom, 6, uint16_t>(a, sh, dyn, ui, ws);
-        else if (kHalf && sh.un.b == 5) unit_run<T, kColor, kRandom, 5, uint16_t>(a, sh, dyn, ui, ws);
+        if (sh.foreign) unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
+        else if (sh.un.b == 6 && sh.un.cnt <= 65535) unit_run<T, kColor, kRandom, 6, false, uint16_t>(a, sh, dyn, ui, ws);
+        else if (kHalf && sh.un.b == 5) unit_run<T, kColor, kRandom, 5, false, uint16_t>(a, sh, dyn, ui, ws);
         else unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
     }
 }
@@ -1550,6 +1687,17 @@ int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_cand
                     : (mode & kModeInter)                              ? launch_units_inter
                                                                        : launch_units_raw;
     return go(a, (mode & kModeRandom) != 0, mean_candidates, any_split, num_sms, stream);
+}
+
+int launch_foreign(const UnitLevelArgs& a, bool colour, int num_sms, cudaStream_t stream) {
+    if (!a.n_units) return 0;
+    // up to eight blocks per SM; units of a level of few are shared by up to 16
+    const uint64_t blocks = (uint64_t)std::max(num_sms, 1) * 8;
+    uint32_t chunks = 1;
+    while (chunks < 16 && (uint64_t)a.n_units * chunks < blocks) chunks <<= 1;
+    k_foreign<<<(unsigned)std::min<uint64_t>((uint64_t)a.n_units * chunks, blocks), kForeignThreads, 0, stream>>>(a, chunks,
+                                                                                                          colour);
+    return 1;
 }
 
 int launch_place_units(const uint64_t* src_off, const uint64_t* dst_off, const uint32_t* count, uint32_t n_nodes,

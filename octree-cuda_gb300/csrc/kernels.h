@@ -316,8 +316,9 @@ struct UnitNodeState {
 };
 
 // Head of the counters a pass starts from zero: level_used (16 x u64), the
-// tickets of the levels' launches (16 x u32), partials per level (16 x u64).
-constexpr size_t kUnitSyncHead = 320;
+// tickets of the levels' launches (16 x u32), partials per level (16 x u64),
+// entries of the foreign list (u32; 16 bytes).
+constexpr size_t kUnitSyncHead = 336;
 
 struct UnitLevelArgs {
     const SubNode* nodes;
@@ -364,6 +365,14 @@ struct UnitLevelArgs {
     uint64_t* partial;      // weighted sums (r, g, b, weight) of face cells over their own unit
     uint64_t* partials;     // entries taken
     uint64_t partial_cap;
+    // Points outside their octants (k_foreign), null while a pass does not
+    // expect any: per node and octant the first segment of those whose cell lies
+    // there, + 1.  A segment is {next segment + 1, points, -, -} and the points
+    // {cell, cloud index, r | g << 16, b}.
+    uint32_t* foreign_head;
+    uint4* foreign;
+    uint32_t* foreign_used;
+    uint32_t foreign_cap;
     uint32_t* ticket;
     int64_t wait_limit;     // clock cycles a unit waits for the node's earlier ones (negative: none, every wait fails)
     uint32_t* err;
@@ -397,6 +406,10 @@ inline int64_t unit_wait_limit(uint32_t debug, uint64_t largest_unit) {
 // launches: the units, then what their outermost cells get from other units.
 int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_candidates, bool any_split, int num_sms,
                        cudaStream_t stream);
+
+// Lists the level's points whose cell lies outside their unit, for the units it
+// lies in; before launch_units_level, in a pass that expects some.
+int launch_foreign(const UnitLevelArgs& a, bool colour, int num_sms, cudaStream_t stream);
 
 // The records of the internal nodes at their post-order positions, made from
 // the cloud points and the staged colours (see k_place_units).

@@ -179,3 +179,71 @@ def test_wait_that_runs_out(n, chunk, sub, mode):
     s.generate()
     compare_results(run_oracle(case, cfg), s)
     s.close()
+
+
+def foreign_side(sub, chunk=512, side=100.0):
+    """A box minimum and a coordinate at the middle of the root's upper child that the counting grid and the child's grid
+    put on different sides."""
+    rng = np.random.default_rng(12)
+    for _ in range(4000):
+        mn = float(rng.uniform(-60, 100))
+        p = np.array([mn + side * 0.75])
+        for _ in range(6):
+            p = np.unique(np.concatenate([p, np.nextafter(p, -np.inf), np.nextafter(p, np.inf)]))
+        a, b = middle_sides(p, mn, side, sub)
+        if (a != b).any():
+            return mn, p[a != b][0]
+    raise AssertionError("no such coordinate")
+
+
+def check_repeat(case, cfg, repeat):
+    """Against the oracle; `repeat`: what the pass was repeated with, by the names of the stages."""
+    ref = run_oracle(case, cfg)
+    s = run_gpu(case, cfg)
+    names = [k for k in s.timings() if k.startswith("repeat")]
+    compare_results(ref, s)
+    assert names == repeat and s.stats()["subsample_passes"] == 1 + len(repeat)
+    s.close()
+
+
+@pytest.mark.parametrize("mode", sorted(MODES))
+@pytest.mark.parametrize("chunk,sub,n", [(512, 128, 60_000), (512, 64, 20_000), (512, 16, 20_000)])
+def test_wall_in_another_octant(chunk, sub, n, mode):
+    """A wall whose points all belong to octants without a child, among other points."""
+    mn, p = foreign_side(sub)
+    xyz, rgb = points("volume", 2 * n)
+    xyz = xyz * 100.0
+    xyz[:, 0] += mn
+    xyz[:n, 0] = p
+    keep = (xyz[:, 0] < mn + 50.0) | (xyz[:, 0] == p)   # nothing else in the child's other half
+    case = case_from_points(xyz[keep], rgb[keep], 1, scale=0.01, bbox=[mn, 0, 0, mn + 100.0, 100.0, 100.0])
+    check_repeat(case, dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=700, output_factor=12.0, **MODES[mode]),
+                 ["repeat_octants"])
+
+
+def test_more_foreign_points_than_the_list_holds():
+    mn, p = foreign_side(8)
+    n = 90_000
+    xyz, rgb = points("volume", n)
+    xyz = xyz * 50.0          # all in one child of the root
+    xyz[:, 0] = p
+    case = case_from_points(xyz, rgb, 1, scale=0.01, bbox=[mn, 0, 0, mn + 100.0, 100.0, 100.0])
+    check_repeat(case, dict(chunk_grid=512, sub_grid=8, merge_threshold=80_000, output_factor=12.0, inter=True),
+                 ["repeat_octants", "repeat_nodes"])
+
+
+@pytest.mark.parametrize("mode", ["first", "first_intra", "first_inter", "random_inter", "first_weighted"])
+@pytest.mark.parametrize("off,side,chunk,sub", [(437000.0, 51.2, 64, 128), (123456.78, 51.2, 64, 32),
+                                                (0.1, 102.4, 128, 64), (5412345.67, 25.6, 32, 16)])
+def test_lattice_cloud(off, side, chunk, sub, mode):
+    """Coordinates that are multiples of 1 cm from an offset, as scans are stored, in a box whose octant planes are
+    among them."""
+    rng = np.random.default_rng(5)
+    n = 80_000
+    steps = int(round(side / 0.01))
+    q = rng.integers(0, steps, (n, 3))
+    q[:, 2] = (q[:, 0] // 7 + q[:, 1] // 5) % steps
+    rgb = rng.integers(0, 256, (n, 3), dtype=np.uint8)
+    case = case_from_points(off + q * 0.01, rgb, 1, scale=0.01, bbox=[off] * 3 + [off + side] * 3)
+    cfg = dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=600, output_factor=12.0, **MODES[mode])
+    check_repeat(case, cfg, ["repeat_octants"])
