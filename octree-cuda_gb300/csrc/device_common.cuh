@@ -131,10 +131,6 @@ enum : uint32_t {
     kErrForeign = 1u << 7,       // a candidate's cell lies outside its child's octant (word 1: the level; the pass is repeated)
 };
 
-// Any of these leaves a level without whole outputs: what reads them does not
-// run (the pass is repeated or the build fails).
-constexpr uint32_t kErrStop = kErrCapacity | kErrTimeout | kErrForeign;
-
 // ---------------------------------------------------------------------------
 // Ordered keys: monotone maps of IEEE bit patterns onto signed integers, so
 // that binary64 / binary32 values compare exactly as integers (negative

@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(1024) k_place_prepare(const uint32_t* __restri
                                                         uint64_t cap, uint64_t* src, uint64_t* dst, uint32_t* cnt,
                                                         uint64_t* node_dst, uint64_t* total, uint32_t* err) {
     __shared__ uint64_t warp_sums[32];
-    const bool skip = (*err & kErrStop) != 0;
+    const bool skip = *err != 0;   // (after any error levels may be without outputs)
     uint64_t running = 0;
     for (uint32_t k0 = 0; k0 < n_internal; k0 += blockDim.x) {
         const uint32_t k = k0 + threadIdx.x;

@@ -1499,7 +1499,7 @@ __global__ void __launch_bounds__(256) k_place_units(const uint64_t* __restrict_
     constexpr uint32_t kRun = 128;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint8_t* stage = s_stage + warp * kStageBytes;
-    if (*err & kErrStop) return;   // nothing was placed
+    if (*err) return;   // levels may be without outputs: nothing was placed
     const uint64_t end = n + *total;
     const uint64_t step = (uint64_t)gridDim.x * 8 * kRun;
     for (uint64_t p0 = n + ((uint64_t)blockIdx.x * 8 + warp) * kRun; p0 < end; p0 += step) {

@@ -247,3 +247,20 @@ def test_lattice_cloud(off, side, chunk, sub, mode):
     case = case_from_points(off + q * 0.01, rgb, 1, scale=0.01, bbox=[off] * 3 + [off + side] * 3)
     cfg = dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=600, output_factor=12.0, **MODES[mode])
     check_repeat(case, cfg, ["repeat_octants"])
+
+
+@pytest.mark.parametrize("sub", [64, 100])
+def test_output_coordinate_beyond_int32(sub):
+    """A scale for which the far points' output coordinates do not fit: an error found before subsampling, after which
+    nothing is subsampled or placed, and the session goes on."""
+    from helpers import octree_api
+
+    rng = np.random.default_rng(11)
+    xyz = np.round(rng.random((20_000, 3)) * 1000)
+    rgb = rng.integers(0, 256, (20_000, 3), dtype=np.uint8)
+    cfg = dict(chunk_grid=32, sub_grid=sub, merge_threshold=400, output_factor=12.0)
+    for scale in (1e-7, 1e-9):
+        case = case_from_points(xyz, rgb, 1, scale=scale, bbox=[0, 0, 0, 1000.0, 1000.0, 1000.0])
+        with pytest.raises(octree_api.OctreeError, match="does not fit int32"):
+            run_gpu(case, cfg)
+    check(case_from_points(xyz, rgb, 1, scale=0.001, bbox=[0, 0, 0, 1000.0, 1000.0, 1000.0]), cfg)
