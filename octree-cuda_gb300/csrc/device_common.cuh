@@ -317,11 +317,27 @@ __device__ __forceinline__ uint32_t pack_frac(uint32_t fx, uint32_t fy, uint32_t
 }
 
 // ---------------------------------------------------------------------------
-// Cell words of octant subsampling: bit 31 says that the cell is proven at
-// every level, bits 0-20 its coordinates x | y << 7 | z << 14 (a leaf's points:
-// in their parent's grid of 128^3 cells; an inner node's: in its own grid).
+// Cell words of octant subsampling: bits 0-20 the cell's coordinates x | y << 7 |
+// z << 14 (a leaf's points: in their parent's grid of 128^3 cells; an inner
+// node's: in its own grid), bits 21-25 how far up they hold.  A point beside a
+// boundary between finest cells that is a multiple of 2^(t-1), for its worst
+// axis, has t there (0: beside none; 31: no position): in grids of cells wider
+// than that its cell is that of its position, in others the binary64 formula
+// decides (unproven).  A unit leaves the result in the word: bit 30 set, the
+// log2 of its node's grid in bits 27-29, the coordinates in that grid, bit 31
+// when they lie outside the unit.
 
-constexpr uint32_t kSafeWord = 0x80000000u;
+constexpr uint32_t kWordEdge = 21;       // t
+constexpr uint32_t kWordEdges = 31u << kWordEdge;
+constexpr uint32_t kWordGrid = 27;       // log2 of the grid of a resolved word
+constexpr uint32_t kWordResolved = 1u << 30;
+constexpr uint32_t kWordForeign = 1u << 31;
+constexpr uint32_t kWordCell = (1u << 21) - 1;
+
+// t of the lowest set bit of a point's boundaries (the largest of its axes).
+__device__ __forceinline__ uint32_t word_edge(uint32_t low) {
+    return min(32u - __clz(low), 31u) << kWordEdge;
+}
 
 // Axis k of a cloud point from its words, as binary64.
 template <bool kFloatInput, int kWords>
@@ -335,24 +351,79 @@ __device__ __forceinline__ double word_coord_exact(const uint32_t (&w)[kWords], 
     return kFloatInput ? (double)__uint_as_float(w[k]) : __hiloint2double((int)w[2 * k + 1], (int)w[2 * k]);
 }
 
-// Quantised output coordinates of a cloud point: (int32_t)floor((p - min) * sf)
-// in binary64, kCoordError outside int32.
-template <bool kFloatInput, int kWords>
-__device__ __forceinline__ void fixed_out_coords(const uint32_t (&w)[kWords], const FixedGrid& f, const OutAxis (&o)[3],
-                                                 uint32_t* out) {
-    bool all = true;
+// 32-bit words w[0..kWords) of a record at any byte alignment in shared memory.
+template <int kWords>
+__device__ __forceinline__ void record_words(const uint8_t* rec, uint32_t (&w)[kWords]) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(rec);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+    const uint32_t s = (uint32_t)(a & 3) * 8;
+    uint32_t raw[kWords + 1];
+#pragma unroll
+    for (int j = 0; j <= kWords; ++j) raw[j] = q[j];
+#pragma unroll
+    for (int j = 0; j < kWords; ++j) w[j] = __funnelshift_r(raw[j], raw[j + 1], s);
+}
+
+// An output coordinate, (int32_t)floor((p - min) * sf) in binary64, kCoordError
+// outside int32; d: the position, `in` the box, by fixed_difference.
+// Coordinates that are multiples of the scale lie beside an integer each; where
+// the position shows that the result is an int32 that is three instructions of
+// the binary64 pipe.
+__device__ __forceinline__ int32_t fixed_out_coord(double p, bool in, uint64_t d, const FixedAxis& f, const OutAxis& o) {
+    bool proven;
+    const uint32_t q = fixed_units(d, f.out, proven);
+    if (in && proven && (int32_t)q >= 0) return (int32_t)q;
+    if (in && f.out.room && q < 0x7FFFFFF0u) return __double2int_rd(__dmul_rn(__dsub_rn(p, o.mn), o.sf));
+    return exact_out_coord(p, o.mn, o.sf);
+}
+
+// Output coordinates of a point beside an integer on some axis; out of line in
+// distribution, so that its registers do not weigh on the other points.
+struct OutCoords {
+    int32_t x, y, z;
+};
+
+template <bool kFloatInput>
+static __device__ __noinline__ OutCoords open_out_coords(const uint8_t* rec, const FixedGrid& f, const OutAxis* o) {
+    uint32_t w[kFloatInput ? 3 : 6];
+    record_words<kFloatInput ? 3 : 6>(rec, w);
+    int32_t q[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         uint64_t d;
-        bool proven;
-        all &= fixed_difference(word_coord<kFloatInput>(w, k), f.ax[k].o, d);
-        out[k] = fixed_units(d, f.ax[k].out, proven);
-        all &= proven && (int32_t)out[k] >= 0;
+        const bool in = fixed_difference(word_coord<kFloatInput>(w, k), f.ax[k].o, d);
+        q[k] = fixed_out_coord(word_coord_exact<kFloatInput>(w, k), in, d, f.ax[k], o[k]);
     }
-    if (all) return;
+    return {q[0], q[1], q[2]};
+}
+
+// Quantised output coordinates of a cloud point from its words.
+template <bool kFloatInput, int kWords>
+__device__ __forceinline__ void fixed_out_coords(const uint32_t (&w)[kWords], const FixedGrid& f, const OutAxis (&o)[3],
+                                                 uint32_t* out) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-        out[k] = (uint32_t)exact_out_coord(word_coord_exact<kFloatInput>(w, k), o[k].mn, o[k].sf);
+    for (int k = 0; k < 3; ++k) {
+        uint64_t d;
+        const bool in = fixed_difference(word_coord<kFloatInput>(w, k), f.ax[k].o, d);
+        out[k] = (uint32_t)fixed_out_coord(word_coord_exact<kFloatInput>(w, k), in, d, f.ax[k], o[k]);
+    }
+}
+
+// Finest cells of a point beside a boundary between cells on some axis, and the
+// lowest set bit of the boundary (see kWordEdge), the largest of the axes.
+template <bool kFloatInput>
+static __device__ __noinline__ uint4 boundary_cells(const uint8_t* rec, const FixedGrid& f) {
+    uint32_t w[kFloatInput ? 3 : 6], c[3], edge = 0;
+    record_words<kFloatInput ? 3 : 6>(rec, w);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        uint64_t d;
+        uint32_t boundary;
+        const bool in = fixed_difference(word_coord<kFloatInput>(w, k), f.ax[k].o, d);
+        c[k] = fixed_cell(d, f.ax[k].cell, f.cells, boundary);
+        edge = max(edge, in ? boundary & (0u - boundary) : 1u << 31);
+    }
+    return make_uint4(c[0], c[1], c[2], edge);
 }
 
 // ---------------------------------------------------------------------------

@@ -184,19 +184,6 @@ __device__ __forceinline__ void tile_loop(const uint8_t* __restrict__ cloud, uin
     }
 }
 
-// 32-bit words w[0..kWords) of a record at any byte alignment in shared memory.
-template <int kWords>
-__device__ __forceinline__ void record_words(const uint8_t* rec, uint32_t (&w)[kWords]) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(rec);
-    const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
-    const uint32_t s = (uint32_t)(a & 3) * 8;
-    uint32_t raw[kWords + 1];
-#pragma unroll
-    for (int j = 0; j <= kWords; ++j) raw[j] = q[j];
-#pragma unroll
-    for (int j = 0; j < kWords; ++j) w[j] = __funnelshift_r(raw[j], raw[j + 1], s);
-}
-
 // Cells of a point from its coordinate words (3 floats or 3 x lo/hi of
 // doubles), exactly as (int64)fmin((p - min) / t, G - 1) in binary64.
 // Returns false when the point lies below the bounding box.
@@ -743,8 +730,9 @@ __device__ __forceinline__ void group_clear(GroupSmem<kMode>& gs) {
 // registers, so that three 448-thread blocks share an SM (47 registers leave
 // room for two: 119.7M-point build 2.73 -> 2.56 ms).
 // kCells: the cell words of octant subsampling instead of sub-step words.  The
-// proven finest cell gives the counting cell as well (its upper bits), so the
-// boundary-key lookup is left out; an unproven point is evaluated in binary64.
+// finest cell gives the counting cell as well (its upper bits), so the
+// boundary-key lookup is left out; a point beside a boundary of the counting
+// grid is evaluated in binary64.
 // Positions are in fixed point: the kernel is bound by the issue of
 // instructions (70% of the slots), and with float-float positions a third of
 // its 490 per point were these (119.7M binary64 points 2.42 -> 2.05 ms, 12.3M
@@ -753,7 +741,8 @@ __device__ __forceinline__ void group_clear(GroupSmem<kMode>& gs) {
 template <bool kF32, bool kCells, int kMode>
 __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3)
     k_distribute(const uint8_t* __restrict__ cloud, uint64_t n,
-                                                              uint32_t stride, CloudGrid g, OutParams op,
+                                                              uint32_t stride, CloudGrid g,
+                                                              const __grid_constant__ OutParams op,
                                                               const __grid_constant__ FixedGrid fg,
                                                               const uint32_t* __restrict__ pyr0,
                                                               const uint64_t* __restrict__ data_idx, uint32_t* fill,
@@ -790,6 +779,7 @@ __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3
             int32_t q[3];      // kCells: output coordinates, finest cells, colour
             uint32_t fine[3];
             bool proven = true, known = true;   // cells, output coordinates
+            uint32_t edge = 0;   // of a point beside a boundary between cells (boundary_cells)
             if (k < cnt) {
                 record_words<kWords>(recs + (uint64_t)k * stride, w);
                 int cell[3];
@@ -806,14 +796,21 @@ __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3
                         known &= in && exact_out && q[a] >= 0;
                     }
                     if (!proven) {
+                        const uint4 c = boundary_cells<kF32>(recs + (uint64_t)k * stride, fg);
+                        fine[0] = c.x;
+                        fine[1] = c.y;
+                        fine[2] = c.z;
+                        edge = c.w;
 #pragma unroll
-                        for (int a = 0; a < 3; ++a)
-                            cell[a] = exact_axis_cell(word_coord_exact<kF32>(w, a), g.ax[a].mn, g.ax[a].t, g.grid);
+                        for (int a = 0; a < 3; ++a)   // (a boundary of the counting grid)
+                            cell[a] = edge < 64 ? (int)(fine[a] >> 6)
+                                                : exact_axis_cell(word_coord_exact<kF32>(w, a), g.ax[a].mn, g.ax[a].t, g.grid);
                     }
                     if (!known) {
-#pragma unroll
-                        for (int a = 0; a < 3; ++a)
-                            q[a] = exact_out_coord(word_coord_exact<kF32>(w, a), op.ax[a].mn, op.ax[a].sf);
+                        const OutCoords c = open_out_coords<kF32>(recs + (uint64_t)k * stride, fg, op.ax);
+                        q[0] = c.x;
+                        q[1] = c.y;
+                        q[2] = c.z;
                     }
                     if ((cell[0] | cell[1] | cell[2]) >= 0) m = cell_morton(cell, smem, L);
                     else set_error(err, kErrBelowBox);
@@ -878,9 +875,8 @@ __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3
                         x = q[0];
                         y = q[1];
                         z = q[2];
-                        fw = proven ? kSafeWord | ((fine[0] >> lv) & 127u) | (((fine[1] >> lv) & 127u) << 7) |
-                                          (((fine[2] >> lv) & 127u) << 14)
-                                    : 0u;
+                        fw = word_edge(edge) | ((fine[0] >> lv) & 127u) | (((fine[1] >> lv) & 127u) << 7) |
+                             (((fine[2] >> lv) & 127u) << 14);
                     } else {
                         Coord c[3];
                         for (int a = 0; a < 3; ++a)

@@ -17,11 +17,12 @@
 //
 // Cell words.  A candidate's cell in a node is the cell its position in the
 // cloud's cube gives at that node's resolution, unless rounding of the
-// reference's binary64 formula could decide otherwise: distribution proves the
-// former for almost every point (fixed_units) and stores the point's cell in its
-// leaf's parent; each level's output stores its own cell, and the parent's is
-// that, halved.  Bit 31 of a word says that the proof holds at every level;
-// without it the cell is evaluated from the cloud point in binary64.  When that
+// reference's binary64 formula could decide otherwise: distribution tells the
+// points for which it could, and at which levels (fixed_cell, kWordEdge), and
+// stores the point's cell in its leaf's parent; each level's output stores its
+// own cell, and the parent's is that, halved.  Where the formula decides, the
+// cell is evaluated from the cloud point in binary64, once: the word keeps it
+// for the unit's later passes.  When that
 // lands outside the unit (a point on an octant boundary that the two levels
 // round differently; common where coordinates are multiples of a scale and the
 // box is too) kErrForeign is set, and the levels from this one on are done again
@@ -228,7 +229,7 @@ struct WeightShared {
 
 // Node-grid cell of a candidate without the proof, as coordinates; foreign
 // when it is not the unit's.
-__device__ __noinline__ uint32_t node_cell(const UnitLevelArgs& a, const Unit& un, uint32_t idx, bool& foreign) {
+__device__ __forceinline__ uint32_t node_cell(const UnitLevelArgs& a, const Unit& un, uint32_t idx, bool& foreign) {
     const uint32_t f = exact_cell(a, a.nodes[un.node], idx);
     const uint32_t x = f & 127, y = (f >> kFieldBits) & 127, z = f >> (2 * kFieldBits), b = un.b;
     const uint32_t h = a.s - 1;
@@ -238,12 +239,29 @@ __device__ __noinline__ uint32_t node_cell(const UnitLevelArgs& a, const Unit& u
     return f;
 }
 
-// The same with ~0 for a foreign candidate: k_foreign has handed it to the unit
-// its cell is in, or the pass is repeated with that, from this level.
-__device__ __forceinline__ uint32_t unproven_cell(const UnitLevelArgs& a, const Unit& un, uint32_t idx) {
+// Whether a word's cell may differ from the formula's in the level's grids.
+__device__ __forceinline__ bool unproven(const UnitLevelArgs& a, uint32_t w) {
+    return ((w >> kWordEdge) & 31u) > a.level + 6 - a.s;
+}
+
+// Cell of an unproven candidate, evaluated once per node; the unit that reads
+// the candidate leaves it in the word.
+__device__ __forceinline__ uint32_t resolved_word(const UnitLevelArgs& a, const Unit& un, uint32_t* word, uint32_t w,
+                                                  uint32_t idx) {
+    if ((w & kWordResolved) && ((w >> kWordGrid) & 7u) == a.s) return w;
     bool foreign;
     const uint32_t f = node_cell(a, un, idx, foreign);
-    if (!foreign) return f;
+    w = f | (w & kWordEdges) | (a.s << kWordGrid) | kWordResolved | (foreign ? kWordForeign : 0u);
+    *word = w;
+    return w;
+}
+
+// The cell, ~0 for a foreign candidate: k_foreign has handed it to the unit its
+// cell is in, or the pass is repeated with that, from this level.
+__device__ __noinline__ uint32_t unproven_cell(const UnitLevelArgs& a, const Unit& un, uint32_t* word, uint32_t w,
+                                               uint32_t idx) {
+    w = resolved_word(a, un, word, w, idx);
+    if (!(w & kWordForeign)) return w & kWordCell;
     if (!a.foreign_head) {
         a.err[1] = a.level;
         atomicOr(a.err, kErrForeign);
@@ -251,8 +269,8 @@ __device__ __forceinline__ uint32_t unproven_cell(const UnitLevelArgs& a, const 
     return ~0u;
 }
 
-// Calls get(cell in the unit's box as Box::cell takes it, cloud index, r | g <<
-// 16, b) for the points of other units whose cell lies in this one: the block's
+// Calls get(cell as Box::cell takes it with its kWordEdge bits, cloud index, r |
+// g << 16, b) for the points of other units whose cell lies in this one: the block's
 // threads take the points of one segment after the other.
 template <class Get>
 __device__ __forceinline__ void foreign_points(const UnitLevelArgs& a, const Unit& un, uint32_t head, Get&& get) {
@@ -260,7 +278,7 @@ __device__ __forceinline__ void foreign_points(const UnitLevelArgs& a, const Uni
         const uint4 h = a.foreign[seg - 1];
         for (uint32_t k = threadIdx.x; k < h.y; k += blockDim.x) {
             const uint4 e = a.foreign[seg + k];
-            const uint32_t b = un.b, x = e.x & 127, y = (e.x >> kFieldBits) & 127, z = e.x >> (2 * kFieldBits);
+            const uint32_t b = un.b, x = e.x & 127, y = (e.x >> kFieldBits) & 127, z = (e.x >> (2 * kFieldBits)) & 127;
             if (un.part && ((((x >> b) & 1) << 2) | (((y >> b) & 1) << 1) | ((z >> b) & 1)) != un.part - 8) continue;
             get(e.x, e.y, e.z, e.w);
         }
@@ -417,7 +435,7 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
         const bool staged = un.staged;
         const uint32_t shift = staged ? 1u : kFieldBits - a.s;
         const uint64_t start = un.start;
-        const uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
+        uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
         const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
         // the weight measures the distance from the point itself to each
         // neighbour cell centre (kernel_inter_cell_filtering.cuh:171-176)
@@ -451,8 +469,8 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
                     const uint32_t w = src_word[k];
                     uint32_t f = w >> shift;
                     bool mine = true;
-                    if (!(w >> 31)) {
-                        f = unproven_cell(a, un, idx);
+                    if ((w & kWordEdges) && unproven(a, w)) {
+                        f = unproven_cell(a, un, src_word + k, w, idx);
                         mine = f != ~0u;
                     }
                     if (mine) i = (int)box.cell(f);
@@ -645,7 +663,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
         const bool staged = un.staged;
         const uint32_t shift = staged ? 1u : kFieldBits - a.s;
         const uint64_t start = un.start;
-        const uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
+        uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
         const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
         uint32_t wide = 0;   // colour bits above 8
         auto add = [&](uint32_t rank, uint32_t idx, uint32_t c0, uint32_t c1) {
@@ -705,8 +723,8 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                         const uint32_t w = src_word[k];
                         uint32_t f = w >> shift;
                         bool mine = true;
-                        if (!(w >> 31)) {
-                            f = unproven_cell(a, un, idx[j]);
+                        if ((w & kWordEdges) && unproven(a, w)) {
+                            f = unproven_cell(a, un, src_word + k, w, idx[j]);
                             mine = f != ~0u;
                         }
                         if (mine) i[j] = (int)box.cell(f);
@@ -721,7 +739,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                 const uint32_t rank = box.rank((uint32_t)i[j]);
                 add(rank, idx[j], c0[j], c1[j]);
                 if (it + j >= 32 || (claim >> (it + j)) & 1u) {
-                    const uint32_t wd = (kSafeWord | base) + box.coordinates((uint32_t)i[j]);
+                    const uint32_t wd = base + box.coordinates((uint32_t)i[j]);
                     if (kLocal) l_word[rank] = wd;
                     else a.stage_word[oo + rank] = wd;
                 }
@@ -729,25 +747,32 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
         }
         if (kForeign && sh.foreign)
             foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t c0, uint32_t c1) {
-                add(box.rank(box.cell(f)), idx, c0, c1);
+                const uint32_t i = box.cell(f), rank = box.rank(i);
+                add(rank, idx, c0, c1);
+                if (kLocal) l_word[rank] = base + box.coordinates(i);
+                else a.stage_word[oo + rank] = base + box.coordinates(i);
             });
         if (kLocal && averaged && wide) sh.redo = 1;
         __syncthreads();
-        // a cell that any candidate without the proof falls in loses it
+        // cells whose point lies beside a boundary take over how far up it matters
         if (sh.unsafe) {
+            auto edge = [&](uint32_t rank, uint32_t idx, uint32_t w) {
+                uint32_t best;
+                if (kLocal) best = kRandom ? (uint32_t)l_key[rank] : l_idx[rank];
+                else best = kRandom ? (uint32_t)__ldcg(a.best + so + rank) : __ldcg(a.stage_lut + oo + rank);
+                if (best != idx) return;
+                if (kLocal) l_word[rank] |= w & kWordEdges;
+                else a.stage_word[oo + rank] |= w & kWordEdges;
+            };
             for (uint32_t k = tid; k < cnt; k += T) {
-                if (src_word[k] >> 31) continue;
-                const uint32_t f = unproven_cell(a, un, src_lut[k]);
-                if (f == ~0u) continue;
-                const uint32_t i = box.cell(f);
-                if (kLocal) l_word[box.rank(i)] = base + box.coordinates(i);
-                else a.stage_word[oo + box.rank(i)] = base + box.coordinates(i);
+                const uint32_t w = src_word[k];
+                if (!(w & kWordEdges)) continue;
+                const uint32_t idx = src_lut[k], f = unproven(a, w) ? unproven_cell(a, un, src_word + k, w, idx) : w >> shift;
+                if (f != ~0u) edge(box.rank(box.cell(f)), idx, w);
             }
             if (kForeign && sh.foreign)
-                foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t, uint32_t, uint32_t) {
-                    const uint32_t i = box.cell(f);
-                    if (kLocal) l_word[box.rank(i)] = base + box.coordinates(i);
-                    else a.stage_word[oo + box.rank(i)] = base + box.coordinates(i);
+                foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t, uint32_t) {
+                    edge(box.rank(box.cell(f)), idx, f);
                 });
         }
     }
@@ -883,8 +908,8 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
     {
         const uint32_t cnt = un.cnt;
         const uint32_t shift = un.staged ? 1u : kFieldBits - a.s;
-        const uint32_t* src_word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
-        bool unsafe = false;
+        uint32_t* src_word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
+        bool beside = false;   // a candidate lies beside a boundary between cells
         for (uint32_t k0 = tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
             uint32_t w[4];
 #pragma unroll
@@ -897,10 +922,12 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                 const uint32_t k = k0 + j * T;
                 if (k >= cnt) break;
                 uint32_t f = w[j] >> shift;
-                if (!(w[j] >> 31)) {
-                    unsafe = true;
-                    f = unproven_cell(a, un, ((un.staged ? a.stage_lut : a.leaf_lut) + un.start)[k]);
-                    if (f == ~0u) continue;
+                if (w[j] & kWordEdges) {
+                    beside = true;
+                    if (unproven(a, w[j])) {
+                        f = unproven_cell(a, un, src_word + k, w[j], ((un.staged ? a.stage_lut : a.leaf_lut) + un.start)[k]);
+                        if (f == ~0u) continue;
+                    }
                 }
                 const uint32_t i = box.cell(f);
                 ++included;
@@ -912,14 +939,14 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
             }
         }
         if (kForeign && sh.foreign) {
-            unsafe = true;
             foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t, uint32_t, uint32_t) {
                 const uint32_t i = box.cell(f);
                 ++included;
+                beside = beside || (f & kWordEdges);
                 atomicOr(&bm[i >> 5], 1u << (i & 31));
             });
         }
-        if (unsafe) sh.unsafe = 1;
+        if (beside) sh.unsafe = 1;
         if (kColor == 3) {
             const uint32_t n = __reduce_add_sync(0xffffffffu, included);
             if (lane == 0) atomicAdd(&sh.included, n);
@@ -1008,6 +1035,7 @@ __device__ __noinline__ void unit_run_other(const UnitLevelArgs& a, BlockShared&
     else unit_run<T, kColor, kRandom, 0, true, uint16_t>(a, sh, bm, ui, ws);
 }
 
+#if OC_UNITS_PART == 0
 // The level's points whose cell lies outside their unit, as a segment per unit
 // (or chunk of one) and octant they belong to.  Reads the words of all
 // candidates, for builds that were found to have such points.
@@ -1024,20 +1052,20 @@ __global__ void __launch_bounds__(kForeignThreads) k_foreign(const __grid_consta
     for (uint32_t item = blockIdx.x; item < a.n_units * chunks; item += gridDim.x) {
         const Unit un = load_unit(a, item / chunks);
         const uint32_t per = un.cnt / chunks + 1, first = min(item % chunks * per, un.cnt), end = min(first + per, un.cnt);
-        const uint32_t* word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
+        uint32_t* word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
         const uint32_t* lut = (un.staged ? a.stage_lut : a.leaf_lut) + un.start;
         auto points = [&](auto&& get) {
             for (uint32_t k0 = first + tid; k0 < end; k0 += 4 * T) {
                 uint32_t w[4];
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) w[j] = k0 + j * T < end ? word[k0 + j * T] : kSafeWord;
+                for (uint32_t j = 0; j < 4; ++j) w[j] = k0 + j * T < end ? word[k0 + j * T] : 0u;
 #pragma unroll
                 for (uint32_t j = 0; j < 4; ++j) {
-                    if (w[j] >> 31) continue;
-                    bool foreign;
-                    const uint32_t f = node_cell(a, un, lut[k0 + j * T], foreign), h = a.s - 1;
-                    const uint32_t x = f & 127, y = (f >> kFieldBits) & 127, z = f >> (2 * kFieldBits);
-                    if (foreign) get(k0 + j * T, f, ((x >> h) << 2) | ((y >> h) << 1) | (z >> h));
+                    if (!unproven(a, w[j])) continue;
+                    const uint32_t k = k0 + j * T, f = resolved_word(a, un, word + k, w[j], lut[k]), h = a.s - 1;
+                    if (!(f & kWordForeign)) continue;
+                    const uint32_t x = f & 127, y = (f >> kFieldBits) & 127, z = (f >> (2 * kFieldBits)) & 127;
+                    get(k, f, ((x >> h) << 2) | ((y >> h) << 1) | (z >> h));
                 }
             }
         };
@@ -1074,6 +1102,7 @@ __global__ void __launch_bounds__(kForeignThreads) k_foreign(const __grid_consta
         __syncthreads();
     }
 }
+#endif
 
 // kColor: 0 raw colour, 1 intra-cell, 2 inter-cell, 3 distance-weighted.  An
 // inter-cell or weighted colour whose neighbourhood reaches into other units keeps its sum and goes to its

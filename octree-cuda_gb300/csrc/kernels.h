@@ -175,7 +175,7 @@ int launch_push_tags(uint32_t* pyr, const uint64_t* level_off_dev, uint32_t dept
 // Level of a leaf beside its first record in data_idx (launch_leaf_prep).
 constexpr uint32_t kLeafLevelShift = 56;
 
-// Distribution that writes cell words (kSafeWord) instead of sub-step
+// Distribution that writes cell words (kWordEdge) instead of sub-step
 // words: for the octant kernels (launch_units_level).
 int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
                             const OutParams& out, const FixedGrid& fixed, const uint32_t* pyr0,
@@ -336,7 +336,7 @@ struct UnitLevelArgs {
     uint32_t stride;
     uint32_t float_input;
     const uint32_t* leaf_lut;
-    const uint32_t* leaf_word;
+    uint32_t* leaf_word;    // (units leave evaluated cells in the words, see kWordResolved)
     const uint8_t* leaf_rec;
     uint32_t* stage_lut;    // per staged point: cloud index
     uint32_t* stage_word;   // cell word

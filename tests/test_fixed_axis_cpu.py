@@ -125,3 +125,47 @@ def test_positions(program, mn, side, scale, depth, f32):
     assert tried > 100_000 and bad == 0
     if mn == 0.0 and side == 1.0 and not f32:   # an ordinary box: about all but the points put on boundaries
         assert known > tried * 0.5 and cells > tried * 0.5
+
+
+# The same points through fixed_cell: the cell holds in every grid of cells wider than the boundary it names, also
+# for points at both ends of the box and beyond its upper one, which the formulas clamp.
+CELLS = r"""
+        uint32_t boundary;
+        const uint32_t c = fixed_cell(d, a.cell, (uint32_t)fine_cells, boundary);
+        if (c >= fine_cells) ++bad;
+        if (a.cell.room == 0 && !boundary && p > mn + side / 4 && p < mn + side * 0.75) ++bad;   // nothing is proven
+        const uint32_t low = boundary & (0u - boundary);
+        if (!low) ++proven_cells;
+        for (unsigned level = 1; level <= depth; ++level) {
+            const long path = c >> (6 + level), in = c & ((128l << (level - 1)) - 1);
+            for (long grid = 8; grid <= 128; grid *= 2)
+                if (low < ((128l << (level - 1)) / grid) &&
+                    node_cell(p, mn, side, depth, level, path, grid) != in * grid >> (6 + level)) ++bad;
+        }
+        if (low < 64 && node_cell(p, mn, side, depth, depth, 0, (long)(fine_cells >> 6)) != (long)(c >> 6)) ++bad;
+    };
+"""
+
+
+@pytest.fixture(scope="module")
+def cells_program(tmp_path_factory):
+    if not shutil.which("g++"):
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("fixed_cells")
+    begin = PROGRAM.index("        const uint32_t c = fixed_units(d, a.cell, ok);")
+    end = PROGRAM.index("    auto around")
+    (d / "t.cpp").write_text(PROGRAM[:begin] + CELLS + PROGRAM[end:])
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", os.path.join(ROOT, "octree-cuda_gb300", "csrc"),
+                    str(d / "t.cpp"), "-o", str(d / "t")], check=True)
+    return str(d / "t")
+
+
+@pytest.mark.parametrize("f32", [0, 1])
+@pytest.mark.parametrize("mn,side,depth", [
+    (0.0, 1.0, 1), (0.0, 1.0, 10), (0.0, 4096.0, 9), (-50.5, 101.0, 7), (1e6, 100.0, 9), (-4.7e6, 5000.0, 10),
+    (437000.0, 51.2, 6), (123456.78, 3000.32, 9), (5412345.67, 25.6, 5), (1e12, 10.0, 4), (0.0, 3e9, 10)])
+def test_cells_beside_boundaries(cells_program, mn, side, depth, f32):
+    out = subprocess.run([cells_program, repr(mn), repr(side), "0.01", str(depth), str(f32)], check=True,
+                         capture_output=True, text=True).stdout
+    bad, tried, _, cells = map(int, out.split())
+    assert tried > 100_000 and bad == 0

@@ -249,6 +249,33 @@ def test_lattice_cloud(off, side, chunk, sub, mode):
     check_repeat(case, cfg, ["repeat_octants"])
 
 
+@pytest.mark.parametrize("mode", ["first", "first_intra", "random_inter", "random_weighted"])
+@pytest.mark.parametrize("cloud_type,steps,scale,sub", [(1, 4096, 0.01, 128), (0, 4096, 0.01, 64), (1, 512, 1 / 64, 32),
+                                                        (0, 65536, 1 / 1024, 128)])
+def test_points_on_cell_boundaries(cloud_type, steps, scale, sub, mode):
+    """Coordinates that are exact multiples of a fraction of the box, most of them on boundaries between cells of some
+    level, at both ends of the box too; output coordinates that lie on integers."""
+    rng = np.random.default_rng(9)
+    n = 70_000
+    xyz = rng.integers(0, steps + 1, (n, 3)) * (64.0 / steps)
+    xyz[:, 2] = np.floor(xyz[:, 0] + xyz[:, 1]) / 2
+    rgb = rng.integers(0, 256, (n, 3), dtype=np.uint8)
+    case = case_from_points(xyz, rgb, cloud_type, scale=scale, bbox=[0, 0, 0, 64.0, 64.0, 64.0])
+    check(case, dict(chunk_grid=64, sub_grid=sub, merge_threshold=500, output_factor=12.0, **MODES[mode]))
+
+
+@pytest.mark.parametrize("box", [64.0, 40.0])
+@pytest.mark.parametrize("off", [0.0, 1e12])
+def test_points_beyond_the_box(box, off):
+    """Points above the box (clamped to its last cells), and a box whose coordinates prove no cell."""
+    rng = np.random.default_rng(10)
+    n = 40_000
+    xyz = off + np.floor(rng.random((n, 3)) * 64 * 64) / 64
+    rgb = rng.integers(0, 256, (n, 3), dtype=np.uint8)
+    case = case_from_points(xyz, rgb, 1, scale=0.125, bbox=[off] * 3 + [off + box] * 3)
+    check(case, dict(chunk_grid=32, sub_grid=64, merge_threshold=400, output_factor=12.0, inter=True))
+
+
 @pytest.mark.parametrize("sub", [64, 100])
 def test_output_coordinate_beyond_int32(sub):
     """A scale for which the far points' output coordinates do not fit: an error found before subsampling, after which
