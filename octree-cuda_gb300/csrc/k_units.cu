@@ -227,6 +227,14 @@ struct WeightShared {
     uint2 rows[kWeightThreads / kWeightLanes][9];
 };
 
+// Units of many candidates per cell have shared sums of 32 bits per colour: the
+// packed ones (exact up to 257 candidates) would mostly have to be done again in
+// global memory, where the cells' reductions queue up (grids of 8: 3M
+// binary64 points 1.23 ms, before octants 0.87).  32 bits hold 16.8M candidates of 8-bit colours.
+__device__ __forceinline__ bool dense_unit(uint32_t candidates, uint32_t cells) {
+    return candidates / 24 > cells && candidates < (1u << 23);
+}
+
 // Node-grid cell of a candidate without the proof, as coordinates; foreign
 // when it is not the unit's.
 __device__ __forceinline__ uint32_t node_cell(const UnitLevelArgs& a, const Unit& un, uint32_t idx, bool& foreign) {
@@ -395,7 +403,7 @@ __device__ __forceinline__ uint32_t weighted_mean(uint64_t sum, uint64_t weight)
 // hold.  (A lane per cell, or lanes sharing each neighbour's points, waits
 // for the longest list: the weight of a pair costs about 45 instructions.)
 // Colours are of 8 bits here: the cloud's, or means of those.
-template <int T, bool kRandom, int kB, bool kLocal, bool kForeign, class Pre>
+template <int T, bool kRandom, int kB, bool kLocal, bool kOther, class Pre>
 __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box,
                                               const uint64_t* l_key, const uint32_t* l_word, uint32_t* l_cnt,
                                               uint32_t cells, const int (&keep)[4], uint64_t so, uint64_t oo,
@@ -489,7 +497,7 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
                 a.csr_pts[c0 + atomicAdd(cur + box.rank((uint32_t)i), 1u)] = v;
             }
         }
-        if (kForeign && sh.foreign)
+        if (kOther && sh.foreign)
             foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t rg, uint32_t bl) {
                 float4 v = cell_units(idx);
                 v.w = __uint_as_float((rg & 0xFFu) | ((rg >> 8) & 0xFF00u) | (bl << 16));
@@ -614,16 +622,18 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
 // sums beyond 16 bits) in the staging arrays and the level's scratch, reached
 // by reductions.  keep: the cells of this thread's first four candidates.
 // Returns false (every thread alike) when a local unit has to be redone.
-template <int T, int kColor, bool kRandom, int kB, bool kLocal, bool kForeign, class Pre>
+template <int T, int kColor, bool kRandom, int kB, bool kLocal, bool kOther, class Pre>
 __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box, uint32_t* pool,
                                            uint32_t ui, uint32_t cells, const int (&keep)[4], uint32_t claim,
                                            uint32_t included, bool placed, WeightShared* ws) {
     constexpr bool averaged = kColor == 1 || kColor == 2, weighted = kColor == 3;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Unit& un = sh.un;
-    // shared: [sums 8 B][random keys 8 B | indices 4 B][words 4 B][weighted: candidates 4 B] per cell
+    // shared: [sums 8 B, dense 16 B][random keys 8 B | indices 4 B][words 4 B][weighted: candidates 4 B] per cell
+    const bool dense = kOther && kLocal && averaged && dense_unit(un.cnt, cells);
     uint2* l_sum = reinterpret_cast<uint2*>(pool);
-    uint64_t* l_key = reinterpret_cast<uint64_t*>(l_sum + (averaged ? cells : 0));
+    uint4* l_wide = reinterpret_cast<uint4*>(pool);   // dense: r, g, b, candidates
+    uint64_t* l_key = reinterpret_cast<uint64_t*>(l_sum + (averaged ? dense ? 2 * cells : cells : 0));
     uint32_t* l_idx = reinterpret_cast<uint32_t*>(l_key);
     uint32_t* l_word = kRandom ? reinterpret_cast<uint32_t*>(l_key + cells) : l_idx + cells;
     uint32_t* l_cnt = l_word + cells;
@@ -639,7 +649,8 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
     }
     for (uint32_t r = tid; r < cells; r += T) {
         if (kLocal) {
-            if (averaged) l_sum[r] = make_uint2(0, 0);
+            if (dense) l_wide[r] = make_uint4(0, 0, 0, 0);
+            else if (averaged) l_sum[r] = make_uint2(0, 0);
             if (weighted) l_cnt[r] = 0;
             if (kRandom) l_key[r] = ~0ull;
             else l_idx[r] = 0xFFFFFFFFu;
@@ -680,7 +691,13 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                 atomicMin(a.stage_lut + oo + rank, idx);
             }
             if (averaged) {
-                if (kLocal) {
+                if (dense) {
+                    atomicAdd(&l_wide[rank].x, c0 & 0xFFFFu);
+                    atomicAdd(&l_wide[rank].y, c0 >> 16);
+                    atomicAdd(&l_wide[rank].z, c1);
+                    atomicAdd(&l_wide[rank].w, 1u);
+                    wide |= (c0 & 0xFF00FF00u) | (c1 & 0xFF00u);
+                } else if (kLocal) {
                     // r | g << 16 and b | 1 << 20: exact while the cell has at
                     // most 257 candidates with colours of 8 bits (checked below)
                     atomicAdd(&l_sum[rank].x, c0);
@@ -745,7 +762,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                 }
             }
         }
-        if (kForeign && sh.foreign)
+        if (kOther && sh.foreign)
             foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t c0, uint32_t c1) {
                 const uint32_t i = box.cell(f), rank = box.rank(i);
                 add(rank, idx, c0, c1);
@@ -770,7 +787,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                 const uint32_t idx = src_lut[k], f = unproven(a, w) ? unproven_cell(a, un, src_word + k, w, idx) : w >> shift;
                 if (f != ~0u) edge(box.rank(box.cell(f)), idx, w);
             }
-            if (kForeign && sh.foreign)
+            if (kOther && sh.foreign)
                 foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t, uint32_t) {
                     edge(box.rank(box.cell(f)), idx, f);
                 });
@@ -779,7 +796,18 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
     // ---- the sums as the packed words of the reference; a count field that
     // overflowed shows as a sum of counts short of the unit's candidates
     if (kLocal) {
-        if (averaged) {
+        if (dense) {
+            // (the packed words go where the reads below expect them, over sums
+            // of lower ranks, which are read first)
+            for (uint32_t r0 = 0; r0 < cells; r0 += T) {
+                const uint32_t r = r0 + tid;
+                const uint4 v = r < cells ? l_wide[r] : make_uint4(0, 0, 0, 0);
+                __syncthreads();
+                if (r < cells)
+                    *reinterpret_cast<uint64_t*>(l_sum + r) =
+                        ((uint64_t)v.x << 46) + ((uint64_t)v.y << 28) + ((uint64_t)v.z << 10) + v.w;
+            }
+        } else if (averaged) {
             int32_t d = -(int32_t)included;
             bool bad = false;
             for (uint32_t r = tid; r < cells; r += T) {
@@ -809,7 +837,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
     const uint64_t* g_packed = a.sum + so;
     const uint32_t m0 = box.m0(), open = un.open;
     if constexpr (weighted) {
-        unit_weighted<T, kRandom, kB, kLocal, kForeign, Pre>(a, sh, box, l_key, l_word, l_cnt, cells, keep, so, oo, *ws);
+        unit_weighted<T, kRandom, kB, kLocal, kOther, Pre>(a, sh, box, l_key, l_word, l_cnt, cells, keep, so, oo, *ws);
     } else {
         for (uint32_t r0 = warp * 32; r0 < cells; r0 += T) {
             const uint32_t r = r0 + lane;
@@ -856,19 +884,19 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
 // seldom need it: inlined, its registers weigh on the other variant's (level
 // 4 of the 119.7M-point build 1.34 -> 1.27 ms; two blocks per SM, which
 // need it often, lose by it: level 1 0.84 -> 1.13 ms).
-template <int T, int kColor, bool kRandom, int kB, bool kForeign, class Pre>
+template <int T, int kColor, bool kRandom, int kB, bool kOther, class Pre>
 __device__ __noinline__ void unit_cells_global(const UnitLevelArgs& a, BlockShared& sh, const uint32_t* bm,
                                                const Pre* pre, uint32_t b, uint32_t ui, uint32_t cells, int4 keep4,
                                                uint32_t claim, uint32_t included, bool placed) {
     const int keep[4] = {keep4.x, keep4.y, keep4.z, keep4.w};
     const Box<kB, Pre> box{bm, pre, b};
-    unit_cells<T, kColor, kRandom, kB, false, kForeign, Pre>(a, sh, box, nullptr, ui, cells, keep, claim, included,
+    unit_cells<T, kColor, kRandom, kB, false, kOther, Pre>(a, sh, box, nullptr, ui, cells, keep, claim, included,
                                                              placed, nullptr);
 }
 
-// One unit: pass A, ranks, then its cells.  kForeign: points of other units
-// may have their cells here.
-template <int T, int kColor, bool kRandom, int kB, bool kForeign, class Pre>
+// One unit: pass A, ranks, then its cells.  kOther: points of other units may
+// have their cells here, or a cell hold very many candidates.
+template <int T, int kColor, bool kRandom, int kB, bool kOther, class Pre>
 __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh, uint32_t* bm, uint32_t ui,
                                          WeightShared* ws) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -938,7 +966,7 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                 if (!(old & bit) && it + j < 32) claim |= 1u << (it + j);
             }
         }
-        if (kForeign && sh.foreign) {
+        if (kOther && sh.foreign) {
             foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t, uint32_t, uint32_t) {
                 const uint32_t i = box.cell(f);
                 ++included;
@@ -1009,18 +1037,19 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
     // (unit_cells starts with a barrier after it cleared the cells)
     const uint32_t room = a.smem_words * 4 - (uint32_t)((pool - bm) * 4);
     bool placed = false;
-    if (sizeof(Pre) == 2 && cells * cell_bytes(kColor, kRandom) <= room) {
-        if (unit_cells<T, kColor, kRandom, kB, true, kForeign, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, false, ws))
+    const uint32_t dense_bytes = kOther && (kColor == 1 || kColor == 2) && dense_unit(un.cnt, cells) ? 8u : 0u;
+    if (sizeof(Pre) == 2 && cells * (cell_bytes(kColor, kRandom) + dense_bytes) <= room) {
+        if (unit_cells<T, kColor, kRandom, kB, true, kOther, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, false, ws))
             return;
         placed = true;
         __syncthreads();
     }
     if constexpr (T == 1024)
-        unit_cells_global<T, kColor, kRandom, kB, kForeign, Pre>(a, sh, bm, pre, b, ui, cells,
+        unit_cells_global<T, kColor, kRandom, kB, kOther, Pre>(a, sh, bm, pre, b, ui, cells,
                                                        make_int4(keep[0], keep[1], keep[2], keep[3]), claim, included,
                                                        placed);
     else
-        unit_cells<T, kColor, kRandom, kB, false, kForeign, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, placed,
+        unit_cells<T, kColor, kRandom, kB, false, kOther, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, placed,
                                                                  ws);
 }
 
@@ -1144,7 +1173,7 @@ __global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_consta
         WeightShared* ws = reinterpret_cast<WeightShared*>(dyn + a.smem_words);
         if (sh.foreign) unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
         else if (sh.un.b == 6 && sh.un.cnt <= 65535) unit_run<T, kColor, kRandom, 6, false, uint16_t>(a, sh, dyn, ui, ws);
-        else if (kHalf && sh.un.b == 5) unit_run<T, kColor, kRandom, 5, false, uint16_t>(a, sh, dyn, ui, ws);
+        else if (kHalf && sh.un.b == 5 && sh.un.cnt <= 32768) unit_run<T, kColor, kRandom, 5, false, uint16_t>(a, sh, dyn, ui, ws);
         else unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
     }
 }

@@ -291,3 +291,16 @@ def test_output_coordinate_beyond_int32(sub):
         with pytest.raises(octree_api.OctreeError, match="does not fit int32"):
             run_gpu(case, cfg)
     check(case_from_points(xyz, rgb, 1, scale=0.001, bbox=[0, 0, 0, 1000.0, 1000.0, 1000.0]), cfg)
+
+
+@pytest.mark.parametrize("mode", ["first_intra", "first_inter", "random_intra", "random_inter"])
+@pytest.mark.parametrize("shape,n,chunk,sub,threshold", [("plane", 150_000, 8, 8, 9_000), ("volume", 150_000, 8, 16, 9_000),
+                                                         ("corner", 200_000, 8, 32, 20_000), ("plane", 250_000, 2, 64, 200_000)])
+def test_many_candidates_per_cell(shape, n, chunk, sub, threshold, mode):
+    """Cells of more than 257 candidates (the shared sums' limit), and of more than 1024 (the packed count's)."""
+    xyz, rgb = points(shape, n)
+    if shape == "plane":
+        xyz[:, 0] = 0.3
+    rgb[: n // 3] = 255
+    case = case_from_points(xyz * 50.0, rgb, 0, scale=0.001, bbox=[0, 0, 0, 50.5, 50.5, 50.5])
+    check(case, dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=threshold, output_factor=4.0, **MODES[mode]))
