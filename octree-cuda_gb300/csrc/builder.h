@@ -194,7 +194,7 @@ public:
     void prefetch_sync();
     uint64_t spare_bytes() const { return spare_.bytes; }
     // Resident state: after a successful generate(), the uploaded cloud, the
-    // count pyramid, the node tree and the leaf records stay on the device.
+    // node tree and the leaf records stay on the device.
     // If `cfg` differs from the last build only in its subsampling settings
     // (grid, modes, seed, output factor), reuse() adopts them and the next
     // generate() runs subsampling alone; otherwise it returns false and
@@ -252,6 +252,7 @@ private:
     void record_params();
     void size_for_config();
     bool octant_subsampling() const;
+    void rewrite_leaf_words(bool cells);
     void subsample();
     void compute_tree_stats();
     void compute_stats();

@@ -1007,6 +1007,52 @@ __global__ void __launch_bounds__(1024) k_place_prepare(const uint32_t* __restri
         for (uint32_t k = threadIdx.x; k < n_internal; k += blockDim.x) cnt[k] = 0;
 }
 
+// The words of the leaf records as distribution writes them, for a resident tree
+// that is subsampled by the other kind of kernels: cell words (kCells) or
+// sub-step words.  leaves: first record and level (kLeafLevelShift) of every
+// leaf, in record order.  Gathers cloud points as k_place_units does.
+template <bool kF32, bool kCells>
+__global__ void __launch_bounds__(256) k_leaf_words(const uint8_t* __restrict__ cloud, uint64_t n, uint32_t stride,
+                                                    const __grid_constant__ OutParams op,
+                                                    const __grid_constant__ FixedGrid fg,
+                                                    const uint64_t* __restrict__ leaves, uint32_t n_leaves,
+                                                    const uint32_t* __restrict__ lut, uint32_t* __restrict__ word) {
+    constexpr uint64_t kMask = (1ull << kLeafLevelShift) - 1;
+    for (uint64_t pos = blockIdx.x * 256ull + threadIdx.x; pos < n; pos += gridDim.x * 256ull) {
+        uint32_t lo = 0, hi = n_leaves;   // last leaf that starts at pos or before
+        while (kCells && hi - lo > 1) {
+            const uint32_t mid = (lo + hi) / 2;
+            if ((leaves[mid] & kMask) <= pos) lo = mid;
+            else hi = mid;
+        }
+        const uint8_t* rec = cloud + (uint64_t)lut[pos] * stride;
+        uint32_t w[kF32 ? 4 : 7];
+        gather_words<kF32, false>(rec, w);
+        if (kCells) {
+            const uint32_t lv = (uint32_t)(leaves[lo] >> kLeafLevelShift);
+            uint32_t c[3], edge = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                uint64_t d;
+                uint32_t boundary;
+                const bool in = fixed_difference(word_coord<kF32>(w, a), fg.ax[a].o, d);
+                c[a] = fixed_cell(d, fg.ax[a].cell, fg.cells, boundary);
+                edge = max(edge, in ? boundary & (0u - boundary) : 1u << 31);
+            }
+            word[pos] = word_edge(edge) | ((c[0] >> lv) & 127u) | (((c[1] >> lv) & 127u) << 7) | (((c[2] >> lv) & 127u) << 14);
+        } else {
+            uint32_t f[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const Coord c = kF32 ? coord_f32(__uint_as_float(w[a]))
+                                     : coord_f64(__hiloint2double((int)w[kF32 ? 0 : 2 * a + 1], (int)w[kF32 ? 0 : 2 * a]));
+                out_coord_frac<kF32>(c, op.ax[a], f[a]);
+            }
+            word[pos] = pack_frac(f[0], f[1], f[2]);
+        }
+    }
+}
+
 __global__ void k_place_lut(const uint64_t* __restrict__ src_off, const uint64_t* __restrict__ dst_off,
                             const uint32_t* __restrict__ count, uint32_t n_nodes,
                             const uint32_t* __restrict__ stage_lut, uint32_t* __restrict__ lut) {
@@ -1111,6 +1157,17 @@ int launch_leaf_prep(const uint32_t* n_nodes, const uint16_t* info, const uint32
                      const uint32_t* key, uint32_t* pyr, const uint64_t* loff_dev, uint64_t* data_idx, uint32_t* fill,
                      uint64_t n_points, uint32_t* err, cudaStream_t stream) {
     k_leaf_prep<<<1, 1024, 0, stream>>>(n_nodes, info, count, level, key, pyr, loff_dev, data_idx, fill, n_points, err);
+    return 1;
+}
+
+int launch_leaf_words(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, bool cells,
+                      const OutParams& out, const FixedGrid& fixed, const uint64_t* leaves, uint32_t n_leaves,
+                      const uint32_t* lut, uint32_t* word, int num_sms, cudaStream_t stream) {
+    if (!n) return 0;
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)num_sms * 8));
+    const auto go = float_input ? cells ? k_leaf_words<true, true> : k_leaf_words<true, false>
+                                : cells ? k_leaf_words<false, true> : k_leaf_words<false, false>;
+    go<<<grid, 256, 0, stream>>>(cloud, n, stride, out, fixed, leaves, n_leaves, lut, word);
     return 1;
 }
 

@@ -182,6 +182,12 @@ int launch_distribute_cells(const uint8_t* cloud, uint64_t n, uint32_t stride, b
                             const uint64_t* data_idx, uint32_t* fill, uint32_t* lut, uint8_t* rec, uint32_t* word,
                             uint32_t* err, int num_sms, cudaStream_t stream);
 
+// Rewrites the words of n leaf records as launch_distribute_cells (cells) or
+// launch_distribute write them.
+int launch_leaf_words(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, bool cells,
+                      const OutParams& out, const FixedGrid& fixed, const uint64_t* leaves, uint32_t n_leaves,
+                      const uint32_t* lut, uint32_t* word, int num_sms, cudaStream_t stream);
+
 int launch_distribute(const uint8_t* cloud, uint64_t n, uint32_t stride, bool float_input, const CloudGrid& g,
                       const OutParams& out, const uint32_t* pyr0, const uint64_t* data_idx, uint32_t* fill,
                       uint32_t* lut, uint8_t* rec, uint32_t* frac, uint32_t* err, int num_sms,

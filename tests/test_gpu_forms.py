@@ -434,3 +434,20 @@ def test_session_random_sequence_equals_fresh_builds():
             assert np.array_equal(a_l, b_l) and a_r.tobytes() == b_r.tobytes(), (step, g0, n, m)
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("kind,cloud_type", [(0, 0), (2, 1), (3, 1)])
+def test_server_reuses_across_kinds_of_grid(kind, cloud_type):
+    """One resident cloud subsampled with grids of both kinds of kernels in turn (powers of two from 8 to 128, others):
+    the leaf words follow, and every result equals the build run alone."""
+    case = make_case(kind, cloud_type, 150_000, seed=43)
+    srv = octree_api.Server(lanes=1, memory_budget=64 << 30)
+    for step, (sub, m) in enumerate([(128, 0), (100, 1), (128, 2), (48, 3), (64, 1), (256, 0), (16, 2), (100, 2)]):
+        want = alone(case, (64, sub), m)
+        buf = buffers(want)
+        t = srv.submit(job_for(case, (64, sub), m, *buf, cloud_id=7))
+        r = srv.wait(t)
+        srv.release(t)
+        check_same(want, r, *buf)
+        assert r.reused == (step > 0)
+    srv.close()
