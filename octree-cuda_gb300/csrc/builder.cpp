@@ -504,7 +504,7 @@ std::vector<std::pair<std::string, uint64_t>> Builder::device_allocations() cons
         {"octant tables", units_.bytes + unit_sync_.bytes + oct_off_.bytes},
         {"subsampling scratch", key_cache_.bytes + unit_cache_.bytes + acc_best_.bytes + acc_sel_.bytes +
                                     acc_intra_.bytes + emit_maps_.bytes + emit_state_.bytes +
-                                    csr_start_.bytes + csr_pts_.bytes},
+                                    csr_start_.bytes + csr_pts_.bytes + partials_.bytes},
         {"brick tables", g_key_.bytes + g_mask_.bytes + g_base_.bytes},
         {"level tables", sub_nodes_.bytes + out_points_.bytes + stage_off_.bytes + post_ii_.bytes + node_dst_.bytes +
                              place_src_.bytes + place_dst_.bytes + place_cnt_.bytes},
@@ -1254,8 +1254,8 @@ void Builder::subsample() {
     // internal node its points, staged offset and final position
     const size_t o_pts = 32, o_soff = (o_pts + (size_t)n_internal * 4 + 7) & ~(size_t)7;
     const size_t o_dst = o_soff + (size_t)n_internal * 8;
-    const size_t o_used = o_dst + (size_t)n_internal * 8;   // octants: scratch slots taken per level
-    back_host_.ensure(o_used + 16 * 8);
+    const size_t o_used = o_dst + (size_t)n_internal * 8;   // octants: the head of the counters
+    back_host_.ensure(o_used + kUnitSyncHead);
     place_src_.ensure((size_t)n_internal * 8 + 8);
     place_dst_.ensure((size_t)n_internal * 8 + 8);
     place_cnt_.ensure((size_t)n_internal * 4 + 4);
@@ -1300,6 +1300,7 @@ void Builder::subsample() {
         else if (averaged && !weighted && !octants) acc_intra_.ensure(scratch_cap * 8);
         if (weighted) {
             unit_cache_.ensure(scratch_cap * 16);   // cell units and counts
+            if (octants && sub_partial_cap_ > scratch_cap * 12 / 32) partials_.ensure(sub_partial_cap_ * 32);
             csr_start_.ensure(scratch_cap * 4);
             csr_pts_.ensure(scratch_cap * 20);
             if (!octants) {
@@ -1423,6 +1424,10 @@ void Builder::subsample() {
                 u.face_sum = stage_rec_.as<uint64_t>() + stage_cap;
                 u.partial = unit_cache_.as<uint64_t>();
                 u.partial_cap = scratch_cap * 12 / 32;
+                if (sub_partial_cap_ > u.partial_cap) {
+                    u.partial = partials_.as<uint64_t>();
+                    u.partial_cap = sub_partial_cap_;
+                }
                 u.partials = reinterpret_cast<uint64_t*>(sync + 192) + l;
                 u.csr_count = unit_cache_.as<uint32_t>() + scratch_cap * 3;
                 u.csr_start = csr_start_.as<uint32_t>();
@@ -1527,13 +1532,13 @@ void Builder::subsample() {
                        "D2H");
         }
         if (octants)
-            check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(o_used), unit_sync_.p, 16 * 8, cudaMemcpyDeviceToHost,
+            check_cuda(cudaMemcpyAsync(back_host_.as<uint8_t>(o_used), unit_sync_.p, kUnitSyncHead, cudaMemcpyDeviceToHost,
                                        stream_),
                        "D2H");
         if (attempt == 0) compute_tree_stats();
         check_cuda(cudaStreamSynchronize(stream_), "subsample");
         const uint32_t e = *back_host_.as<uint32_t>(0);
-        if (e & ~(kErrCapacity | kErrForeign)) {
+        if (e & ~(kErrCapacity | kErrForeign | kErrPartials)) {
             // the tables behind the results may not agree: nothing is taken from them
             if (copy_stream_) check_cuda(cudaStreamSynchronize(copy_stream_), "output copies");
             throw_device_errors(e, (e & kErrCapacity) ? "subsample" : "generate");
@@ -1556,6 +1561,17 @@ void Builder::subsample() {
             stage_mark(octants ? "repeat_octants" : "repeat_nodes");
             continue;
         }
+        if ((e & kErrPartials) && !(e & kErrCapacity)) {
+            // a level of more face cells than their sums were given room for
+            // (small grids, or walls along octant boundaries): from it on again
+            const uint64_t cap = std::max<uint64_t>(sub_partial_cap_, scratch_cap * 12 / 32);
+            from_level = std::max(back_host_.as<uint32_t>(0)[1], 1u);
+            const uint64_t wanted = back_host_.as<uint64_t>(o_used)[24 + from_level];
+            sub_partial_cap_ = std::max(wanted + wanted / 4, cap * 2);
+            check_cuda(cudaMemsetAsync(err_.p, 0, 8, stream_), "memset");
+            stage_mark("repeat_partials");
+            continue;
+        }
         if (!(e & kErrCapacity)) {
             stage_used_ = *back_host_.as<uint64_t>(8);
             if (octants) {
@@ -1573,7 +1589,7 @@ void Builder::subsample() {
         stage_cap *= 2;
         scratch_cap = std::min<uint64_t>(scratch_cap * 2, std::max(max_level_bound, scratch_cap));
         rec_cap = std::max<uint64_t>(rec_cap * 2, (uint64_t)cfg_.n + stage_cap);
-        const uint32_t keep = e & ~kErrCapacity;
+        const uint32_t keep = 0;
         check_cuda(cudaMemcpyAsync(err_.p, &keep, 4, cudaMemcpyHostToDevice, stream_), "H2D err");
     }
     sub_stage_cap_ = stage_cap;

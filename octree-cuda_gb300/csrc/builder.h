@@ -280,6 +280,7 @@ private:
     DevBuf stage_lut_, stage_rec_;      // staged internal outputs
     DevBuf sub_nodes_, out_points_, work_;
     DevBuf key_cache_, unit_cache_, acc_best_, acc_sel_, acc_intra_, emit_maps_, emit_state_, csr_start_, csr_pts_;
+    DevBuf partials_;                   // weighted sums of face cells, of builds whose share of unit_cache_ did not do
     DevBuf place_src_, place_dst_, place_cnt_;
     DevBuf g_key_, g_mask_, g_base_;   // per-block global brick tables
     DevBuf cell_keys_, spread_;         // chunking-grid boundary keys and Morton spread table
@@ -314,6 +315,7 @@ private:
     bool counted_ = false;           // upload() binned the cloud: the next generate() skips counting
     std::vector<cudaEvent_t> chunk_ready_;   // chunks of an overlapped upload
     uint64_t sub_stage_cap_ = 0, sub_scratch_cap_ = 0, sub_rec_cap_ = 0;   // capacities that fit the last build
+    uint64_t sub_partial_cap_ = 0;
     uint32_t g_cap_ = 0, g_shift_ = 0;
     uint32_t launches_ = 0;
     size_t place_count_ = 0;

@@ -129,6 +129,7 @@ enum : uint32_t {
     kErrTimeout = 1u << 5,       // a bounded wait (on a bulk copy, on an earlier unit) gave up
     kErrNodeCap = 1u << 6,       // the tree has more nodes than the node table holds
     kErrForeign = 1u << 7,       // a candidate's cell lies outside its child's octant (word 1: the level; the pass is repeated)
+    kErrPartials = 1u << 8,      // no room for the weighted sums of face cells (word 1: the level; it is repeated with more)
 };
 
 // ---------------------------------------------------------------------------

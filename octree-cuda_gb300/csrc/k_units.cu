@@ -607,7 +607,8 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
                 a.partial[slot * 4 + 2] = sb;
                 a.partial[slot * 4 + 3] = sw;
             } else {
-                atomicOr(a.err, kErrForeign);   // more face cells than there is room for: the other kernels
+                a.err[1] = a.level;   // more face cells than there is room for: the level again, with more
+                atomicOr(a.err, kErrPartials);
                 slot = 0;
             }
         }

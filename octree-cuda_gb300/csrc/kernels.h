@@ -394,6 +394,7 @@ inline const char* device_error_message(uint32_t e) {
     if (e & kErrTag) return "a point found no leaf";
     if (e & kErrTimeout) return "a wait on the device (for a bulk copy or for another block) gave up";
     if (e & kErrForeign) return "points outside their octants were left over";
+    if (e & kErrPartials) return "weighted sums of face cells did not fit";
     return e ? "unknown device error" : nullptr;
 }
 

@@ -304,3 +304,20 @@ def test_many_candidates_per_cell(shape, n, chunk, sub, threshold, mode):
     rgb[: n // 3] = 255
     case = case_from_points(xyz * 50.0, rgb, 0, scale=0.001, bbox=[0, 0, 0, 50.5, 50.5, 50.5])
     check(case, dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=threshold, output_factor=4.0, **MODES[mode]))
+
+
+@pytest.mark.parametrize("mode", ["first_weighted", "random_weighted"])
+def test_more_face_cells_than_their_sums_have_room_for(mode):
+    """A small grid, most of whose cells lie on faces between units, with few points per cell: the level is repeated
+    with more room for their weighted sums, by the same kernels, and a later build has the room."""
+    xyz, rgb = points("volume", 40_000)
+    case = case_from_points(xyz * 50.0, rgb, 1, scale=0.001, bbox=[0, 0, 0, 50.5, 50.5, 50.5])
+    cfg = dict(chunk_grid=32, sub_grid=8, merge_threshold=24, output_factor=12.0, **MODES[mode])
+    ref = run_oracle(case, cfg)
+    s = run_gpu(case, cfg)
+    assert [k for k in s.timings() if k.startswith("repeat")] == ["repeat_partials"]
+    compare_results(ref, s)
+    s.generate()
+    assert s.stats()["subsample_passes"] == 1
+    compare_results(ref, s)
+    s.close()
