@@ -321,3 +321,20 @@ def test_more_face_cells_than_their_sums_have_room_for(mode):
     assert s.stats()["subsample_passes"] == 1
     compare_results(ref, s)
     s.close()
+
+
+@pytest.mark.parametrize("cloud_type,stride", [(0, 15), (0, 16), (0, 20), (0, 28), (0, 64), (0, 65), (0, 80), (1, 27), (1, 28),
+                                               (1, 32), (1, 64), (1, 72), (1, 100)])
+@pytest.mark.parametrize("scattered", [False, True])
+def test_strides(cloud_type, stride, scattered):
+    """Record strides on both sides of what the grouped distribution takes, in leaf order and scattered, with enough
+    points (262,144) for the choice by the sampled order."""
+    from helpers import Case
+
+    n = 270_001
+    case = make_case(2, cloud_type, n, seed=17, stride=stride)
+    if scattered:
+        rec = case.cloud.reshape(n, stride)
+        case = Case(np.ascontiguousarray(rec[np.random.default_rng(4).permutation(n)]).reshape(-1), n, stride, cloud_type,
+                    case.scale, case.bb_min, case.bb_max)
+    check(case, dict(chunk_grid=128, sub_grid=64, merge_threshold=1500, random=True, inter=True))
