@@ -1129,17 +1129,28 @@ void Builder::subsample() {
     while ((1u << s_log2) < S) ++s_log2;
     // every_octant: octants without a child get a unit too, for points of other
     // octants whose cell lies there (a repeat with those, see k_foreign).
+    // Leaves that are shared by blocks have the first maps of their level.
+    std::vector<uint32_t> large;             // their numbers among the level's units
+    std::vector<uint32_t> large_first(depth_ + 2, 0), largest(depth_ + 2, 0);
+    const uint32_t large_points = large_leaf_points(cfg_.n);
     auto lay_out_units = [&](bool every_octant) {
         units.clear();
         oct_unit.clear();
+        large.clear();
         map_words = 0;
         // the part of the memory estimate that a brick table would take
         const uint64_t map_room = (uint64_t)num_sms_ * memory_terms(cfg_, num_sms_).slots * 8;
         for (uint32_t l = 1; l <= depth_; ++l) {
             unit_first[l] = (uint32_t)units.size();
             any_split[l] = 0;
-            uint64_t whole = 0;
-            for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) whole += table[k].nchild;
+            large_first[l] = (uint32_t)large.size();
+            largest[l] = 0;
+            uint64_t whole = 0, large_words = 0;
+            for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
+                whole += table[k].nchild;
+                for (uint32_t c = 0; c < table[k].nchild; ++c)   // (0 for inner children)
+                    if (table[k].child_count[c] > large_points) large_words += large_map_words(s_log2);
+            }
             const bool few = S >= 64 && whole < (uint64_t)num_sms_ * 3;
             // inter-cell colours cost less: the extra launch's lookups in global
             // memory pay only where a unit has an SM of its own (level of 79
@@ -1147,7 +1158,7 @@ void Builder::subsample() {
             spread[l] = few && inter && whole && (weighted || whole <= (uint64_t)num_sms_);
             oct_first[l] = oct_unit.size();
             if (spread[l]) oct_unit.resize(oct_unit.size() + 8 * (size_t)(level_first[l + 1] - level_first[l]), ~0u);
-            uint64_t words = 0, candidates = 0;
+            uint64_t words = large_words, candidates = 0;
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
                 const NodeHost& v = nodes_[order[k]];
                 uint32_t c = v.child_first, number = 0, q0 = 0;
@@ -1160,10 +1171,17 @@ void Builder::subsample() {
                         const uint32_t ci = c++;
                         const NodeHost& ch = nodes_[ci];
                         split = few && ch.internal && out_bound[ci] > 4096;
-                        candidates += ch.internal ? std::min<uint64_t>(out_bound[ci], 16384) : ch.points;
                         e.flags = (uint32_t)ch.internal << 7;
                         e.src = ch.internal ? ii_of[ci] : (uint32_t)ch.data_idx;
                         e.count = ch.internal ? 0 : ch.points;
+                        if (e.count > large_points) {
+                            e.flags |= 1u << 20;
+                            e.map = (uint32_t)((large.size() - large_first[l]) * large_map_words(s_log2));
+                            large.push_back((uint32_t)units.size() - unit_first[l]);
+                            largest[l] = std::max(largest[l], e.count);
+                        } else {
+                            candidates += ch.internal ? std::min<uint64_t>(out_bound[ci], 16384) : ch.points;
+                        }
                     } else if (!every_octant) {
                         continue;
                     }
@@ -1177,7 +1195,7 @@ void Builder::subsample() {
                     for (uint32_t part = split ? 8 : 0; part < (split ? 16u : 1u); ++part) {
                         UnitEntry u = e;
                         u.flags |= s | (part << 3) | ((uint32_t)(number == 0) << 8) | (number << 10) | (q0 << 16);
-                        if (spread[l]) {
+                        if (spread[l] && !(u.flags >> 20)) {
                             u.map = (uint32_t)words;
                             words += 2 * ((uint64_t)1 << (3 * (s_log2 - (split ? 2 : 1)) - 5)) + 4;
                         }
@@ -1191,9 +1209,10 @@ void Builder::subsample() {
             const uint64_t count = units.size() - unit_first[l];
             mean_candidates[l] = count ? (uint32_t)(candidates / count) : 0;
             if (words * 4 > map_room) spread[l] = 0;
-            if (spread[l]) map_words = std::max(map_words, words);
+            map_words = std::max(map_words, spread[l] ? words : large_words);
         }
         unit_first[depth_ + 1] = (uint32_t)units.size();
+        large_first[depth_ + 1] = (uint32_t)large.size();
     };
     if (octants) lay_out_units(false);
 
@@ -1230,10 +1249,11 @@ void Builder::subsample() {
     const size_t table_bytes = (size_t)n_internal * sizeof(SubNode);
     const size_t o_post = (table_bytes + 15) & ~(size_t)15;
     const size_t o_units = (o_post + (size_t)n_internal * 4 + 15) & ~(size_t)15;
-    size_t o_oct_unit = 0, units_bytes = 0;   // units, then octant tables
+    size_t o_oct_unit = 0, o_large = 0, units_bytes = 0;   // units, then octant tables and large leaves
     auto stage_tables = [&]() {
         o_oct_unit = units.size() * sizeof(UnitEntry);
-        units_bytes = o_oct_unit + oct_unit.size() * 4;
+        o_large = o_oct_unit + oct_unit.size() * 4;
+        units_bytes = o_large + large.size() * 4;
         table_host_.ensure(o_units + units_bytes + 16);
         if (!n_internal) return;
         std::memcpy(table_host_.p, table.data(), table_bytes);
@@ -1242,6 +1262,8 @@ void Builder::subsample() {
         std::memcpy(table_host_.as<uint8_t>(o_units), units.data(), o_oct_unit);
         if (!oct_unit.empty())
             std::memcpy(table_host_.as<uint8_t>(o_units + o_oct_unit), oct_unit.data(), oct_unit.size() * 4);
+        if (!large.empty())
+            std::memcpy(table_host_.as<uint8_t>(o_units + o_large), large.data(), large.size() * 4);
     };
     stage_tables();
     post_ii_.ensure(std::max<size_t>((size_t)n_internal * 4, 4));
@@ -1378,7 +1400,8 @@ void Builder::subsample() {
                                        stream_),
                        "memset");
             uint64_t largest_unit = S3;
-            for (const UnitEntry& e : units) largest_unit = std::max<uint64_t>(largest_unit, e.count);
+            for (const UnitEntry& e : units)
+                if (!(e.flags >> 20)) largest_unit = std::max<uint64_t>(largest_unit, e.count);
             uint8_t* sync = unit_sync_.as<uint8_t>();
             UnitNodeState* node_state = reinterpret_cast<UnitNodeState*>(sync + kUnitSyncHead);
             uint64_t* unit_state = reinterpret_cast<uint64_t*>(node_state + n_internal);
@@ -1415,6 +1438,11 @@ void Builder::subsample() {
                 u.spread = spread[l];
                 u.oct_unit = reinterpret_cast<const uint32_t*>(units_.as<uint8_t>() + o_oct_unit) + oct_first[l];
                 u.maps = g_mask_.as<uint32_t>();
+                u.large = reinterpret_cast<const uint32_t*>(units_.as<uint8_t>() + o_large) + large_first[l];
+                u.n_large = large_first[l + 1] - large_first[l];
+                u.largest = largest[l];
+                if (u.n_large)
+                    check_cuda(cudaMemsetAsync(g_mask_.p, 0, u.n_large * large_map_words(s_log2) * 4, stream_), "memset");
                 u.level_used = reinterpret_cast<uint64_t*>(sync);
                 u.stage_cap = stage_cap;
                 u.scratch_cap = scratch_cap;

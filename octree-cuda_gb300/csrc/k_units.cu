@@ -113,6 +113,7 @@ __device__ __forceinline__ uint64_t pack_colour(uint16_t r, uint16_t g, uint16_t
 struct Unit {
     uint32_t node, octant, part, index;
     uint32_t staged, first, last, q0;
+    uint32_t large, map;   // a large leaf (k_large_mark); word offset of its bitmap and ranks
     uint32_t cnt;
     uint32_t b;
     uint32_t base;    // fields(x0, y0, z0)
@@ -131,6 +132,8 @@ __device__ __forceinline__ Unit load_unit(const UnitLevelArgs& a, uint32_t u) {
     v.last = (e.flags >> 9) & 1;
     v.index = (e.flags >> 10) & 63;
     v.q0 = (e.flags >> 16) & 15;
+    v.large = (e.flags >> 20) & 1;
+    v.map = e.map;
     v.start = e.src;
     v.cnt = e.count;
     if (v.staged) {
@@ -176,6 +179,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint64_t bytes) {
 template <int kColor>
 __device__ __forceinline__ void prefetch_unit(const UnitLevelArgs& a, uint32_t u) {
     const Unit v = load_unit(a, u);
+    if (v.large) return;
     prefetch_l2((v.staged ? a.stage_word : a.leaf_word) + v.start, (uint64_t)v.cnt * 4);
     prefetch_l2((v.staged ? a.stage_lut : a.leaf_lut) + v.start, (uint64_t)v.cnt * 4);
     if (kColor) {
@@ -205,6 +209,12 @@ __device__ __forceinline__ void append_faces(const UnitLevelArgs& a, uint32_t no
         a.face_sum[f] = sum;
     }
 }
+
+// Words of a unit's bitmap, and in the map of a large leaf (bitmap, one word
+// more, ranks) the place of what its blocks share: candidates, whether one lies
+// beside a boundary, and the unit's first candidate in the node.
+__host__ __device__ constexpr uint32_t bitmap_words(uint32_t b) { return 3 * b > 5 ? 1u << (3 * b - 5) : 1u; }
+__host__ __device__ constexpr uint32_t large_state(uint32_t b) { return 2 * bitmap_words(b) + 4; }
 
 struct BlockShared {
     Unit un;
@@ -395,7 +405,29 @@ __device__ __forceinline__ uint32_t weighted_mean(uint64_t sum, uint64_t weight)
     return q;
 }
 
-// The emit of a distance-weighted unit: its candidates grouped by cell, then
+// Position of a cloud point in the node's grid, in cell units: the weight
+// measures the distance from the point itself to each neighbour cell centre
+// (kernel_inter_cell_filtering.cuh:171-176).
+__device__ __forceinline__ float4 cell_units(const UnitLevelArgs& a, const SubNode& nd, uint32_t idx) {
+    Coord co[3];
+    uint32_t col[3];
+    float4 v;
+    const uint8_t* p = a.cloud + (uint64_t)idx * a.stride;
+    if (a.float_input) {
+        gather_point<true, false>(p, co, col);
+        v.x = point_units<true>(co[0], nd.ax[0]);
+        v.y = point_units<true>(co[1], nd.ax[1]);
+        v.z = point_units<true>(co[2], nd.ax[2]);
+    } else {
+        gather_point<false, false>(p, co, col);
+        v.x = point_units<false>(co[0], nd.ax[0]);
+        v.y = point_units<false>(co[1], nd.ax[1]);
+        v.z = point_units<false>(co[2], nd.ax[2]);
+    }
+    return v;
+}
+
+// The emit of a distance-weighted unit, whose candidates are grouped by cell:
 // four lanes per cell.  The points of a row of up to three cells follow each
 // other, so a cell's points are at most nine ranges: the lanes look them up,
 // the ranges become one list by a prefix sum, and the lanes walk it four
@@ -403,120 +435,16 @@ __device__ __forceinline__ uint32_t weighted_mean(uint64_t sum, uint64_t weight)
 // hold.  (A lane per cell, or lanes sharing each neighbour's points, waits
 // for the longest list: the weight of a pair costs about 45 instructions.)
 // Colours are of 8 bits here: the cloud's, or means of those.
-template <int T, bool kRandom, int kB, bool kLocal, bool kOther, class Pre>
-__device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box,
-                                              const uint64_t* l_key, const uint32_t* l_word, uint32_t* l_cnt,
-                                              uint32_t cells, const int (&keep)[4], uint64_t so, uint64_t oo,
+// cur: past each cell's last candidate of the unit; sh.next counts from the
+// first cell to do up to `cells`.
+template <bool kLocal, int kB, class Pre>
+__device__ __forceinline__ void weighted_emit(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box,
+                                              const uint32_t* l_word, const uint32_t* cur, uint32_t cells, uint64_t oo,
                                               WeightShared& ws) {
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
     const Unit& un = sh.un;
-    const uint32_t* l_idx = reinterpret_cast<const uint32_t*>(l_key);
-    // ---- exclusive scan of the cells' counts, in place: the cursor of each
-    // cell (first its first candidate, in the end one past its last)
-    uint32_t* cur = kLocal ? l_cnt : a.csr_count + so;
-    {
-        const uint32_t per = (cells + T - 1) / T, r0 = min(tid * per, cells), r1 = min(r0 + per, cells);
-        uint32_t sum = 0;
-        for (uint32_t r = r0; r < r1; ++r) sum += kLocal ? cur[r] : __ldcg(cur + r);
-        uint32_t incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (uint32_t)o) incl += y;
-        }
-        if (lane == 31) sh.warp[warp] = incl;
-        __syncthreads();
-        uint32_t run = incl - sum;
-        for (uint32_t q = 0; q < warp; ++q) run += sh.warp[q];
-        for (uint32_t r = r0; r < r1; ++r) {
-            const uint32_t n = kLocal ? cur[r] : __ldcg(cur + r);
-            if (kLocal) cur[r] = run;
-            else __stcg(cur + r, run);
-            run += n;
-        }
-        __syncthreads();
-    }
     const uint64_t c0 = sh.off + sh.cand0;   // the unit's first candidate in the level's scratch
-    {
-        const SubNode& nd = a.nodes[un.node];
-        const uint32_t cnt = un.cnt;
-        const bool staged = un.staged;
-        const uint32_t shift = staged ? 1u : kFieldBits - a.s;
-        const uint64_t start = un.start;
-        uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
-        const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
-        // the weight measures the distance from the point itself to each
-        // neighbour cell centre (kernel_inter_cell_filtering.cuh:171-176)
-        auto cell_units = [&](uint32_t idx) {
-            Coord co[3];
-            uint32_t col[3];
-            float4 v;
-            const uint8_t* p = a.cloud + (uint64_t)idx * a.stride;
-            if (a.float_input) {
-                gather_point<true, false>(p, co, col);
-                v.x = point_units<true>(co[0], nd.ax[0]);
-                v.y = point_units<true>(co[1], nd.ax[1]);
-                v.z = point_units<true>(co[2], nd.ax[2]);
-            } else {
-                gather_point<false, false>(p, co, col);
-                v.x = point_units<false>(co[0], nd.ax[0]);
-                v.y = point_units<false>(co[1], nd.ax[1]);
-                v.z = point_units<false>(co[2], nd.ax[2]);
-            }
-            return v;
-        };
-        for (uint32_t k0 = tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t k = k0 + j * T;
-                if (k >= cnt) break;
-                const uint32_t idx = src_lut[k];
-                int i = keep[j];
-                if (it) {
-                    i = -1;
-                    const uint32_t w = src_word[k];
-                    uint32_t f = w >> shift;
-                    bool mine = true;
-                    if ((w & kWordEdges) && unproven(a, w)) {
-                        f = unproven_cell(a, un, src_word + k, w, idx);
-                        mine = f != ~0u;
-                    }
-                    if (mine) i = (int)box.cell(f);
-                }
-                if (i < 0) continue;
-                float4 v = cell_units(idx);
-                uint32_t c;
-                if (staged) {
-                    const uint2 q = *reinterpret_cast<const uint2*>(a.stage_col + start + k);
-                    c = (q.x & 0xFFu) | ((q.x >> 8) & 0xFF00u) | (q.y << 16);
-                } else {
-                    const uint16_t* q = reinterpret_cast<const uint16_t*>(a.leaf_rec + (start + k) * 18 + 12);
-                    c = (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16);
-                }
-                v.w = __uint_as_float(c);
-                a.csr_pts[c0 + atomicAdd(cur + box.rank((uint32_t)i), 1u)] = v;
-            }
-        }
-        if (kOther && sh.foreign)
-            foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t rg, uint32_t bl) {
-                float4 v = cell_units(idx);
-                v.w = __uint_as_float((rg & 0xFFu) | ((rg >> 8) & 0xFF00u) | (bl << 16));
-                a.csr_pts[c0 + atomicAdd(cur + box.rank(box.cell(f)), 1u)] = v;
-            });
-    }
-    __syncthreads();
     auto cell_end = [&](uint32_t r) { return kLocal ? cur[r] : __ldcg(cur + r); };
-    for (uint32_t r = tid; r < cells; r += T) {
-        a.csr_start[so + r] = sh.cand0 + (r ? cell_end(r - 1) : 0u);   // read by other units' face cells
-        if (kLocal) {
-            a.stage_word[oo + r] = l_word[r];
-            a.stage_lut[oo + r] = kRandom ? (uint32_t)l_key[r] : l_idx[r];
-        } else if (kRandom) {
-            a.stage_lut[oo + r] = (uint32_t)__ldcg(a.best + so + r);
-        }
-    }
-    if (a.spread) return;
-    // ---- emit
     constexpr uint32_t kG = kWeightLanes;
     const uint32_t m0 = box.m0(), b = box.b(), g = lane / kG, s = lane % kG;
     uint2* rows = ws.rows[tid / kG];
@@ -618,6 +546,102 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
     }
 }
 
+// A distance-weighted unit after pass B: its candidates grouped by cell, and the emit.
+template <int T, bool kRandom, int kB, bool kLocal, bool kOther, class Pre>
+__device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShared& sh, const Box<kB, Pre>& box,
+                                              const uint64_t* l_key, const uint32_t* l_word, uint32_t* l_cnt,
+                                              uint32_t cells, const int (&keep)[4], uint64_t so, uint64_t oo,
+                                              WeightShared& ws) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Unit& un = sh.un;
+    const uint32_t* l_idx = reinterpret_cast<const uint32_t*>(l_key);
+    // ---- exclusive scan of the cells' counts, in place: the cursor of each
+    // cell (first its first candidate, in the end one past its last)
+    uint32_t* cur = kLocal ? l_cnt : a.csr_count + so;
+    {
+        const uint32_t per = (cells + T - 1) / T, r0 = min(tid * per, cells), r1 = min(r0 + per, cells);
+        uint32_t sum = 0;
+        for (uint32_t r = r0; r < r1; ++r) sum += kLocal ? cur[r] : __ldcg(cur + r);
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        if (lane == 31) sh.warp[warp] = incl;
+        __syncthreads();
+        uint32_t run = incl - sum;
+        for (uint32_t q = 0; q < warp; ++q) run += sh.warp[q];
+        for (uint32_t r = r0; r < r1; ++r) {
+            const uint32_t n = kLocal ? cur[r] : __ldcg(cur + r);
+            if (kLocal) cur[r] = run;
+            else __stcg(cur + r, run);
+            run += n;
+        }
+        __syncthreads();
+    }
+    const uint64_t c0 = sh.off + sh.cand0;   // the unit's first candidate in the level's scratch
+    {
+        const SubNode& nd = a.nodes[un.node];
+        const uint32_t cnt = un.cnt;
+        const bool staged = un.staged;
+        const uint32_t shift = staged ? 1u : kFieldBits - a.s;
+        const uint64_t start = un.start;
+        uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
+        const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
+        for (uint32_t k0 = tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t k = k0 + j * T;
+                if (k >= cnt) break;
+                const uint32_t idx = src_lut[k];
+                int i = keep[j];
+                if (it) {
+                    i = -1;
+                    const uint32_t w = src_word[k];
+                    uint32_t f = w >> shift;
+                    bool mine = true;
+                    if ((w & kWordEdges) && unproven(a, w)) {
+                        f = unproven_cell(a, un, src_word + k, w, idx);
+                        mine = f != ~0u;
+                    }
+                    if (mine) i = (int)box.cell(f);
+                }
+                if (i < 0) continue;
+                float4 v = cell_units(a, nd, idx);
+                uint32_t c;
+                if (staged) {
+                    const uint2 q = *reinterpret_cast<const uint2*>(a.stage_col + start + k);
+                    c = (q.x & 0xFFu) | ((q.x >> 8) & 0xFF00u) | (q.y << 16);
+                } else {
+                    const uint16_t* q = reinterpret_cast<const uint16_t*>(a.leaf_rec + (start + k) * 18 + 12);
+                    c = (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16);
+                }
+                v.w = __uint_as_float(c);
+                a.csr_pts[c0 + atomicAdd(cur + box.rank((uint32_t)i), 1u)] = v;
+            }
+        }
+        if (kOther && sh.foreign)
+            foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t idx, uint32_t rg, uint32_t bl) {
+                float4 v = cell_units(a, nd, idx);
+                v.w = __uint_as_float((rg & 0xFFu) | ((rg >> 8) & 0xFF00u) | (bl << 16));
+                a.csr_pts[c0 + atomicAdd(cur + box.rank(box.cell(f)), 1u)] = v;
+            });
+    }
+    __syncthreads();
+    auto cell_end = [&](uint32_t r) { return kLocal ? cur[r] : __ldcg(cur + r); };
+    for (uint32_t r = tid; r < cells; r += T) {
+        a.csr_start[so + r] = sh.cand0 + (r ? cell_end(r - 1) : 0u);   // read by other units' face cells
+        if (kLocal) {
+            a.stage_word[oo + r] = l_word[r];
+            a.stage_lut[oo + r] = kRandom ? (uint32_t)l_key[r] : l_idx[r];
+        } else if (kRandom) {
+            a.stage_lut[oo + r] = (uint32_t)__ldcg(a.best + so + r);
+        }
+    }
+    if (!a.spread) weighted_emit<kLocal, kB, Pre>(a, sh, box, l_word, cur, cells, oo, ws);
+}
+
 // Pass B and the emit of one unit.  kLocal: the cells' keys, sums and words
 // are in shared memory (`pool`); otherwise (more cells than fit, or colour
 // sums beyond 16 bits) in the staging arrays and the level's scratch, reached
@@ -662,6 +686,10 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
             if (kColor == 2) a.sum[so + r] = 0;
             if (weighted) a.csr_count[so + r] = 0;
         }
+    }
+    if (kOther && !kLocal && un.large) {   // the rest is k_large_cells' and k_large_emit's
+        if (tid == 0) a.maps[un.map + large_state(un.b) + 2] = sh.cand0;
+        return true;
     }
     if (tid == 0) {
         sh.next = 0;
@@ -903,7 +931,7 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Unit& un = sh.un;
     const uint32_t b = kB ? (uint32_t)kB : un.b;
-    const uint32_t W = 3 * b > 5 ? 1u << (3 * b - 5) : 1u;   // bitmap words
+    const uint32_t W = bitmap_words(b);
     // one word past the bitmap is read; both areas in steps of 16 bytes
     Pre* pre = reinterpret_cast<Pre*>(bm + ((W + 4) & ~3u));
     uint32_t* pool = bm + ((W + 4) & ~3u) + ((W * (uint32_t)sizeof(Pre) / 4 + 4) & ~3u);
@@ -939,7 +967,12 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
         const uint32_t shift = un.staged ? 1u : kFieldBits - a.s;
         uint32_t* src_word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
         bool beside = false;   // a candidate lies beside a boundary between cells
-        for (uint32_t k0 = tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
+        if (kOther && un.large) {
+            const uint32_t* map = a.maps + un.map;
+            for (uint32_t i = tid; i < W; i += T) bm[i] = map[i];
+            if (tid == 0) included = map[large_state(b)];
+        }
+        for (uint32_t k0 = kOther && un.large ? cnt : tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
             uint32_t w[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -967,7 +1000,7 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                 if (!(old & bit) && it + j < 32) claim |= 1u << (it + j);
             }
         }
-        if (kOther && sh.foreign) {
+        if (kOther && sh.foreign && !un.large) {
             foreign_points(a, un, sh.foreign, [&](uint32_t f, uint32_t, uint32_t, uint32_t) {
                 const uint32_t i = box.cell(f);
                 ++included;
@@ -1026,9 +1059,9 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                     ((run + c[q]) & 0xFFFFu) | ((run + c[q + (kP > 1)]) << 16);
         }
     }
-    if (kColor >= 2 && a.spread) {
+    if ((kColor >= 2 && a.spread) || (kOther && un.large)) {
         __syncthreads();
-        uint32_t* map = a.maps + a.units[ui].map;
+        uint32_t* map = a.maps + un.map;
         for (uint32_t i = tid; i < W; i += T) {
             map[i] = bm[i];
             map[W + 4 + i] = pre[i];
@@ -1039,7 +1072,7 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
     const uint32_t room = a.smem_words * 4 - (uint32_t)((pool - bm) * 4);
     bool placed = false;
     const uint32_t dense_bytes = kOther && (kColor == 1 || kColor == 2) && dense_unit(un.cnt, cells) ? 8u : 0u;
-    if (sizeof(Pre) == 2 && cells * (cell_bytes(kColor, kRandom) + dense_bytes) <= room) {
+    if (sizeof(Pre) == 2 && cells * (cell_bytes(kColor, kRandom) + dense_bytes) <= room && !(kOther && un.large)) {
         if (unit_cells<T, kColor, kRandom, kB, true, kOther, Pre>(a, sh, box, pool, ui, cells, keep, claim, included, false, ws))
             return;
         placed = true;
@@ -1054,8 +1087,8 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                                                                  ws);
 }
 
-// Units of other kinds than the level's frequent ones (among them those with
-// points from other units), out of line, so that
+// Units of other kinds than the level's frequent ones (among them large leaves
+// and those with points from other units), out of line, so that
 // their registers do not weigh on those (see launch_units).
 template <int T, int kColor, bool kRandom>
 __device__ __noinline__ void unit_run_other(const UnitLevelArgs& a, BlockShared& sh, uint32_t* bm, uint32_t ui,
@@ -1172,10 +1205,281 @@ __global__ void __launch_bounds__(T, unit_blocks(T)) k_units(const __grid_consta
         if (kColor != 3 && tid == T - 33 && a.n_units - ui > gridDim.x) prefetch_unit<kColor>(a, ui + gridDim.x);
         // (the weighted lists follow the pool)
         WeightShared* ws = reinterpret_cast<WeightShared*>(dyn + a.smem_words);
-        if (sh.foreign) unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
+        if (sh.foreign || sh.un.large) unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
         else if (sh.un.b == 6 && sh.un.cnt <= 65535) unit_run<T, kColor, kRandom, 6, false, uint16_t>(a, sh, dyn, ui, ws);
         else if (kHalf && sh.un.b == 5 && sh.un.cnt <= 32768) unit_run<T, kColor, kRandom, 5, false, uint16_t>(a, sh, dyn, ui, ws);
         else unit_run_other<T, kColor, kRandom>(a, sh, dyn, ui, ws);
+    }
+}
+
+// Leaves of many points (dense spots of a scan, coarse counting grids) would keep
+// one block busy for milliseconds: `slices` blocks share each of them.  Before
+// the level's units k_large_mark marks their cells in the bitmaps of their maps;
+// their units (k_units) give the cells ranks and places and clear them; then
+// k_large_cells adds the candidates to the cells by reductions in L2, and
+// k_large_emit makes colours.  In distance weighting k_large_scan and
+// k_large_scatter group the candidates by cell in between.
+// Builds of 20M points, 16M of them in 16^3 cells of one leaf: first point 54.9
+// -> 7.6 ms, inter-cell 93.7 -> 8.4, weighted 175 -> 32; 10M points of terrain
+// on a counting grid of 8 (927,000 in a leaf): inter-cell 7.7 -> 1.0.
+constexpr int kLargeThreads = 512;
+
+// A block's share of a large leaf: the unit, its box over the map in global
+// memory, and its part of n items.
+struct LargePart {
+    Unit un;
+    uint32_t ui, slice, stop;
+    __device__ __forceinline__ uint32_t first(uint32_t n, uint32_t slices) const {
+        return (uint32_t)((uint64_t)n * slice / slices);
+    }
+    __device__ __forceinline__ uint32_t end(uint32_t n, uint32_t slices) const {
+        return (uint32_t)((uint64_t)n * (slice + 1) / slices);
+    }
+};
+
+__device__ __forceinline__ void load_large(const UnitLevelArgs& a, uint32_t slices, LargePart& s) {
+    if (threadIdx.x == 0) {
+        s.stop = *(volatile uint32_t*)a.err;
+        s.ui = a.large[blockIdx.x / slices];
+        s.slice = blockIdx.x % slices;
+        if (!s.stop) s.un = load_unit(a, s.ui);
+    }
+    __syncthreads();
+}
+
+// The unit's first cell in the level's scratch.
+__device__ __forceinline__ uint64_t large_cells_at(const UnitLevelArgs& a, const LargePart& s) {
+    return a.node_state[s.un.node].off1 - 1 + a.unit_rank[s.ui];
+}
+
+__device__ __forceinline__ uint64_t level_base_of(const UnitLevelArgs& a) {
+    uint64_t b = 0;
+    for (uint32_t l = 1; l < a.level; ++l) b += a.level_used[l];
+    return b;
+}
+
+// Calls get(cell in the box, word, position) for the part's own candidates.
+template <class Get>
+__device__ __forceinline__ void large_candidates(const UnitLevelArgs& a, const LargePart& s, uint32_t slices,
+                                                 const Box<0, uint32_t>& box, Get&& get) {
+    uint32_t* src_word = a.leaf_word + s.un.start;
+    const uint32_t* src_lut = a.leaf_lut + s.un.start;
+    const uint32_t first = s.first(s.un.cnt, slices), end = s.end(s.un.cnt, slices);
+    for (uint32_t k0 = first + threadIdx.x; k0 < end; k0 += 4 * kLargeThreads) {
+        uint32_t w[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) w[j] = k0 + j * kLargeThreads < end ? src_word[k0 + j * kLargeThreads] : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t k = k0 + j * kLargeThreads;
+            if (k >= end) break;
+            uint32_t f = w[j] >> (kFieldBits - a.s);
+            if ((w[j] & kWordEdges) && unproven(a, w[j])) {
+                f = unproven_cell(a, s.un, src_word + k, w[j], src_lut[k]);
+                if (f == ~0u) continue;
+            }
+            get(box.cell(f), w[j], k);
+        }
+    }
+}
+
+// Points of other units whose cells lie in the leaf's (the first slice takes them).
+__device__ __forceinline__ uint32_t large_foreign(const UnitLevelArgs& a, const LargePart& s) {
+    return a.foreign_head && s.slice == 0 ? a.foreign_head[s.un.node * 8 + s.un.octant] : 0u;
+}
+
+__global__ void __launch_bounds__(kLargeThreads) k_large_mark(const __grid_constant__ UnitLevelArgs a, uint32_t slices) {
+    __shared__ LargePart s;
+    __shared__ __align__(16) uint32_t bm[bitmap_words(6)];
+    load_large(a, slices, s);
+    if (s.stop) return;
+    const uint32_t W = bitmap_words(s.un.b);
+    const Box<0, uint32_t> box{bm, nullptr, s.un.b};
+    for (uint32_t i = threadIdx.x; i < W; i += kLargeThreads) bm[i] = 0;
+    __syncthreads();
+    uint32_t included = 0;
+    bool beside = false;
+    auto mark = [&](uint32_t i, uint32_t w) {
+        ++included;
+        beside = beside || (w & kWordEdges);
+        const uint32_t bit = 1u << (i & 31);
+        if (!(*(volatile uint32_t*)&bm[i >> 5] & bit)) atomicOr(&bm[i >> 5], bit);
+    };
+    large_candidates(a, s, slices, box, [&](uint32_t i, uint32_t w, uint32_t) { mark(i, w); });
+    foreign_points(a, s.un, large_foreign(a, s), [&](uint32_t f, uint32_t, uint32_t, uint32_t) { mark(box.cell(f), f); });
+    uint32_t* map = a.maps + s.un.map;
+    const uint32_t n = __reduce_add_sync(0xffffffffu, included);
+    if ((threadIdx.x & 31) == 0) atomicAdd(map + large_state(s.un.b), n);
+    if (beside) map[large_state(s.un.b) + 1] = 1;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < W; i += kLargeThreads)
+        if (bm[i]) atomicOr(map + i, bm[i]);
+}
+
+template <int kColor, bool kRandom>
+__global__ void __launch_bounds__(kLargeThreads) k_large_cells(const __grid_constant__ UnitLevelArgs a, uint32_t slices) {
+    __shared__ LargePart s;
+    load_large(a, slices, s);
+    if (s.stop) return;
+    const Unit& un = s.un;
+    const uint32_t* map = a.maps + un.map;
+    const Box<0, uint32_t> box{map, map + bitmap_words(un.b) + 4, un.b};
+    const uint64_t so = large_cells_at(a, s), oo = level_base_of(a) + so;
+    const SubNode& nd = a.nodes[un.node];
+    auto add = [&](uint32_t i, uint32_t idx, uint32_t c0, uint32_t c1) {
+        const uint32_t rank = box.rank(i);
+        if (kRandom)
+            atomicMin(reinterpret_cast<unsigned long long*>(a.best + so + rank),
+                      ((unsigned long long)rp_priority(a.seed, nd.level, nd.morton, idx) << 32) | idx);
+        else
+            atomicMin(a.stage_lut + oo + rank, idx);
+        if (kColor == 1 || kColor == 2)
+            atomicAdd(reinterpret_cast<unsigned long long*>(kColor == 1 ? a.stage_col + oo + rank : a.sum + so + rank),
+                      (unsigned long long)encode_colors(c0 & 0xFFFFu, c0 >> 16, c1));
+        if (kColor == 3) atomicAdd(a.csr_count + so + rank, 1u);
+        a.stage_word[oo + rank] = un.base + box.coordinates(i);   // (the same by every candidate of the cell)
+    };
+    large_candidates(a, s, slices, box, [&](uint32_t i, uint32_t, uint32_t k) {
+        uint32_t c0 = 0, c1 = 0;
+        if (kColor == 1 || kColor == 2) {
+            const uint16_t* q = reinterpret_cast<const uint16_t*>(a.leaf_rec + (un.start + k) * 18 + 12);
+            c0 = q[0] | ((uint32_t)q[1] << 16);
+            c1 = q[2];
+        }
+        add(i, a.leaf_lut[un.start + k], c0, c1);
+    });
+    foreign_points(a, un, large_foreign(a, s), [&](uint32_t f, uint32_t idx, uint32_t c0, uint32_t c1) {
+        add(box.cell(f), idx, c0, c1);
+    });
+}
+
+// Exclusive scan of the cells' candidates, in place: a block per leaf.
+__global__ void __launch_bounds__(1024) k_large_scan(const __grid_constant__ UnitLevelArgs a) {
+    __shared__ LargePart s;
+    __shared__ uint32_t s_warp[32];
+    load_large(a, 1, s);
+    if (s.stop) return;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cells = (uint32_t)a.unit_state[s.ui] - 1u;
+    uint32_t* count = a.csr_count + large_cells_at(a, s);
+    uint32_t running = 0;
+    for (uint32_t r0 = 0; r0 < cells; r0 += 1024) {
+        const uint32_t r = r0 + tid, n = r < cells ? count[r] : 0u;
+        uint32_t incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t before = running, total = 0;
+        for (uint32_t q = 0; q < 32; ++q) {
+            before += q < warp ? s_warp[q] : 0u;
+            total += s_warp[q];
+        }
+        if (r < cells) count[r] = before + incl - n;
+        running += total;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kLargeThreads) k_large_scatter(const __grid_constant__ UnitLevelArgs a, uint32_t slices) {
+    __shared__ LargePart s;
+    load_large(a, slices, s);
+    if (s.stop) return;
+    const Unit& un = s.un;
+    const uint32_t* map = a.maps + un.map;
+    const Box<0, uint32_t> box{map, map + bitmap_words(un.b) + 4, un.b};
+    uint32_t* cur = a.csr_count + large_cells_at(a, s);
+    const uint64_t c0 = a.node_state[un.node].off1 - 1 + map[large_state(un.b) + 2];
+    const SubNode& nd = a.nodes[un.node];
+    large_candidates(a, s, slices, box, [&](uint32_t i, uint32_t, uint32_t k) {
+        const uint16_t* q = reinterpret_cast<const uint16_t*>(a.leaf_rec + (un.start + k) * 18 + 12);
+        float4 v = cell_units(a, nd, a.leaf_lut[un.start + k]);
+        v.w = __uint_as_float((uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16));
+        a.csr_pts[c0 + atomicAdd(cur + box.rank(i), 1u)] = v;
+    });
+    foreign_points(a, un, large_foreign(a, s), [&](uint32_t f, uint32_t idx, uint32_t rg, uint32_t bl) {
+        float4 v = cell_units(a, nd, idx);
+        v.w = __uint_as_float((rg & 0xFFu) | ((rg >> 8) & 0xFF00u) | (bl << 16));
+        a.csr_pts[c0 + atomicAdd(cur + box.rank(box.cell(f)), 1u)] = v;
+    });
+}
+
+// The cells' selected points, how far up they matter (kWordEdge), and colours.
+template <int kColor, bool kRandom>
+__global__ void __launch_bounds__(kLargeThreads) k_large_emit(const __grid_constant__ UnitLevelArgs a, uint32_t slices) {
+    __shared__ LargePart s;
+    load_large(a, slices, s);
+    if (s.stop) return;
+    const Unit& un = s.un;
+    const uint32_t* map = a.maps + un.map;
+    const Box<0, uint32_t> box{map, map + bitmap_words(un.b) + 4, un.b};
+    const uint64_t so = large_cells_at(a, s), oo = level_base_of(a) + so;
+    const uint32_t cells = (uint32_t)a.unit_state[s.ui] - 1u, first = s.first(cells, slices), end = s.end(cells, slices);
+    if (map[large_state(un.b) + 1]) {
+        // (the point that a cell keeps has one lane, and the words' other bits stay)
+        auto edge = [&](uint32_t rank, uint32_t idx, uint32_t w) {
+            const uint32_t best = kRandom ? (uint32_t)a.best[so + rank] : a.stage_lut[oo + rank];
+            if (best == idx) atomicOr(a.stage_word + oo + rank, w & kWordEdges);
+        };
+        large_candidates(a, s, slices, box, [&](uint32_t i, uint32_t w, uint32_t k) {
+            if (w & kWordEdges) edge(box.rank(i), a.leaf_lut[un.start + k], w);
+        });
+        foreign_points(a, un, large_foreign(a, s), [&](uint32_t f, uint32_t idx, uint32_t, uint32_t) {
+            edge(box.rank(box.cell(f)), idx, f);
+        });
+    }
+    const uint32_t rank0 = a.unit_rank[s.ui];
+    if constexpr (kColor == 3) {
+        const uint32_t cand0 = map[large_state(un.b) + 2];
+        const uint32_t* cur = a.csr_count + so;
+        for (uint32_t r = first + threadIdx.x; r < end; r += kLargeThreads) {
+            a.csr_start[so + r] = cand0 + (r ? cur[r - 1] : 0u);
+            if (kRandom) a.stage_lut[oo + r] = (uint32_t)a.best[so + r];
+        }
+        if (a.spread) return;
+        __shared__ BlockShared sh;
+        __shared__ WeightShared ws;
+        if (threadIdx.x == 0) {
+            sh.un = un;
+            sh.off = a.node_state[un.node].off1 - 1;
+            sh.cand0 = cand0;
+            sh.rank0 = rank0;
+            sh.next = first;
+        }
+        __syncthreads();
+        weighted_emit<false, 0, uint32_t>(a, sh, box, nullptr, cur, end, oo, ws);
+    } else {
+        const uint32_t lane = threadIdx.x & 31, m0 = box.m0();
+        for (uint32_t r0 = first + (threadIdx.x & ~31u); r0 < end; r0 += kLargeThreads) {
+            const uint32_t r = r0 + lane;
+            bool face = false;
+            uint32_t w = 0;
+            uint64_t own = 0;
+            if (r < end) {
+                if (kRandom) a.stage_lut[oo + r] = (uint32_t)a.best[so + r];
+                uint64_t e = 0;
+                if (kColor == 1) e = a.stage_col[oo + r];
+                if (kColor == 2 && !a.spread) {
+                    w = a.stage_word[oo + r];
+                    const uint32_t x = w & m0, y = (w >> kFieldBits) & m0, z = (w >> (2 * kFieldBits)) & m0;
+                    face = (faces_of(x, y, z, m0) & un.open) != 0;
+                    own = a.sum[so + r];
+                    e = box.sum27(x, y, z, [&](uint32_t q) { return a.sum[so + q]; });
+                }
+                if (kColor == 1 || (kColor == 2 && !a.spread)) {
+                    if (!face) {
+                        uint16_t cr, cg, cb;
+                        decode_colors(e, cr, cg, cb);
+                        e = pack_colour(cr, cg, cb);
+                    }
+                    a.stage_col[oo + r] = e;
+                }
+            }
+            if (kColor == 2 && !a.spread)
+                append_faces(a, un.node, a.node_state[un.node].off1 - 1, rank0 + r, w, own, face);
+        }
     }
 }
 
@@ -1660,13 +1964,34 @@ void launch_units(const UnitLevelArgs& a, uint32_t mean_candidates, bool half, i
     }
 }
 
+template <int kColor, bool kRandom>
+int launch_large(const UnitLevelArgs& a, uint32_t slices, cudaStream_t stream) {
+    const unsigned grid = a.n_large * slices;
+    k_large_cells<kColor, kRandom><<<grid, kLargeThreads, 0, stream>>>(a, slices);
+    if (kColor == 3) {
+        k_large_scan<<<a.n_large, 1024, 0, stream>>>(a);
+        k_large_scatter<<<grid, kLargeThreads, 0, stream>>>(a, slices);
+    }
+    k_large_emit<kColor, kRandom><<<grid, kLargeThreads, 0, stream>>>(a, slices);
+    return kColor == 3 ? 5 : 3;
+}
+
 // Half-size units are frequent where children are split and on grids up to 64.
+// Large leaves are shared by blocks of about 4096 candidates, up to eight per SM.
 template <int kColor>
-void launch_units_as(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
-                     cudaStream_t stream) {
+int launch_units_as(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
+                    cudaStream_t stream) {
     const bool half = any_split || a.s <= 6;
+    uint32_t slices = 1;
+    if (a.n_large) {
+        const uint64_t sms = (uint64_t)std::max(num_sms, 1);
+        slices = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(a.largest / 4096, (8 * sms + a.n_large - 1) / a.n_large));
+        k_large_mark<<<a.n_large * slices, kLargeThreads, 0, stream>>>(a, slices);
+    }
     if (random) launch_units<kColor, true>(a, mean_candidates, half, num_sms, stream);
     else launch_units<kColor, false>(a, mean_candidates, half, num_sms, stream);
+    if (!a.n_large) return 1;
+    return 1 + (random ? launch_large<kColor, true>(a, slices, stream) : launch_large<kColor, false>(a, slices, stream));
 }
 
 template <int kColor>
@@ -1714,28 +2039,26 @@ int launch_units_weighted(const UnitLevelArgs& a, bool random, uint32_t mean_can
 #if OC_UNITS_PART == 1
 int launch_units_inter(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
                        cudaStream_t stream) {
-    launch_units_as<2>(a, random, mean_candidates, any_split, num_sms, stream);
+    const int launches = launch_units_as<2>(a, random, mean_candidates, any_split, num_sms, stream);
     launch_colours<2>(a, any_split, num_sms, stream);
-    return 2;
+    return launches + 1;
 }
 #elif OC_UNITS_PART == 2
 int launch_units_weighted(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
                           cudaStream_t stream) {
-    launch_units_as<3>(a, random, mean_candidates, any_split, num_sms, stream);
+    const int launches = launch_units_as<3>(a, random, mean_candidates, any_split, num_sms, stream);
     launch_colours<3>(a, any_split, num_sms, stream);
-    return 2;
+    return launches + 1;
 }
 #else
 int launch_units_raw(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
                      cudaStream_t stream) {
-    launch_units_as<0>(a, random, mean_candidates, any_split, num_sms, stream);
-    return 1;
+    return launch_units_as<0>(a, random, mean_candidates, any_split, num_sms, stream);
 }
 
 int launch_units_intra(const UnitLevelArgs& a, bool random, uint32_t mean_candidates, bool any_split, int num_sms,
                        cudaStream_t stream) {
-    launch_units_as<1>(a, random, mean_candidates, any_split, num_sms, stream);
-    return 1;
+    return launch_units_as<1>(a, random, mean_candidates, any_split, num_sms, stream);
 }
 
 int launch_units_level(const UnitLevelArgs& a, uint32_t mode, uint32_t mean_candidates, bool any_split, int num_sms,

@@ -307,11 +307,11 @@ struct UnitEntry {
     uint32_t node;    // in the level's node table
     // bits 0-2 octant, 3-6 part (0 whole, 8 + o part o), 7 staged (the child is
     // an inner node), 8 / 9 first / last unit of the node, 10-15 its number in
-    // the node, 16-19 first octant whose offset the unit writes
+    // the node, 16-19 first octant whose offset the unit writes, 20 a large leaf
     uint32_t flags;
     uint32_t src;     // leaf: first record; inner node: its internal index
     uint32_t count;   // leaf: points
-    uint32_t map;     // spread levels: word offset of the unit's bitmap and ranks in `maps`
+    uint32_t map;     // spread levels and large leaves: word offset of the unit's bitmap and ranks in `maps`
     uint32_t pad;
 };
 
@@ -355,7 +355,9 @@ struct UnitLevelArgs {
     uint64_t* unit_state;   // of this level: cells + 1 (0: not counted yet), candidates << 32
     uint32_t* unit_rank;    // of this level: rank of the unit's first cell in its node
     const uint32_t* oct_unit;   // spread levels, per node and octant: its first unit | split in parts << 31, or ~0
-    uint32_t* maps;         // spread levels: per unit its bitmap, one word more, and the ranks of its words (32 bits)
+    const uint32_t* large;  // numbers of the units that are large leaves (shared by blocks, k_large_mark)
+    uint32_t n_large, largest;   // ... how many, and candidates of the largest
+    uint32_t* maps;         // spread levels, large leaves: per unit its bitmap, one word more, and the ranks of its words (32 bits)
     uint64_t* level_used;   // per level: scratch slots taken
     uint64_t stage_cap, scratch_cap;
     // per scratch slot
@@ -400,6 +402,18 @@ inline const char* device_error_message(uint32_t e) {
 
 // Debug flag (ocpi_set_debug_flags): the waits between units give up at once.
 constexpr uint32_t kDebugNoWait = 2;
+
+// A leaf that is shared by blocks: one block takes 0.2 to 0.4 ms for 65536
+// points, and at most 1024 of them are in a cloud.
+inline uint32_t large_leaf_points(uint64_t n) {
+    return (uint32_t)std::max<uint64_t>(65536, n >> 10);
+}
+
+// Words of a large leaf's map (k_units.cu: bitmap, one word more, ranks, and
+// what its blocks share) on a grid 2^s.
+inline uint64_t large_map_words(uint32_t s) {
+    return 2 * (1ull << (3 * s - 8)) + 8;
+}
 
 // How long a unit waits for the node's earlier units: 2^31 cycles (a second),
 // and 1024 for each candidate of the largest unit, which covers a unit whose

@@ -338,3 +338,51 @@ def test_strides(cloud_type, stride, scattered):
         case = Case(np.ascontiguousarray(rec[np.random.default_rng(4).permutation(n)]).reshape(-1), n, stride, cloud_type,
                     case.scale, case.bb_min, case.bb_max)
     check(case, dict(chunk_grid=128, sub_grid=64, merge_threshold=1500, random=True, inter=True))
+
+
+@pytest.mark.parametrize("mode", sorted(MODES))
+@pytest.mark.parametrize("cloud_type,chunk,sub,around", [(0, 2, 128, 0), (1, 4, 64, 0), (0, 8, 32, 20_000), (1, 16, 128, 60_000),
+                                                         (1, 16, 8, 30_000)])
+def test_large_leaves(cloud_type, chunk, sub, around, mode):
+    """Leaves of more points than one block takes: a few alone (colours spread over blocks where the grid allows it), and
+    one among the units of a level of many, with points beyond both count limits of a cell."""
+    rng = np.random.default_rng(21)
+    n = 160_000
+    xyz = rng.random((n, 3)) ** 2 * 0.06 + 0.52 if around else rng.random((n, 3)) * 0.9 * rng.random((n, 1))
+    xyz[: n // 8] = xyz[0]                     # one cell of very many
+    xyz = np.concatenate([xyz, rng.random((around, 3))])
+    xyz = xyz[rng.permutation(len(xyz))]
+    rgb = rng.integers(0, 256, (len(xyz), 3), dtype=np.uint8)
+    case = case_from_points(xyz * 50.0, rgb, cloud_type, scale=0.001, bbox=[0, 0, 0, 50.5, 50.5, 50.5])
+    cfg = dict(chunk_grid=chunk, sub_grid=sub, merge_threshold=100, output_factor=12.0, **MODES[mode])
+    ref = run_oracle(case, cfg)
+    assert ref.stats["max_leaf_points"] > 65536
+    s = run_gpu(case, cfg)
+    compare_results(ref, s)
+    assert not [k for k in s.timings() if k.startswith("repeat")]
+    s.close()
+
+
+@pytest.mark.parametrize("mode", ["first", "first_intra", "random_inter", "first_weighted"])
+@pytest.mark.parametrize("sub", [16, 64])
+def test_large_leaves_with_points_of_other_octants(sub, mode):
+    """Eight large leaves of one node whose points are multiples of 1 cm, some of them on the planes between the leaves
+    where the node's grid puts them on another side than the counting grid."""
+    rng = np.random.default_rng(22)
+    side, steps = 51.2, 5120
+    for _ in range(1000):
+        off = float(np.round(rng.uniform(1e5, 9e5), 2))
+        p = off + (steps * 3 // 8) * 0.01
+        cubic = (off + side) - off
+        m = off + cubic / 4
+        if (np.floor((p - off) / (cubic / 8)) >= 3) != (np.floor((p - m) / (((m + cubic / 4) - m) / sub)) >= sub // 2):
+            break
+    else:
+        raise AssertionError("no such offset")
+    n = 620_000
+    q = rng.integers(-60, 60, (n, 3)) + steps * 3 // 8
+    rgb = rng.integers(0, 256, (n, 3), dtype=np.uint8)
+    case = case_from_points(off + q * 0.01, rgb, 1, scale=0.01, bbox=[off] * 3 + [off + side] * 3)
+    cfg = dict(chunk_grid=8, sub_grid=sub, merge_threshold=1000, output_factor=4.0, **MODES[mode])
+    assert run_oracle(case, cfg).stats["max_leaf_points"] > 65536
+    check_repeat(case, cfg, ["repeat_octants"])
