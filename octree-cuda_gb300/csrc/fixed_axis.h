@@ -101,18 +101,23 @@ OC_FIXED_FN uint32_t fixed_units(uint64_t d, const FixedScale& s, bool& proven) 
     return (uint32_t)(u >> 32);
 }
 
-// Finest cell of a position, of `cells` on the axis, and the boundary between
-// cells that it lies so near to that the binary64 formulas could put it on
-// either side (0: none, 2^31: nothing is proven on this axis).  The cell of a coarser grid, 2^j finest cells wide, is
-// the upper bits unless the boundary is a multiple of 2^j.  Below the first
-// boundary and above the last the formulas clamp to the outermost cells of
-// every grid.
-OC_FIXED_FN uint32_t fixed_cell(uint64_t d, const FixedScale& s, uint32_t cells, uint32_t& boundary) {
+// Finest cell of a position, of `cells` on the axis.  low becomes the lowest set
+// bit of a boundary between cells, if greater, that the position lies so near to
+// that the binary64 formulas could put it on either side (2^31 where nothing is
+// proven on the axis).  The cell of a coarser grid, 2^j finest cells wide, is the
+// upper bits unless the boundary is a multiple of 2^j.  Below the first boundary
+// and above the last the formulas clamp to the outermost cells of every grid.
+OC_FIXED_FN uint32_t fixed_cell(uint64_t d, const FixedScale& s, uint32_t cells, uint32_t& low) {
     const uint32_t dl = (uint32_t)d, dh = (uint32_t)(d >> 32);
     const uint64_t u = (uint64_t)dh * s.hi + (uint32_t)((uint64_t)dh * s.lo >> 32) + (uint32_t)((uint64_t)dl * s.hi >> 32);
-    const uint32_t f = (uint32_t)u, c = (uint32_t)(u >> 32), b = c + (f >> 31);
-    boundary = f - s.e < s.room ? 0u : s.room == 0 ? 1u << 31 : b < cells ? b : 0u;
-    return c < cells ? c : cells - 1;
+    const uint32_t f = (uint32_t)u;
+    uint32_t c = (uint32_t)(u >> 32);
+    if (f - s.e >= s.room || c >= cells) {
+        const uint32_t b = s.room == 0 ? 1u << 31 : c + (f >> 31) < cells ? c + (f >> 31) : 0u;
+        if ((b & (0u - b)) > low) low = b & (0u - b);
+        if (c >= cells) c = cells - 1;
+    }
+    return c;
 }
 
 // One axis of the cloud's cube: output coordinates and the finest subsampling

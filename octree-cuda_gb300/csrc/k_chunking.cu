@@ -778,8 +778,8 @@ __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3
             uint32_t m = kNoKey;
             int32_t q[3];      // kCells: output coordinates, finest cells, colour
             uint32_t fine[3];
-            bool proven = true, known = true;   // cells, output coordinates
-            uint32_t edge = 0;   // of a point beside a boundary between cells (boundary_cells)
+            bool proven = true, known[3];   // cells; output coordinates
+            uint32_t edge = 0;              // boundary_cells
             if (k < cnt) {
                 record_words<kWords>(recs + (uint64_t)k * stride, w);
                 int cell[3];
@@ -787,13 +787,18 @@ __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
                         uint64_t d;
-                        bool exact_cell, exact_out;
+                        bool exact_cell;
                         const bool in = fixed_difference(word_coord<kF32>(w, a), fg.ax[a].o, d);
                         fine[a] = fixed_units(d, fg.ax[a].cell, exact_cell);
-                        q[a] = (int32_t)fixed_units(d, fg.ax[a].out, exact_out);
+                        q[a] = (int32_t)fixed_units(d, fg.ax[a].out, known[a]);
                         cell[a] = (int)(fine[a] >> 6);
                         proven &= in && exact_cell && fine[a] < fg.cells;
-                        known &= in && exact_out && q[a] >= 0;
+                        known[a] = known[a] && in && q[a] >= 0;
+                    }
+                    if (!(known[0] && known[1] && known[2])) {
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+                            if (!known[a]) q[a] = formula_out_coord<kF32>(w, a, op.ax[a]);
                     }
                     if (!proven) {
                         const uint4 c = boundary_cells<kF32>(recs + (uint64_t)k * stride, fg);
@@ -802,15 +807,9 @@ __global__ void __launch_bounds__(dist_threads(kMode), kMode == kGrouped ? 2 : 3
                         fine[2] = c.z;
                         edge = c.w;
 #pragma unroll
-                        for (int a = 0; a < 3; ++a)   // (a boundary of the counting grid)
+                        for (int a = 0; a < 3; ++a)   // (64: a boundary of the counting grid)
                             cell[a] = edge < 64 ? (int)(fine[a] >> 6)
                                                 : exact_axis_cell(word_coord_exact<kF32>(w, a), g.ax[a].mn, g.ax[a].t, g.grid);
-                    }
-                    if (!known) {
-                        const OutCoords c = open_out_coords<kF32>(recs + (uint64_t)k * stride, fg, op.ax);
-                        q[0] = c.x;
-                        q[1] = c.y;
-                        q[2] = c.z;
                     }
                     if ((cell[0] | cell[1] | cell[2]) >= 0) m = cell_morton(cell, smem, L);
                     else set_error(err, kErrBelowBox);
@@ -1031,14 +1030,14 @@ __global__ void __launch_bounds__(256) k_leaf_words(const uint8_t* __restrict__ 
         if (kCells) {
             const uint32_t lv = (uint32_t)(leaves[lo] >> kLeafLevelShift);
             uint32_t c[3], edge = 0;
+            bool in = true;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 uint64_t d;
-                uint32_t boundary;
-                const bool in = fixed_difference(word_coord<kF32>(w, a), fg.ax[a].o, d);
-                c[a] = fixed_cell(d, fg.ax[a].cell, fg.cells, boundary);
-                edge = max(edge, in ? boundary & (0u - boundary) : 1u << 31);
+                in &= fixed_difference(word_coord<kF32>(w, a), fg.ax[a].o, d);
+                c[a] = fixed_cell(d, fg.ax[a].cell, fg.cells, edge);
             }
+            if (!in) edge = 1u << 31;
             word[pos] = word_edge(edge) | ((c[0] >> lv) & 127u) | (((c[1] >> lv) & 127u) << 7) | (((c[2] >> lv) & 127u) << 14);
         } else {
             uint32_t f[3];

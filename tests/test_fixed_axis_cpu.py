@@ -130,11 +130,10 @@ def test_positions(program, mn, side, scale, depth, f32):
 # The same points through fixed_cell: the cell holds in every grid of cells wider than the boundary it names, also
 # for points at both ends of the box and beyond its upper one, which the formulas clamp.
 CELLS = r"""
-        uint32_t boundary;
-        const uint32_t c = fixed_cell(d, a.cell, (uint32_t)fine_cells, boundary);
+        uint32_t low = 0;
+        const uint32_t c = fixed_cell(d, a.cell, (uint32_t)fine_cells, low);
         if (c >= fine_cells) ++bad;
-        if (a.cell.room == 0 && !boundary && p > mn + side / 4 && p < mn + side * 0.75) ++bad;   // nothing is proven
-        const uint32_t low = boundary & (0u - boundary);
+        if (a.cell.room == 0 && !low && p > mn + side / 4 && p < mn + side * 0.75) ++bad;   // nothing is proven
         if (!low) ++proven_cells;
         for (unsigned level = 1; level <= depth; ++level) {
             const long path = c >> (6 + level), in = c & ((128l << (level - 1)) - 1);
