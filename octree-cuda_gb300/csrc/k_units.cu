@@ -257,9 +257,10 @@ __device__ __forceinline__ uint32_t node_cell(const UnitLevelArgs& a, const Unit
     return f;
 }
 
-// Whether a word's cell may differ from the formula's in the level's grids.
+// Whether a word's cell may differ from the formula's in the level's grids, or
+// was evaluated for another grid (a leaf's, of a resident tree).
 __device__ __forceinline__ bool unproven(const UnitLevelArgs& a, uint32_t w) {
-    return ((w >> kWordEdge) & 31u) > a.level + 6 - a.s;
+    return ((w >> kWordEdge) & 31u) > a.level + 6 - a.s || ((w & kWordResolved) && ((w >> kWordGrid) & 7u) != a.s);
 }
 
 // Cell of an unproven candidate, evaluated once per node; the unit that reads

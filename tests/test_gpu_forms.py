@@ -4,7 +4,7 @@ hierarchy.bin byte-identical, each node's records equal as a multiset."""
 import numpy as np
 import pytest
 
-from helpers import make_case, node_sorted, octree_api, run_gpu
+from helpers import case_from_points, make_case, node_sorted, octree_api, run_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -443,6 +443,27 @@ def test_server_reuses_across_kinds_of_grid(kind, cloud_type):
     case = make_case(kind, cloud_type, 150_000, seed=43)
     srv = octree_api.Server(lanes=1, memory_budget=64 << 30)
     for step, (sub, m) in enumerate([(128, 0), (100, 1), (128, 2), (48, 3), (64, 1), (256, 0), (16, 2), (100, 2)]):
+        want = alone(case, (64, sub), m)
+        buf = buffers(want)
+        t = srv.submit(job_for(case, (64, sub), m, *buf, cloud_id=7))
+        r = srv.wait(t)
+        srv.release(t)
+        check_same(want, r, *buf)
+        assert r.reused == (step > 0)
+    srv.close()
+
+
+@pytest.mark.parametrize("cloud_type,steps", [(0, 4096), (1, 512)])
+def test_server_reuses_points_on_cell_boundaries(cloud_type, steps):
+    """A resident cloud whose points lie on boundaries between cells, subsampled with finer and coarser grids in turn: a
+    cell that was evaluated for one grid is not taken for another's."""
+    rng = np.random.default_rng(9)
+    n = 70_000
+    xyz = rng.integers(0, steps + 1, (n, 3)) * (64.0 / steps)
+    rgb = rng.integers(0, 256, (n, 3), dtype=np.uint8)
+    case = case_from_points(xyz, rgb, cloud_type, scale=0.01, bbox=[0, 0, 0, 64.0, 64.0, 64.0])
+    srv = octree_api.Server(lanes=1, memory_budget=64 << 30)
+    for step, (sub, m) in enumerate([(64, 0), (32, 0), (16, 1), (8, 3), (128, 0), (64, 2), (8, 0), (32, 3)]):
         want = alone(case, (64, sub), m)
         buf = buffers(want)
         t = srv.submit(job_for(case, (64, sub), m, *buf, cloud_id=7))
