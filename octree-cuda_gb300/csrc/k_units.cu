@@ -275,11 +275,11 @@ __device__ __forceinline__ uint32_t resolved_word(const UnitLevelArgs& a, const 
     return w;
 }
 
-// The cell, ~0 for a foreign candidate: k_foreign has handed it to the unit its
+// The cell of candidate k, ~0 for a foreign one: k_foreign has handed it to the unit its
 // cell is in, or the pass is repeated with that, from this level.
-__device__ __noinline__ uint32_t unproven_cell(const UnitLevelArgs& a, const Unit& un, uint32_t* word, uint32_t w,
-                                               uint32_t idx) {
-    w = resolved_word(a, un, word, w, idx);
+__device__ __noinline__ uint32_t unproven_cell(const UnitLevelArgs& a, const Unit& un, uint32_t k, uint32_t w) {
+    const uint64_t at = un.start + k;
+    w = resolved_word(a, un, (un.staged ? a.stage_word : a.leaf_word) + at, w, (un.staged ? a.stage_lut : a.leaf_lut)[at]);
     if (!(w & kWordForeign)) return w & kWordCell;
     if (!a.foreign_head) {
         a.err[1] = a.level;
@@ -588,7 +588,7 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
         const bool staged = un.staged;
         const uint32_t shift = staged ? 1u : kFieldBits - a.s;
         const uint64_t start = un.start;
-        uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
+        const uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
         const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
         for (uint32_t k0 = tid, it = 0; k0 < cnt; k0 += 4 * T, it += 4) {
 #pragma unroll
@@ -603,7 +603,7 @@ __device__ __forceinline__ void unit_weighted(const UnitLevelArgs& a, BlockShare
                     uint32_t f = w >> shift;
                     bool mine = true;
                     if ((w & kWordEdges) && unproven(a, w)) {
-                        f = unproven_cell(a, un, src_word + k, w, idx);
+                        f = unproven_cell(a, un, k, w);
                         mine = f != ~0u;
                     }
                     if (mine) i = (int)box.cell(f);
@@ -704,7 +704,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
         const bool staged = un.staged;
         const uint32_t shift = staged ? 1u : kFieldBits - a.s;
         const uint64_t start = un.start;
-        uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
+        const uint32_t* src_word = (staged ? a.stage_word : a.leaf_word) + start;
         const uint32_t* src_lut = (staged ? a.stage_lut : a.leaf_lut) + start;
         uint32_t wide = 0;   // colour bits above 8
         auto add = [&](uint32_t rank, uint32_t idx, uint32_t c0, uint32_t c1) {
@@ -771,7 +771,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
                         uint32_t f = w >> shift;
                         bool mine = true;
                         if ((w & kWordEdges) && unproven(a, w)) {
-                            f = unproven_cell(a, un, src_word + k, w, idx[j]);
+                            f = unproven_cell(a, un, k, w);
                             mine = f != ~0u;
                         }
                         if (mine) i[j] = (int)box.cell(f);
@@ -814,7 +814,7 @@ __device__ __forceinline__ bool unit_cells(const UnitLevelArgs& a, BlockShared& 
             for (uint32_t k = tid; k < cnt; k += T) {
                 const uint32_t w = src_word[k];
                 if (!(w & kWordEdges)) continue;
-                const uint32_t idx = src_lut[k], f = unproven(a, w) ? unproven_cell(a, un, src_word + k, w, idx) : w >> shift;
+                const uint32_t idx = src_lut[k], f = unproven(a, w) ? unproven_cell(a, un, k, w) : w >> shift;
                 if (f != ~0u) edge(box.rank(box.cell(f)), idx, w);
             }
             if (kOther && sh.foreign)
@@ -966,7 +966,7 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
     {
         const uint32_t cnt = un.cnt;
         const uint32_t shift = un.staged ? 1u : kFieldBits - a.s;
-        uint32_t* src_word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
+        const uint32_t* src_word = (un.staged ? a.stage_word : a.leaf_word) + un.start;
         bool beside = false;   // a candidate lies beside a boundary between cells
         if (kOther && un.large) {
             const uint32_t* map = a.maps + un.map;
@@ -988,7 +988,7 @@ __device__ __forceinline__ void unit_run(const UnitLevelArgs& a, BlockShared& sh
                 if (w[j] & kWordEdges) {
                     beside = true;
                     if (unproven(a, w[j])) {
-                        f = unproven_cell(a, un, src_word + k, w[j], ((un.staged ? a.stage_lut : a.leaf_lut) + un.start)[k]);
+                        f = unproven_cell(a, un, k, w[j]);
                         if (f == ~0u) continue;
                     }
                 }
@@ -1263,8 +1263,7 @@ __device__ __forceinline__ uint64_t level_base_of(const UnitLevelArgs& a) {
 template <class Get>
 __device__ __forceinline__ void large_candidates(const UnitLevelArgs& a, const LargePart& s, uint32_t slices,
                                                  const Box<0, uint32_t>& box, Get&& get) {
-    uint32_t* src_word = a.leaf_word + s.un.start;
-    const uint32_t* src_lut = a.leaf_lut + s.un.start;
+    const uint32_t* src_word = a.leaf_word + s.un.start;
     const uint32_t first = s.first(s.un.cnt, slices), end = s.end(s.un.cnt, slices);
     for (uint32_t k0 = first + threadIdx.x; k0 < end; k0 += 4 * kLargeThreads) {
         uint32_t w[4];
@@ -1276,7 +1275,7 @@ __device__ __forceinline__ void large_candidates(const UnitLevelArgs& a, const L
             if (k >= end) break;
             uint32_t f = w[j] >> (kFieldBits - a.s);
             if ((w[j] & kWordEdges) && unproven(a, w[j])) {
-                f = unproven_cell(a, s.un, src_word + k, w[j], src_lut[k]);
+                f = unproven_cell(a, s.un, k, w[j]);
                 if (f == ~0u) continue;
             }
             get(box.cell(f), w[j], k);
