@@ -1080,6 +1080,8 @@ void Builder::subsample() {
             while (nk) st.push_back({kids[--nk], false});
         }
     }
+    const uint32_t large_points = large_leaf_points(cfg_.n);
+    uint32_t largest_leaf = 0;
     std::vector<SubNode> table(n_internal);
     for (uint32_t k = 0; k < n_internal; ++k) {
         const NodeHost& v = nodes_[order[k]];
@@ -1107,6 +1109,7 @@ void Builder::subsample() {
             } else {
                 sn.child_start[nc] = ch.data_idx;
                 sn.child_count[nc] = ch.points;
+                largest_leaf = std::max(largest_leaf, ch.points);
             }
             ++nc;
         }
@@ -1118,7 +1121,8 @@ void Builder::subsample() {
     // (the top of the tree) inner children are split in parts, down to 4096
     // candidates.
     bool octants = leaf_cells_ && octant_subsampling();
-    std::vector<UnitEntry> units;
+    std::vector<UnitEntry>& units = unit_list_;
+    units.clear();
     std::vector<uint32_t> unit_first(depth_ + 2, 0);
     std::vector<uint8_t> any_split(depth_ + 2, 0), spread(depth_ + 2, 0);
     std::vector<uint32_t> oct_unit;          // spread levels, per node and octant
@@ -1132,12 +1136,19 @@ void Builder::subsample() {
     // Leaves that are shared by blocks have the first maps of their level.
     std::vector<uint32_t> large;             // their numbers among the level's units
     std::vector<uint32_t> large_first(depth_ + 2, 0), largest(depth_ + 2, 0);
-    const uint32_t large_points = large_leaf_points(cfg_.n);
     auto lay_out_units = [&](bool every_octant) {
         units.clear();
         oct_unit.clear();
         large.clear();
         map_words = 0;
+        // (by pointer: through the captures every access would be loaded again)
+        const NodeHost* const node_at = nodes_.data();
+        SubNode* const table_at = table.data();
+        const uint32_t* const order_at = order.data();
+        const uint32_t* const ii_at = ii_of.data();
+        const uint64_t* const bound_at = out_bound.data();
+        const uint32_t large_above = large_points;
+        const bool any_large = largest_leaf > large_above;
         // the part of the memory estimate that a brick table would take
         const uint64_t map_room = (uint64_t)num_sms_ * memory_terms(cfg_, num_sms_).slots * 8;
         for (uint32_t l = 1; l <= depth_; ++l) {
@@ -1147,9 +1158,9 @@ void Builder::subsample() {
             largest[l] = 0;
             uint64_t whole = 0, large_words = 0;
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
-                whole += table[k].nchild;
-                for (uint32_t c = 0; c < table[k].nchild; ++c)   // (0 for inner children)
-                    if (table[k].child_count[c] > large_points) large_words += large_map_words(s_log2);
+                whole += table_at[k].nchild;
+                for (uint32_t c = 0; any_large && c < table_at[k].nchild; ++c)   // (0 for inner children)
+                    if (table_at[k].child_count[c] > large_above) large_words += large_map_words(s_log2);
             }
             const bool few = S >= 64 && whole < (uint64_t)num_sms_ * 3;
             // inter-cell colours cost less: the extra launch's lookups in global
@@ -1160,34 +1171,34 @@ void Builder::subsample() {
             if (spread[l]) oct_unit.resize(oct_unit.size() + 8 * (size_t)(level_first[l + 1] - level_first[l]), ~0u);
             uint64_t words = large_words, candidates = 0;
             for (uint32_t k = level_first[l]; k < level_first[l + 1]; ++k) {
-                const NodeHost& v = nodes_[order[k]];
+                const NodeHost& v = node_at[order_at[k]];
                 uint32_t c = v.child_first, number = 0, q0 = 0;
-                table[k].child_kind &= 0xFFFFu;
+                table_at[k].child_kind &= 0xFFFFu;
                 for (uint32_t s = 0; s < 8; ++s) {
                     UnitEntry e{};
                     e.node = k - level_first[l];
                     bool split = false;
                     if (v.mask & (1u << s)) {
                         const uint32_t ci = c++;
-                        const NodeHost& ch = nodes_[ci];
-                        split = few && ch.internal && out_bound[ci] > 4096;
+                        const NodeHost& ch = node_at[ci];
+                        split = few && ch.internal && bound_at[ci] > 4096;
                         e.flags = (uint32_t)ch.internal << 7;
-                        e.src = ch.internal ? ii_of[ci] : (uint32_t)ch.data_idx;
+                        e.src = ch.internal ? ii_at[ci] : (uint32_t)ch.data_idx;
                         e.count = ch.internal ? 0 : ch.points;
-                        if (e.count > large_points) {
+                        if (e.count > large_above) {
                             e.flags |= 1u << 20;
                             e.map = (uint32_t)((large.size() - large_first[l]) * large_map_words(s_log2));
                             large.push_back((uint32_t)units.size() - unit_first[l]);
                             largest[l] = std::max(largest[l], e.count);
                         } else {
-                            candidates += ch.internal ? std::min<uint64_t>(out_bound[ci], 16384) : ch.points;
+                            candidates += ch.internal ? std::min<uint64_t>(bound_at[ci], 16384) : ch.points;
                         }
                     } else if (!every_octant) {
                         continue;
                     }
                     if (split) {
                         any_split[l] = 1;
-                        table[k].child_kind |= 1u << (16 + s);
+                        table_at[k].child_kind |= 1u << (16 + s);
                     }
                     if (spread[l])
                         oct_unit[oct_first[l] + (size_t)(k - level_first[l]) * 8 + s] =
@@ -1399,9 +1410,7 @@ void Builder::subsample() {
                                            units.size() * 8,
                                        stream_),
                        "memset");
-            uint64_t largest_unit = S3;
-            for (const UnitEntry& e : units)
-                if (!(e.flags >> 20)) largest_unit = std::max<uint64_t>(largest_unit, e.count);
+            const uint64_t largest_unit = std::max<uint64_t>(S3, std::min(largest_leaf, large_points));
             uint8_t* sync = unit_sync_.as<uint8_t>();
             UnitNodeState* node_state = reinterpret_cast<UnitNodeState*>(sync + kUnitSyncHead);
             uint64_t* unit_state = reinterpret_cast<uint64_t*>(node_state + n_internal);

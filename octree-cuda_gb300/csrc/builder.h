@@ -287,6 +287,7 @@ private:
     DevBuf leaf_frac_, stage_frac_;     // sub-step or cell words of leaf and staged records
     bool leaf_cells_ = false;           // the leaf words are cell words (octant subsampling)
     DevBuf units_, unit_sync_, oct_off_;   // octant subsampling: unit table, counters and waits, octant offsets
+    std::vector<UnitEntry> unit_list_;     // the unit table on the host (kept: fresh pages cost 0.1 ms at 38,000 units)
     DevBuf bbox_keys_;                  // ordered keys of the coordinate minima / maxima
     DevBuf stage_off_, level_base_;     // staged position of each internal node's outputs; staging fill
     uint8_t* host_rec_ = nullptr;      // caller's output arrays (set_output_host)
